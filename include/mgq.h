@@ -189,9 +189,9 @@ int mgq_exchange_all_gather_rows(const float *slice, uint32_t slice_pitch, uint3
 /* c[m,n] = a[m,k] . dequant(w)[k,n] (+ addend[m,n]); a is f32 or bf16 row-major, c is f32.
  * Stands in for the MatMul / FusedMatMulAdd dispatches with a quantized weight_format
  * (src/compile.rs:1408-1419, 1511-1522; src/shaders/matmul.wgsl:28-109).
- * bf16 activations with m >= 64 and k % 128 == 0 run on the tensor cores (tcgen05, TMEM
- * accumulator, TMA-fed activations, weights dequantized into bf16 hi+lo operand tiles); every
- * other case runs the register-tiled CUDA-core kernel. */
+ * Calls with k > 128 run on the tensor cores (tcgen05, operands as sums of f16 values, f32 accuracy) with a
+ * stream-ordered workspace from a memory pool of the library (at most 256 MB of it are kept between calls); shorter k, and
+ * calls whose workspace cannot be allocated, run the register-tiled CUDA-core kernel. */
 int mgq_gemm(int fmt, const void *a, int a_dtype, const void *w, const float *addend, float *c,
              uint32_t m, uint32_t k, uint32_t n, void *stream);
 

@@ -1,0 +1,849 @@
+// Dequantize-fused GEMM on the sm_100a tensor cores for any number of rows, any K and N:
+//     C[m,n] = A[m,k] (f32 or bf16) . dequant(W)[k,n] (+ addend),   f32 results at f32 accuracy.
+//
+// Stands in for the MatMul / FusedMatMulAdd dispatch with a quantized weight_format
+// (src/compile.rs:1408-1419, 1511-1522 of meganeura; kernel src/shaders/matmul.wgsl with
+// dequant_q4 / dequant_q8 as the B-tile load).
+//
+// Operands are sums of f16 values, whose products the tensor cores form exactly:
+//   activations  x = (hi + lo) * 2^e, e per row and 128 k (split_rows_kernel): all 24 bits of an f32 but the last
+//                one or two; a bf16 value fits hi alone, so that case has one plane and two products instead of three.
+//   weights      code * scale has at most 19 bits: hi = rn16(code * d), lo = fma16(code, d, -hi), both exact, two
+//                instructions for two weights.  Every such product is a multiple of 2^-24, so nothing is lost for small
+//                scales.  Q4 codes are centred (q - 8); what is left of the block's minimum, b = m + 8 d, times the
+//                block's sum s of activations takes one more step of K = 16 per chunk: for each of the chunk's four
+//                blocks b.hi s.hi + b.hi s.lo + b.lo s.hi.
+// The tensor core truncates when it adds to its f32 accumulator, which over a long K would cost more than f32 sums do
+// (9e-6 for bf16 activations and K = 4096 in one accumulator).  So one accumulator takes a chunk of 128 k only, the small
+// products first; then it is added to a register sum in f32, times 2^e: 2.2e-7 off the exact product at K = 4096 and 2.0e-7 at
+// K = 512, where f32 sums in order of k are 1.1e-6 and 3.9e-7 off.
+//
+// Weights are the left operand, straight from TMEM: a tile is 128 weight columns (TMEM lanes) by up to 128
+// tokens (any multiple of 16), so that few tokens cost few products and no shared-memory pass for weights.
+// Tiles are cut along K into chunks and the chunks of all tiles are shared out evenly over the CTAs (1 per SM); where a
+// tile is spread over several CTAs, each leaves its partial sums in the workspace and the one that finishes last adds
+// them up in order: results do not depend on timing.
+//   warp 0        token planes, 64 k of one plane per copy (cp.async.bulk of a block that split_rows_kernel has laid
+//                 out in the 128-byte swizzle), ring of 8; scales and (Q4) sums of a chunk, ring of 8.
+//   warp 1        MMA issue: tcgen05.mma.kind::f16, M=128 (weight columns), N=tokens, K=16, A in TMEM.
+//   warps 4-11    drain: 32 weight columns by half of the tokens per warp, sums in registers; results.
+//   warps 12-19   weights: two groups of four, chunks in turn; cp.async of a warp's 32 columns two chunks
+//                 of its own ahead, conversion, tcgen05.st.
+// TMEM: two accumulators of 128 columns, two weight stages of 64 (hi) + 64 (lo) columns.
+// Sums that are not finite (non-finite inputs, |code * scale| or |m + 8 d| beyond the f16 range) are computed again
+// element by element on the CUDA cores.
+//
+// What bounds it: of the 2650 cycles that a chunk of 128 x 128 takes with f32 activations the tensor core needs 1536 (2100 and 1024
+// for bf16), the rest is the hand-over of a weight stage: products of chunk i - 2 done, conversion (1500 cycles, four warps),
+// products of chunk i; 52 % of the issue slots are taken.  Measured and dropped: weight stages of 64 k (147 instead
+// of 112 us for bf16, twice the waits), two issuing warps and both groups on every chunk (no change).
+// 512 x 4096 x 12288 Q4 f32: 138 us against 1991 on the CUDA cores; 512 x 4096 x 14336 Q8 bf16: 127 against 141 us of a
+// kernel with one 112-column strip of bf16 weight pairs per CTA and 512 tokens.
+//
+// Every mbarrier wait is bounded; when one runs out the device-wide error word is raised (mgq_device_status reports
+// MGQ_ERR_TIMEOUT), the roles run to their ends without waiting and the CTA frees its TMEM.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <mutex>
+
+#include "mgq_launch.cuh"
+#include "mgq_tcgen05.cuh"
+
+namespace mgq {
+namespace {
+
+constexpr uint32_t kChunk = 128;                   // k per accumulator
+constexpr uint32_t kCols = 128;                    // weight columns of a tile
+constexpr uint32_t kMaxTok = 128;                  // tokens of a tile
+constexpr uint32_t kSlots = 8;                     // ring of token sub-tiles (64 k of one plane)
+constexpr uint32_t kScaleSlots = 8;
+constexpr uint32_t kRaw = 4;                       // chunks of packed weights in flight, two per group
+constexpr uint32_t kSplitThreads = 640;
+constexpr uint32_t kPassElems = 1u << 25;          // activations per launch: bounds the workspace (128 MB of planes)
+
+__device__ unsigned int g_split_error = 0;
+
+struct SplitParams {
+    const uint8_t *w;
+    const void *a;
+    const float *addend;
+    float *c;
+    const uint8_t *planes;          // [m tile][chunk][slot][tokens * 128 B]
+    const uint8_t *side;            // [m tile][chunk]: scales [tokens] f32 | Q4: sums [tokens][16] f16, see sums_at
+    float *partial;                 // [CTA][2][128 tokens][128 columns]
+    unsigned int *counters;         // one per tile
+    unsigned long long num_blocks;
+    uint32_t m, k, n, bpc;
+    uint32_t tok, m_tiles, tiles;   // tokens of a tile, tiles
+    uint32_t chunks;                // per tile
+    uint32_t units;                 // tiles * chunks
+    uint32_t wide;                  // packed weights can be copied 16 bytes at a time
+};
+
+struct __align__(16) SplitShared {
+    unsigned long long slot_full[kSlots], slot_empty[kSlots / 2];      // empty: a chunk's sub-tiles together
+    unsigned long long sc_full[kScaleSlots], sc_empty[kScaleSlots];
+    unsigned long long w_full[2], d_empty[2], done[2], flushed;        // done: a chunk's products (its weight stage is free, its accumulator full)
+    uint32_t tmem_base;
+    volatile int failed;
+    uint32_t last;
+};
+
+__host__ __device__ constexpr uint32_t raw_bytes(int fmt) { return fmt == MGQ_FMT_Q8 ? 144u : 80u; }      // of a column and chunk: Q4 = 16 header bytes | 64 nibble bytes
+
+// K = 16 operands of the minimum step: no swizzle, 8 rows x 16 bytes side by side, the two halves of K 128 bytes apart.
+__host__ __device__ constexpr uint32_t sums_at(uint32_t row, uint32_t half) { return (row >> 3) * 256u + half * 128u + (row & 7u) * 16u; }
+__host__ __device__ constexpr uint32_t side_bytes(int fmt, uint32_t tok) { return tok * (fmt == MGQ_FMT_Q4 ? 36u : 4u); }
+constexpr uint32_t kMinBytes = kCols * 32;         // minima of a chunk
+
+// CTA that owns unit u, and first unit of CTA g, when `units` are shared out over `ctas`.
+__host__ __device__ inline uint32_t unit_owner(uint32_t u, uint32_t units, uint32_t ctas)
+{
+    return (uint32_t)((((unsigned long long)u + 1) * ctas - 1) / units);
+}
+__host__ __device__ inline uint32_t unit_start(uint32_t g, uint32_t units, uint32_t ctas)
+{
+    return (uint32_t)((unsigned long long)g * units / ctas);
+}
+
+// ------------------------------------------------------------------------------------ activations
+
+__device__ __forceinline__ float load_act(const void *a, size_t i, bool bf16)
+{
+    return bf16 ? __bfloat162float(static_cast<const __nv_bfloat16 *>(a)[i]) : static_cast<const float *>(a)[i];
+}
+
+// Powers of two: values up to `top` come out below 2^15 when multiplied by `down`.
+__device__ __forceinline__ void pick_scale(float top, float &down, float &up)
+{
+    const int e = (int)((__float_as_uint(top) >> 23) & 0xFFu) - 127;      // 128: infinity or NaN
+    const int s = max(min(14 - e, 126), -126);
+    down = __uint_as_float((uint32_t)(127 + s) << 23);
+    up = __uint_as_float((uint32_t)(127 - s) << 23);
+}
+
+// Four consecutive places of one row: f16 parts of v * down into the planes' swizzled sub-tiles.  pos: place within the chunk.
+__device__ __forceinline__ void store4(uint8_t *block, uint32_t sub, uint32_t planes, uint32_t t, uint32_t pos, const float (&v)[4], float down)
+{
+    __align__(8) __half hi[4], lo[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float s = v[i] * down;
+        hi[i] = __float2half_rn(s);
+        lo[i] = __float2half_rn(s - __half2float(hi[i]));
+    }
+    const uint32_t half = pos >> 6, byte = (pos & 63u) * 2u;
+    uint8_t *h = block + (size_t)((planes == 2 ? 2u : 0u) + half) * sub + t * 128u, *l = block + (size_t)half * sub + t * 128u;      // lo, lo, hi, hi
+    const uint32_t at = (((byte >> 4) ^ (t & 7u)) << 4) | (byte & 15u);
+    *reinterpret_cast<uint2 *>(h + at) = *reinterpret_cast<const uint2 *>(hi);
+    if (planes == 2) *reinterpret_cast<uint2 *>(l + at) = *reinterpret_cast<const uint2 *>(lo);
+}
+
+// A warp per row and chunk.  Bound by the read of the activations (8 MB for 512 x 4096 f32) and as many bytes written,
+// all of which stay in L2 for the GEMM behind it.
+__global__ void __launch_bounds__(256) split_rows_kernel(const void *a, bool bf16, bool vec, uint8_t *planes_out, uint8_t *side_out, unsigned int *counters, uint32_t tiles,
+                                                         uint32_t m, uint32_t k, uint32_t tok, uint32_t chunks, uint32_t planes, bool q4)
+{
+    pdl_launch_dependents();
+    const uint32_t lane = threadIdx.x & 31u, gid = blockIdx.x * 8 + (threadIdx.x >> 5);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < tiles; i += gridDim.x * blockDim.x) counters[i] = 0;      // the GEMM's tile counters
+    const uint32_t row = gid / chunks, chunk = gid % chunks;
+    if (row >= m) return;
+    const uint32_t mt = row / tok, t = row % tok, sub = tok * 128u;
+    float v[4] = {};
+    const uint32_t kk = chunk * kChunk + lane * 4;
+    if (kk < k) {
+        const size_t at = (size_t)row * k + kk;
+        if (vec && !bf16) {
+            const float4 q = *reinterpret_cast<const float4 *>(static_cast<const float *>(a) + at);
+            v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+        } else if (vec) {
+            const uint2 q = *reinterpret_cast<const uint2 *>(static_cast<const __nv_bfloat16 *>(a) + at);
+            v[0] = __uint_as_float(q.x << 16); v[1] = __uint_as_float(q.x & 0xFFFF0000u);
+            v[2] = __uint_as_float(q.y << 16); v[3] = __uint_as_float(q.y & 0xFFFF0000u);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] = load_act(a, at + i, bf16);
+        }
+    }
+    uint32_t top = 0;                                           // largest magnitude by its bits: NaN stays the largest
+#pragma unroll
+    for (int i = 0; i < 4; i++) top = max(top, __float_as_uint(v[i]) & 0x7FFFFFFFu);
+    float sum = 0.f;                                            // of this lane's block of 32
+    if (q4) {
+        sum = (v[0] + v[1]) + (v[2] + v[3]);
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        top = max(top, __float_as_uint(sum) & 0x7FFFFFFFu);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    float down, up;
+    pick_scale(__uint_as_float(top), down, up);
+    const size_t block = (size_t)mt * chunks + chunk;
+    uint8_t *side = side_out + block * side_bytes(q4 ? MGQ_FMT_Q4 : MGQ_FMT_Q8, tok);
+    // not finite: a NaN scale makes the row's sums NaN, which the GEMM computes again
+    if (lane == 0) reinterpret_cast<float *>(side)[t] = top >= 0x7F800000u ? __uint_as_float(0x7FC00000u) : up;
+    if (q4) {
+        // Q4 weights unpack as pairs (k, k + 4) of eight: order 0 4 1 5 2 6 3 7
+        const bool odd = lane & 1u;
+        const float r0 = __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[2], 1), r1 = __shfl_xor_sync(0xffffffffu, odd ? v[1] : v[3], 1);
+        if (odd) { v[0] = r0; v[1] = v[2]; v[2] = r1; }
+        else     { v[3] = r1; v[2] = v[1]; v[1] = r0; }
+        // places 0-3 s.hi, 4-7 s.lo, 8-11 s.hi, 12-15 zero, beside the weights' b.hi, b.hi, b.lo, zero
+        if ((lane & 7u) == 0) {
+            const uint32_t b = lane >> 3;
+            const float s = sum * down;
+            const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
+            __half *first = reinterpret_cast<__half *>(side + tok * 4u + sums_at(t, 0)), *second = reinterpret_cast<__half *>(side + tok * 4u + sums_at(t, 1));
+            first[b] = hi; first[4 + b] = lo;
+            second[b] = hi; second[4 + b] = __float2half_rn(0.f);
+        }
+    }
+    store4(planes_out + block * 2 * planes * sub, sub, planes, t, lane * 4, v, down);
+}
+
+// ------------------------------------------------------------------------------------------ pieces
+
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, unsigned long long *bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+// 16 or 4 bytes; live false: zeros.
+__device__ __forceinline__ void copy16(uint32_t dst, const void *src, bool live)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16u : 0u) : "memory");
+}
+__device__ __forceinline__ void copy4(uint32_t dst, const void *src, bool live)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(live ? 4u : 0u) : "memory");
+}
+
+// D[128 lanes, N] (+)= A (f16 pairs in TMEM, 8 columns) . B (shared memory)
+template <bool ACC>
+__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint64_t desc_b, uint32_t instr)
+{
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "setp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "l"(desc_b), "r"(instr), "n"(ACC ? 1 : 0) : "memory");
+}
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t is;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
+    return is != 0;
+}
+// A converged warp waits for several barriers at once, a lane (with `mine` set) for each: the try_waits share one latency.
+__device__ __forceinline__ bool mbar_wait_lanes(unsigned long long *bar, uint32_t parity, bool mine, volatile int *failed)
+{
+    bool done = !mine;
+    for (uint32_t i = 0; i < kWaitLimit; i++) {
+        if (!done) done = mbar_try_wait(bar, parity);
+        if (__all_sync(0xffffffffu, done)) return true;
+        if (__any_sync(0xffffffffu, *failed != 0)) return false;
+    }
+    *failed = 1;
+    atomicExch(&g_split_error, 1u);
+    return false;
+}
+// K-major without a swizzle: halves of K 128 bytes apart, groups of 8 rows 256.
+__device__ __forceinline__ uint64_t plain_desc(uint32_t smem_addr)
+{
+    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (uint64_t)(128 >> 4) << 16 | (uint64_t)(256 >> 4) << 32 | (uint64_t)1 << 46;
+}
+// kind::f16 instruction descriptor: D f32, A and B f16, both K-major.
+__device__ __forceinline__ uint32_t split_instr(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((kCols >> 4) << 24); }
+
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+                 "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+
+__device__ __forceinline__ __half2 as_half2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
+__device__ __forceinline__ uint32_t as_word(__half2 v) { return *reinterpret_cast<const uint32_t *>(&v); }
+
+// Two codes as f16 1024 + c in one word -> exact parts of (c - offset) * d.
+__device__ __forceinline__ void split_codes(uint32_t magic, __half2 offset, __half2 d, uint32_t &hi, uint32_t &lo)
+{
+    const __half2 c = __hsub2(as_half2(magic), offset);
+    const __half2 h = __hmul2_rn(c, d);                         // never contracted into the fma below
+    hi = as_word(h);
+    lo = as_word(__hfma2(c, d, __hneg2(h)));
+}
+
+// The element (row, col) in plain f32, the way the tiled kernel sums it.
+template <int FMT>
+__device__ __noinline__ float plain_element(const SplitParams &p, bool bf16, uint32_t row, uint32_t col)
+{
+    float acc = 0.f;
+    const uint32_t *w32 = reinterpret_cast<const uint32_t *>(p.w);
+    for (uint32_t b = 0; b < p.bpc; b++) {
+        const unsigned long long g = (unsigned long long)col * p.bpc + b;
+        float d, lo = 0.f;
+        const uint32_t *q;
+        if (FMT == MGQ_FMT_Q4) {
+            const float2 dm = __half22float2(as_half2(w32[g]));
+            d = dm.x; lo = dm.y;
+            q = w32 + p.num_blocks + g * 4;
+        } else {
+            d = __half2float(__ushort_as_half((unsigned short)(w32[g * 9] & 0xFFFFu)));
+            q = w32 + g * 9 + 1;
+        }
+        for (uint32_t i = 0; i < 32; i++) {
+            const float code = FMT == MGQ_FMT_Q4 ? (float)((q[i >> 3] >> (4 * (i & 7u))) & 0xFu) : (float)(int)(signed char)((q[i >> 2] >> (8 * (i & 3u))) & 0xFFu);
+            const float w = FMT == MGQ_FMT_Q4 ? code * d + lo : code * d;
+            acc = fmaf(load_act(p.a, (size_t)row * p.k + b * 32u + i, bf16), w, acc);
+        }
+    }
+    return acc;
+}
+
+// Asynchronous copy of the packed bytes that a warp's 32 columns (from col0) hold of a chunk; neighbouring lanes copy
+// neighbouring pieces of a column, and a lane's addresses advance by constants.  Blocks beyond K read as zeros; columns
+// beyond N are left out (a weight column is a row of the product: nothing else depends on it).
+template <int FMT>
+__device__ __forceinline__ void fetch_weights(const SplitParams &p, uint32_t dst, uint32_t col0, uint32_t chunk, uint32_t lane)
+{
+    constexpr uint32_t kBytes = raw_bytes(FMT);
+    const uint32_t b0 = chunk * 4, cols = col0 < p.n ? min(32u, p.n - col0) : 0u;
+    const unsigned long long block = (unsigned long long)col0 * p.bpc + b0;
+    if (FMT == MGQ_FMT_Q8) {
+        const uint8_t *src = p.w + block * 36u;
+        const size_t pitch = (size_t)p.bpc * 36u;
+        if (p.wide) {                                           // 9 pieces of 16 bytes: three lanes per column
+            const uint32_t c = lane / 3, piece = (lane % 3) * 16u;
+            const uint8_t *from = src + c * pitch + piece;
+            const uint32_t to = dst + c * kBytes + piece;
+#pragma unroll
+            for (uint32_t i = 0; i < 3; i++)
+                if (c < 10 && c + i * 10 < cols) {
+#pragma unroll
+                    for (uint32_t x = 0; x < 3; x++) copy16(to + i * 10 * kBytes + x * 48u, from + i * 10 * pitch + x * 48u, true);
+                }
+            const uint32_t rest = 30 + lane / 9;                // columns 30 and 31: 18 lanes
+            if (lane < 18 && rest < cols) copy16(dst + rest * kBytes + (lane % 9) * 16u, src + rest * pitch + (lane % 9) * 16u, true);
+        } else {                                                // 36 words: a whole warp per column, the last four words of eight columns at a time
+            const bool live = b0 + lane / 9 < p.bpc;
+            const uint8_t *from = live ? src + lane * 4u : p.w;
+            const size_t step = live ? pitch : 0;
+            const uint32_t to = dst + lane * 4u;
+#pragma unroll 8
+            for (uint32_t c = 0; c < cols; c++) copy4(to + c * kBytes, from + c * step, live);
+            const uint32_t c = lane / 4, word = 32 + lane % 4;
+            const bool rest = b0 + 3 < p.bpc;
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++)
+                if (c + i * 8 < cols) copy4(dst + (c + i * 8) * kBytes + word * 4u, rest ? src + (c + i * 8) * pitch + word * 4u : p.w, rest);
+        }
+    } else {
+        const uint32_t c = lane / 4, b = lane % 4;              // four blocks of eight columns at a time
+        const bool live = b0 + b < p.bpc;
+        const uint8_t *hdr = p.w + (block + (unsigned long long)c * p.bpc + b) * 4u, *nib = p.w + (p.num_blocks + (block + (unsigned long long)c * p.bpc + b) * 4u) * 4u;
+#pragma unroll
+        for (uint32_t i = 0; i < 4; i++)
+            if (c + i * 8 < cols) copy4(dst + (c + i * 8) * kBytes + b * 4u, live ? hdr + (size_t)i * 8 * p.bpc * 4u : p.w, live);
+        if (p.wide) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++)
+                if (c + i * 8 < cols) copy16(dst + (c + i * 8) * kBytes + 16u + b * 16u, live ? nib + (size_t)i * 8 * p.bpc * 16u : p.w, live);
+        } else {
+            const uint32_t c2 = lane / 16, word = lane % 16;
+            const bool live2 = b0 + word / 4 < p.bpc;
+            const uint8_t *from = p.w + (p.num_blocks + (block + (unsigned long long)c2 * p.bpc) * 4u + word) * 4u;
+#pragma unroll 4
+            for (uint32_t i = 0; i < 16; i++)
+                if (c2 + i * 2 < cols) copy4(dst + (c2 + i * 2) * kBytes + 16u + word * 4u, live2 ? from + (size_t)i * 2 * p.bpc * 16u : p.w, live2);
+        }
+    }
+}
+
+// a += v * s for two neighbours in one instruction (each rounded as by fmaf).
+__device__ __forceinline__ void fma_pair(float &a0, float &a1, uint32_t v0, uint32_t v1, float s0, float s1)
+{
+    asm("{\n\t.reg .b64 a, v, s;\n\t"
+        "mov.b64 a, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tmov.b64 s, {%4, %5};\n\t"
+        "fma.rn.f32x2 a, v, s, a;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t}"
+        : "+f"(a0), "+f"(a1) : "r"(v0), "r"(v1), "f"(s0), "f"(s1));
+}
+
+// COUNT groups of 16 tokens: sums += accumulator * scale.
+template <int G0, int COUNT>
+__device__ __forceinline__ void drain_part(uint32_t from, const uint8_t *scale, float (&acc)[4][16])
+{
+    uint32_t r[COUNT][16];
+#pragma unroll
+    for (int g = 0; g < COUNT; g++)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                     "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                     : "=r"(r[g][0]), "=r"(r[g][1]), "=r"(r[g][2]), "=r"(r[g][3]), "=r"(r[g][4]), "=r"(r[g][5]), "=r"(r[g][6]), "=r"(r[g][7]),
+                       "=r"(r[g][8]), "=r"(r[g][9]), "=r"(r[g][10]), "=r"(r[g][11]), "=r"(r[g][12]), "=r"(r[g][13]), "=r"(r[g][14]), "=r"(r[g][15])
+                     : "r"(from + (G0 + g) * 16) : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int g = 0; g < COUNT; g++)
+#pragma unroll
+        for (int e = 0; e < 16; e += 4) {
+            const float4 s = *reinterpret_cast<const float4 *>(scale + ((G0 + g) * 16 + e) * 4);
+            fma_pair(acc[G0 + g][e], acc[G0 + g][e + 1], r[g][e], r[g][e + 1], s.x, s.y);
+            fma_pair(acc[G0 + g][e + 2], acc[G0 + g][e + 3], r[g][e + 2], r[g][e + 3], s.z, s.w);
+        }
+}
+
+// acc += the sums that another CTA has left.
+__device__ __forceinline__ void add_part(const float *src, uint32_t groups, float (&acc)[4][16])
+{
+#pragma unroll
+    for (int g = 0; g < 4; g++)
+        if (g < (int)groups) {
+            float v[16];
+#pragma unroll
+            for (int e = 0; e < 16; e++) v[e] = __ldcg(src + (g * 16 + e) * kCols);
+#pragma unroll
+            for (int e = 0; e < 16; e++) acc[g][e] += v[e];
+        }
+}
+
+template <int FMT, int PLANES>
+__global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __grid_constant__ SplitParams p)
+{
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ SplitShared sh;
+    constexpr uint32_t kRawChunk = kCols * raw_bytes(FMT);
+    constexpr uint32_t kParts = 2 * PLANES, kDepth = kSlots / kParts;       // sub-tiles of a chunk, chunks in the ring
+    uint8_t *ring = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    const uint32_t sub = p.tok * 128u;                          // bytes of a token sub-tile, a multiple of 2048
+    const uint32_t side = side_bytes(FMT, p.tok);               // a multiple of 64
+    uint8_t *side_ring = ring + kSlots * sub;
+    uint8_t *raw = side_ring + kScaleSlots * side;
+    uint8_t *minima = raw + kRaw * kRawChunk;                   // Q4: two stages
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t u_begin = unit_start(blockIdx.x, p.units, gridDim.x), u_end = unit_start(blockIdx.x + 1, p.units, gridDim.x);
+
+    if (tid == 0) {
+        for (uint32_t s = 0; s < kSlots; s++) mbar_init(&sh.slot_full[s], 1);
+        for (uint32_t s = 0; s < kDepth; s++) mbar_init(&sh.slot_empty[s], 1);
+        for (uint32_t s = 0; s < kScaleSlots; s++) { mbar_init(&sh.sc_full[s], 1); mbar_init(&sh.sc_empty[s], 8); }
+        for (uint32_t s = 0; s < 2; s++) {
+            mbar_init(&sh.w_full[s], 4);
+            mbar_init(&sh.d_empty[s], 8);
+            mbar_init(&sh.done[s], 1);
+        }
+        mbar_init(&sh.flushed, 1);
+        sh.failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc(&sh.tmem_base, 512);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sh.tmem_base;
+    const uint32_t tmem_w = tmem + 2 * kMaxTok;                 // stage s: hi at +128 s, lo at +128 s + 64
+
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        if (warp == 0) {
+            // ------------------------------------------------------------------ token planes and scales
+            // lane x: the x-th sub-tile of every chunk; lane kParts: scales and sums.  One lane for all of them was late: a
+            // wait, an arrival and a copy take it 300 cycles.
+            if (lane <= kParts) {
+                pdl_wait();
+                const uint32_t depth = lane < kParts ? kDepth : kScaleSlots, count = u_end - u_begin;
+                const uint32_t bytes = lane < kParts ? sub : side, pitch = lane < kParts ? kParts * sub : side;
+                const uint8_t *base = lane < kParts ? p.planes + lane * sub : p.side;
+                // [m tile][chunk]: the tiles of a column strip follow one another
+                uint32_t at = u_begin / p.chunks % p.m_tiles * p.chunks + u_begin % p.chunks, armed = 0;
+                const uint32_t wrap = p.m_tiles * p.chunks;
+                for (uint32_t i = 0; i < count; i++, at = at + 1 == wrap ? 0 : at + 1) {
+                    const uint32_t s = i % depth, slot = s * kParts + lane;
+                    unsigned long long *full = lane < kParts ? &sh.slot_full[slot] : &sh.sc_full[s], *empty = lane < kParts ? &sh.slot_empty[s] : &sh.sc_empty[s];
+                    if (!mbar_wait(empty, ((i / depth) & 1u) ^ 1u, &sh.failed, &g_split_error)) continue;
+                    mbar_arrive_expect_tx(full, bytes);
+                    bulk_load(lane < kParts ? ring + slot * sub : side_ring + s * side, base + (size_t)at * pitch, bytes, full);
+                    armed = i + 1;
+                }
+                if (sh.failed)                                  // let this lane's own copies land before the CTA exits
+                    for (uint32_t j = armed > depth ? armed - depth : 0; j < armed; j++) {
+                        unsigned long long *full = lane < kParts ? &sh.slot_full[j % depth * kParts + lane] : &sh.sc_full[j % depth];
+                        for (uint32_t i = 0; i < kWaitLimit && !mbar_try_wait(full, (j / depth) & 1u); i++) { }
+                    }
+            }
+        } else if (warp == 1) {
+            // ------------------------------------------------------------------ MMA issue
+            // The whole warp runs the loop and one elected lane issues: addresses and descriptors then stay in uniform registers (a
+            // lane in a branch of its own took 100 cycles per MMA, N = 128 needs 64).  All waits of a chunk at once and two
+            // commits per chunk (each takes the warp 170 cycles).
+            const uint32_t instr = split_instr(p.tok);
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), count = __shfl_sync(0xffffffffu, u_end - u_begin, 0);
+            const bool leader = elect_one();
+            const uint64_t ring_desc = umma_desc(smem_u32(ring));
+            const uint32_t sub16 = sub >> 4;
+            bool ok = true;
+            for (uint32_t i = 0; i < count; i++) {
+                const uint32_t b = i & 1u, ph = (i >> 1) & 1u, s = i % kDepth;
+                const uint32_t d = tm + b * kMaxTok, w_hi = tm + 2 * kMaxTok + b * 128u, w_lo = w_hi + 64u;
+                // lane 0: accumulator, 1: weights, 2: sums (Q4), 4..: the chunk's sub-tiles
+                unsigned long long *bar = lane == 0 ? &sh.d_empty[b] : lane == 1 ? &sh.w_full[b] : lane == 2 ? &sh.sc_full[i % kScaleSlots] : &sh.slot_full[(s * kParts + lane - 4u) % kSlots];
+                const uint32_t parity = lane == 0 ? ph ^ 1u : lane == 1 ? ph : lane == 2 ? (i / kScaleSlots) & 1u : (i / kDepth) & 1u;
+                ok = mbar_wait_lanes(bar, parity, lane < 2 || (FMT == MGQ_FMT_Q4 && lane == 2) || (lane >= 4 && lane < 4 + kParts), &sh.failed);
+                if (!ok) break;
+                tc_fence_after();
+                if (leader) {
+                    const uint64_t x_lo = ring_desc + s * kParts * sub16, x_hi = x_lo + (kParts - 2) * sub16;
+                    if (FMT == MGQ_FMT_Q4)
+                        umma_f16(d, plain_desc(smem_u32(minima + b * kMinBytes)), plain_desc(smem_u32(side_ring + (i % kScaleSlots) * side + p.tok * 4u)), instr, 0u);
+                    if (FMT == MGQ_FMT_Q4) umma_f16_ts<true>(d, w_lo, x_hi, instr);
+                    else                   umma_f16_ts<false>(d, w_lo, x_hi, instr);
+#pragma unroll
+                    for (uint32_t j = 1; j < 8; j++) umma_f16_ts<true>(d, w_lo + j * 8u, x_hi + (j / 4) * sub16 + (j % 4) * 2u, instr);
+                    if (PLANES == 2)
+#pragma unroll
+                        for (uint32_t j = 0; j < 8; j++) umma_f16_ts<true>(d, w_hi + j * 8u, x_lo + (j / 4) * sub16 + (j % 4) * 2u, instr);
+#pragma unroll
+                    for (uint32_t j = 0; j < 8; j++) umma_f16_ts<true>(d, w_hi + j * 8u, x_hi + (j / 4) * sub16 + (j % 4) * 2u, instr);
+                    umma_commit(&sh.done[b]);
+                    umma_commit(&sh.slot_empty[s]);
+                }
+                __syncwarp();
+            }
+            if (!ok && leader) {                                // products in flight end before the CTA does
+                umma_commit(&sh.flushed);
+                for (uint32_t i = 0; i < kWaitLimit && !mbar_try_wait(&sh.flushed, 0); i++) { }
+            }
+        }
+    } else if (warp < 12) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 128;");
+        // ---------------------------------------------------------------------- drain and results
+        const uint32_t quad = warp & 3u, wg = (warp - 4) >> 2;
+        const uint32_t lane_addr = (quad * 32u) << 16;
+        // the first four warps take the first half of the tile's groups of 16 tokens, the others the rest
+        const uint32_t groups = p.tok / 16, half = (groups + 1) / 2;
+        const uint32_t first = wg * half * 16, mine = wg ? groups - half : half;
+        const uint32_t j = quad * 32 + lane;                    // weight column within the tile
+        float acc[4][16];                                       // tokens first + 16 g + e
+        uint32_t i = 0;
+        for (uint32_t u = u_begin; u < u_end;) {
+            const uint32_t tile = u / p.chunks, c0 = u % p.chunks;
+            const uint32_t c1 = min(p.chunks, c0 + (u_end - u));
+#pragma unroll
+            for (int g = 0; g < 4; g++)
+#pragma unroll
+                for (int e = 0; e < 16; e++) acc[g][e] = 0.f;
+            for (uint32_t c = c0; c < c1; c++, i++) {
+                const uint32_t b = i & 1u, sc = i % kScaleSlots;
+                mbar_wait_lanes(lane == 0 ? &sh.done[b] : &sh.sc_full[sc], lane == 0 ? (i >> 1) & 1u : (i / kScaleSlots) & 1u, lane < 2, &sh.failed);
+                __syncwarp();                                   // tcgen05.ld is warp-collective
+                tc_fence_after();
+                const uint32_t from = tmem + lane_addr + b * kMaxTok + first;
+                const uint8_t *scale = side_ring + sc * side + first * 4u;
+                if (mine > 1) drain_part<0, 2>(from, scale, acc);
+                else if (mine > 0) drain_part<0, 1>(from, scale, acc);
+                if (mine > 3) drain_part<2, 2>(from, scale, acc);
+                else if (mine > 2) drain_part<2, 1>(from, scale, acc);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&sh.d_empty[b]);
+                    mbar_arrive(&sh.sc_empty[sc]);
+                }
+            }
+            u += c1 - c0;
+
+            bool finish = true;
+            if (c0 != 0 || c1 != p.chunks) {
+                // part of a tile: leave the sums, the last CTA to get here adds all parts in the order of their chunks
+                const uint32_t head = unit_owner(tile * p.chunks, p.units, gridDim.x), tail = unit_owner((tile + 1) * p.chunks - 1, p.units, gridDim.x);
+                auto part_of = [&](uint32_t s) {
+                    return p.partial + ((size_t)s * 2 + (unit_start(s, p.units, gridDim.x) <= tile * p.chunks ? 1 : 0)) * (kMaxTok * kCols) + first * kCols + j;
+                };
+                bool waiting = false;                           // the other one of two parts is there already: no need to leave this one
+                if (tail == head + 1) {
+                    if (tid == 128) {
+                        uint32_t seen;
+                        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(p.counters + tile) : "memory");
+                        sh.last = seen;
+                    }
+                    asm volatile("bar.sync 1, 256;" ::: "memory");
+                    waiting = sh.last != 0;
+                    asm volatile("bar.sync 1, 256;" ::: "memory");      // sh.last may be written again
+                }
+                if (waiting) {
+                    add_part(part_of(blockIdx.x == head ? tail : head), mine, acc);
+                } else {
+                    float *part = part_of(blockIdx.x);
+#pragma unroll
+                    for (int g = 0; g < 4; g++)
+                        if (g < (int)mine)
+#pragma unroll
+                            for (int e = 0; e < 16; e++) __stcg(part + (g * 16 + e) * kCols, acc[g][e]);
+                    __threadfence();
+                    asm volatile("bar.sync 1, 256;" ::: "memory");
+                    if (tid == 128) {
+                        sh.last = atomicAdd(p.counters + tile, 1u) == tail - head ? 1u : 0u;
+                        __threadfence();
+                    }
+                    asm volatile("bar.sync 1, 256;" ::: "memory");
+                    finish = sh.last != 0;
+                    asm volatile("bar.sync 1, 256;" ::: "memory");      // sh.last may be written again
+                    if (finish) {
+                        __threadfence();
+#pragma unroll
+                        for (int g = 0; g < 4; g++)
+#pragma unroll
+                            for (int e = 0; e < 16; e++) acc[g][e] = 0.f;
+                        for (uint32_t s = head; s <= tail; s++) add_part(part_of(s), mine, acc);      // this CTA's own part among them
+                    }
+                }
+            }
+            if (finish) {
+                const uint32_t col = (tile / p.m_tiles) * kCols + j, m0 = (tile % p.m_tiles) * p.tok + first;
+                const uint32_t rows = col < p.n && m0 < p.m ? min(mine * 16u, p.m - m0) : 0u;
+                const size_t o0 = (size_t)m0 * p.n + col;
+                unsigned long long odd = 0;                     // sums that are not finite
+#pragma unroll
+                for (int g = 0; g < 4; g++) {
+#pragma unroll
+                    for (int e = 0; e < 16; e++)
+                        if (!(fabsf(acc[g][e]) < __uint_as_float(0x7F800000u))) odd |= 1ull << (g * 16 + e);
+                    if (p.addend) {
+                        float v[16];
+#pragma unroll
+                        for (int e = 0; e < 16; e++) v[e] = g * 16 + e < (int)rows ? p.addend[o0 + (size_t)(g * 16 + e) * p.n] : 0.f;
+#pragma unroll
+                        for (int e = 0; e < 16; e++) acc[g][e] += v[e];
+                    }
+#pragma unroll
+                    for (int e = 0; e < 16; e++)
+                        if (g * 16 + e < (int)rows && !(odd >> (g * 16 + e) & 1u)) p.c[o0 + (size_t)(g * 16 + e) * p.n] = acc[g][e];
+                }
+                if (rows < 64) odd &= (1ull << rows) - 1;
+                while (odd) {
+                    const uint32_t row = m0 + __ffsll((long long)odd) - 1;
+                    odd &= odd - 1;
+                    const float v = plain_element<FMT>(p, PLANES == 1, row, col);
+                    const size_t o = (size_t)row * p.n + col;
+                    p.c[o] = p.addend ? v + p.addend[o] : v;
+                }
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+        // ---------------------------------------------------------------------- weights
+        const uint32_t group = (warp - 12) >> 2, quad = warp & 3u;
+        const uint32_t count = u_end - u_begin;
+        const uint32_t mine = smem_u32(raw) + quad * 32u * raw_bytes(FMT);     // + place * kRawChunk
+        uint32_t next = group, tile = (u_begin + group) / p.chunks, chunk = (u_begin + group) % p.chunks, col0 = (tile / p.m_tiles) * kCols + quad * 32;
+        auto fetch = [&] {                                      // this group's next chunk, into the ring's place for it
+            if (next < count) fetch_weights<FMT>(p, mine + (next % kRaw) * kRawChunk, col0, chunk, lane);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            next += 2;
+            chunk += 2;
+            if (chunk >= p.chunks) {
+                tile += chunk / p.chunks;
+                chunk %= p.chunks;
+                col0 = (tile / p.m_tiles) * kCols + quad * 32;
+            }
+        };
+        fetch();
+        fetch();
+        for (uint32_t i = group; i < count; i += 2) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            const uint8_t *src = raw + (i % kRaw) * kRawChunk + (quad * 32 + lane) * raw_bytes(FMT);
+            mbar_wait(&sh.done[group], ((i >> 1) & 1u) ^ 1u, &sh.failed, &g_split_error);
+            __syncwarp();
+            tc_fence_after();
+            const uint32_t dst = tmem_w + ((quad * 32u) << 16) + group * 128u;
+            if (FMT == MGQ_FMT_Q4) {
+                const uint4 head = *reinterpret_cast<const uint4 *>(src);
+                const uint32_t h[4] = {head.x, head.y, head.z, head.w};
+                const __half2 offset = __float2half2_rn(1032.f);
+                float b[4];
+#pragma unroll
+                for (int blk = 0; blk < 4; blk++) {
+                    uint32_t hi[16], lo[16];
+                    const float2 dm = __half22float2(as_half2(h[blk]));
+                    b[blk] = fmaf(8.f, dm.x, dm.y);
+                    const __half2 d = __half2half2(__low2half(as_half2(h[blk])));
+                    const uint4 q4 = *reinterpret_cast<const uint4 *>(src + 16u + blk * 16u);
+                    const uint32_t q[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+#pragma unroll
+                        for (int s = 0; s < 4; s++)             // codes s and s + 4 of eight
+                            split_codes(((q[e] >> (4 * s)) & 0x000F000Fu) | 0x64006400u, offset, d, hi[e * 4 + s], lo[e * 4 + s]);
+                    tmem_st16(dst + blk * 16u, hi);
+                    tmem_st16(dst + 64u + blk * 16u, lo);
+                }
+                const __half2 h01 = __floats2half2_rn(b[0], b[1]), h23 = __floats2half2_rn(b[2], b[3]);
+                const __half2 l01 = __floats2half2_rn(b[0] - __low2float(h01), b[1] - __high2float(h01));
+                const __half2 l23 = __floats2half2_rn(b[2] - __low2float(h23), b[3] - __high2float(h23));
+                uint8_t *mins = minima + group * kMinBytes;
+                *reinterpret_cast<uint4 *>(mins + sums_at(quad * 32 + lane, 0)) = make_uint4(as_word(h01), as_word(h23), as_word(h01), as_word(h23));
+                *reinterpret_cast<uint4 *>(mins + sums_at(quad * 32 + lane, 1)) = make_uint4(as_word(l01), as_word(l23), 0u, 0u);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            } else {
+                uint32_t words[36];                             // four blocks of 9
+#pragma unroll
+                for (int x = 0; x < 9; x++) {
+                    const uint4 v = *reinterpret_cast<const uint4 *>(src + x * 16);
+                    words[4 * x] = v.x; words[4 * x + 1] = v.y; words[4 * x + 2] = v.z; words[4 * x + 3] = v.w;
+                }
+                const __half2 offset = __float2half2_rn(1152.f);
+#pragma unroll
+                for (int blk = 0; blk < 4; blk++) {
+                    uint32_t hi[16], lo[16];
+                    const __half2 d = __half2half2(__low2half(as_half2(words[blk * 9])));
+#pragma unroll
+                    for (int e = 0; e < 8; e++) {
+                        const uint32_t c = words[blk * 9 + 1 + e] ^ 0x80808080u;      // code + 128
+                        split_codes(__byte_perm(c, 0x64646464u, 0x4140), offset, d, hi[e * 2], lo[e * 2]);
+                        split_codes(__byte_perm(c, 0x64646464u, 0x4342), offset, d, hi[e * 2 + 1], lo[e * 2 + 1]);
+                    }
+                    tmem_st16(dst + blk * 16u, hi);
+                    tmem_st16(dst + 64u + blk * 16u, lo);
+                }
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();                                       // every lane has read its bytes and stored its weights
+            if (lane == 0) mbar_arrive(&sh.w_full[group]);
+            fetch();
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        tmem_free(tmem, 512);
+    }
+}
+
+// ------------------------------------------------------------------------------------------ workspace
+
+// Stream-ordered, so calls on different streams and threads never share a block; up to kKeep bytes stay with the pool
+// between calls, the rest goes back to the device.
+constexpr unsigned long long kKeep = 256ull << 20;
+cudaMemPool_t g_pool[64] = {};
+std::mutex g_pool_mu;
+
+cudaMemPool_t workspace_pool(int dev)
+{
+    if (dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    if (!g_pool[dev]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;          // the calling thread may be capturing: this is no part of it
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        unsigned long long keep = kKeep;
+        const bool ok = cudaMemPoolCreate(&pool, &props) == cudaSuccess && cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (!ok) { cudaGetLastError(); return nullptr; }
+        g_pool[dev] = pool;
+    }
+    return g_pool[dev];
+}
+
+template <int FMT, int PLANES>
+int launch_split(const SplitParams &p, uint32_t ctas, cudaStream_t stream)
+{
+    const size_t smem = 1024 + (size_t)kSlots * p.tok * 128 + (size_t)kScaleSlots * side_bytes(FMT, p.tok) + (size_t)kRaw * kCols * raw_bytes(FMT) +
+                        (FMT == MGQ_FMT_Q4 ? 2 * kMinBytes : 0);
+    if (int rc = allow_smem(gemm_split_kernel<FMT, PLANES>, smem)) return rc;
+    return launch(gemm_split_kernel<FMT, PLANES>, dim3(ctas), dim3(kSplitThreads), smem, stream, p);
+}
+
+}  // namespace
+
+// When there is no room for the workspace, nothing is launched for the rows from *done on.
+int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const float *addend, float *c,
+                      uint32_t m, uint32_t k, uint32_t n, void *stream_v, uint32_t *done)
+{
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    int dev = 0, sms = 0;
+    MGQ_CUDA(cudaGetDevice(&dev));
+    MGQ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    *done = 0;
+    cudaMemPool_t pool = workspace_pool(dev);
+    if (!pool) return MGQ_OK;
+    const bool bf16 = a_dtype == MGQ_A_BF16, q4 = fmt == MGQ_FMT_Q4;
+    const uint32_t planes = bf16 ? 1 : 2;
+    const size_t elem = bf16 ? 2 : 4;
+    uint32_t pass = kPassElems / k / kMaxTok * kMaxTok;
+    if (pass < kMaxTok) pass = kMaxTok;
+    for (uint32_t r0 = 0; r0 < m; r0 += *done - r0) {
+        SplitParams p{};
+        p.m = m - r0 < pass ? m - r0 : pass;
+        p.k = k; p.n = n; p.bpc = k / 32;
+        p.num_blocks = (unsigned long long)p.bpc * n;
+        p.w = static_cast<const uint8_t *>(w);
+        p.a = static_cast<const uint8_t *>(a) + (size_t)r0 * k * elem;
+        p.addend = addend ? addend + (size_t)r0 * n : nullptr;
+        p.c = c + (size_t)r0 * n;
+        // tiles of equal numbers of tokens, in steps of the MMA's 16
+        p.m_tiles = (p.m + kMaxTok - 1) / kMaxTok;
+        p.tok = ((p.m + p.m_tiles - 1) / p.m_tiles + 15) / 16 * 16;
+        p.m_tiles = (p.m + p.tok - 1) / p.tok;
+        p.chunks = (k + kChunk - 1) / kChunk;
+        const unsigned long long units = (unsigned long long)p.m_tiles * ((n + kCols - 1) / kCols) * p.chunks;
+        if (units >= (1ull << 31)) return MGQ_OK;
+        p.tiles = (uint32_t)(units / p.chunks);
+        p.units = (uint32_t)units;
+        // Q8: whole 16-byte pieces of 4 blocks; Q4: nibbles behind num_blocks header words
+        p.wide = q4 ? p.num_blocks % 4 == 0 : p.bpc % 4 == 0;
+        const uint32_t ctas = p.units / 2 < 1 ? 1 : p.units / 2 < (uint32_t)sms ? p.units / 2 : (uint32_t)sms;
+
+        const size_t plane_bytes = (size_t)p.m_tiles * p.chunks * 2 * planes * p.tok * 128;
+        const size_t all_side = ((size_t)p.m_tiles * p.chunks * side_bytes(fmt, p.tok) + 255) / 256 * 256;
+        const size_t part_bytes = (size_t)ctas * 2 * kMaxTok * kCols * 4;
+        uint8_t *ws = nullptr;
+        if (cudaMallocFromPoolAsync(reinterpret_cast<void **>(&ws), plane_bytes + all_side + part_bytes + (size_t)p.tiles * 4, pool, stream) != cudaSuccess) {
+            cudaGetLastError();
+            return MGQ_OK;
+        }
+        uint8_t *side_dev = ws + plane_bytes;
+        p.planes = ws;
+        p.side = side_dev;
+        p.partial = reinterpret_cast<float *>(side_dev + all_side);
+        p.counters = reinterpret_cast<unsigned int *>(side_dev + all_side + part_bytes);
+        const bool vec = reinterpret_cast<uintptr_t>(p.a) % 16 == 0;
+        const unsigned long long warps = (unsigned long long)p.m * p.chunks;
+        split_rows_kernel<<<(uint32_t)((warps + 7) / 8), 256, 0, stream>>>(p.a, bf16, vec, ws, side_dev, p.counters, p.tiles, p.m, k, p.tok, p.chunks, planes, q4);
+        int rc = cuda_check((int)cudaGetLastError(), "split_rows_kernel", __FILE__, __LINE__);
+        if (rc == MGQ_OK)
+            rc = q4 ? (bf16 ? launch_split<MGQ_FMT_Q4, 1>(p, ctas, stream) : launch_split<MGQ_FMT_Q4, 2>(p, ctas, stream))
+                    : (bf16 ? launch_split<MGQ_FMT_Q8, 1>(p, ctas, stream) : launch_split<MGQ_FMT_Q8, 2>(p, ctas, stream));
+        const int freed = cuda_check((int)cudaFreeAsync(ws, stream), "cudaFreeAsync", __FILE__, __LINE__);
+        if (rc != MGQ_OK) return rc;
+        if (freed != MGQ_OK) return freed;
+        *done = r0 + p.m;
+    }
+    return MGQ_OK;
+}
+
+int tc_device_status()
+{
+    unsigned int err = 0;
+    MGQ_CUDA(cudaMemcpyFromSymbol(&err, g_split_error, sizeof err));
+    if (err) {
+        const unsigned int zero = 0;
+        MGQ_CUDA(cudaMemcpyToSymbol(g_split_error, &zero, sizeof zero));
+        return fail(MGQ_ERR_TIMEOUT, "a bounded wait inside the tensor-core GEMM ran out");
+    }
+    return linear_tc_status();
+}
+
+}  // namespace mgq

@@ -48,10 +48,9 @@ bool force_tiled();
 int launch_gemm(int fmt, const void *a, int a_dtype, const void *w, const float *addend, float *c,
                 uint32_t m, uint32_t k, uint32_t n, void *stream);
 
-// Tensor-core GEMM (mgq_gemm_tc.cu): bf16 activations, M >= 64, K % 128 == 0.
-bool gemm_tc_eligible(int a_dtype, uint32_t m, uint32_t k, uint32_t n, const void *a);
-int launch_gemm_tc(int fmt, const void *a, const void *w, const float *addend, float *c,
-                   uint32_t m, uint32_t k, uint32_t n, void *stream);
+// Tensor-core GEMM with split operands (mgq_gemm_split.cu): any shape; rows from *done on are left when there is no room for its workspace.
+int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const float *addend, float *c,
+                      uint32_t m, uint32_t k, uint32_t n, void *stream, uint32_t *done);
 int tc_device_status();
 int linear_tc_status();               // mgq_linear_tc.cu
 

@@ -10,8 +10,10 @@
 //   warp 1      allocates TMEM, issues 4 tcgen05.mma (M=128, N=TN, K=16) per stage, commits the stage
 //               to empty[s] and the tile to acc_full[b].
 //   warps 2-5   epilogue of one accumulator while the other is being filled (2 x TN TMEM columns).
-// Every wait is bounded like in mgq_gemm_tc.cu.
+// Every mbarrier wait is bounded; when one runs out the device-wide error word is raised (mgq_device_status) and the roles end.
 #include <cuda_fp16.h>
+
+#include <mutex>
 
 #include "mgq_linear.cuh"
 #include "mgq_tcgen05.cuh"
@@ -322,6 +324,22 @@ int launch_tc_sized(const LinearGroup &g, cudaStream_t stream)
 }
 
 }  // namespace
+
+int encode_fn(EncodeTiledFn &out)
+{
+    static std::mutex mu;
+    static EncodeTiledFn cached = nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!cached) {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        MGQ_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres));
+        if (qres != cudaDriverEntryPointSuccess || !fn) return fail(MGQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+        cached = reinterpret_cast<EncodeTiledFn>(fn);
+    }
+    out = cached;
+    return MGQ_OK;
+}
 
 int launch_linear_tc(const LinearGroup &g, void *stream)
 {

@@ -122,6 +122,6 @@ __device__ __forceinline__ void tmem_free(uint32_t base, uint32_t columns)
 using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                   const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-int encode_fn(EncodeTiledFn &out);                 // mgq_gemm_tc.cu
+int encode_fn(EncodeTiledFn &out);                 // mgq_linear_tc.cu
 
 }  // namespace mgq

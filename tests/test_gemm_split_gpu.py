@@ -1,0 +1,139 @@
+"""The tensor-core GEMM with split operands: edges of its tiles and chunks, packed alignments, ranges, streams, capture.
+
+Tolerance 1e-6 (relative 2-norm): a chunk of 128 k takes at most 25 truncating steps of 2^-24 on an accumulator that grows with
+the root of the steps, so its sum is at most 25 * 2/3 * 2^-24 = 1e-6 off; chunks add up in quadrature, and so do their f32 sums.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from gpu_util import run_matmul, to_dev
+
+pytestmark = pytest.mark.gpu
+
+FMTS = [O.FMT_Q4, O.FMT_Q8]
+
+
+def _inputs(fmt, m, k, n, seed=0):
+    rng = np.random.Generator(np.random.PCG64(seed + m + k + n))
+    return O.synth_weights(fmt, k, n, seed=seed + 1), rng.standard_normal((m, k)).astype(np.float32)
+
+
+def _dense(fmt, w, k, n):
+    from meganeura_b200 import ops
+    return ops.dequantize(fmt, w, k, n).astype(np.float64)
+
+
+@pytest.mark.parametrize("act", ["f32", "bf16"])
+@pytest.mark.parametrize("fmt", FMTS)
+# tokens: one group of 16, one tile, two tiles, three; k: odd block counts, a chunk and one block, several chunks;
+# n: less than a tile, ragged, block counts of every remainder by 4
+@pytest.mark.parametrize("m,k,n", [(1, 160, 1), (16, 256, 128), (17, 288, 33), (128, 416, 127), (129, 608, 129), (257, 1056, 259), (300, 4128, 70), (40, 8192, 2048)])
+def test_edges(fmt, act, m, k, n):
+    import torch
+    from meganeura_b200 import ops
+    w, x = _inputs(fmt, m, k, n)
+    d = np.random.Generator(np.random.PCG64(3)).standard_normal((m, n)).astype(np.float32) if m % 2 else None
+    xd = torch.from_numpy(x).cuda()
+    if act == "bf16":
+        xd = xd.to(torch.bfloat16)
+        x = xd.float().cpu().numpy()
+    got = run_matmul(fmt, xd, w, k, n, addend=d, route="gemm")
+    ops.device_status()
+    want = x.astype(np.float64) @ _dense(fmt, w, k, n) + (0.0 if d is None else d)
+    assert O.rel_l2(got, want) <= 1e-6
+
+
+def test_unaligned_activations():
+    import torch
+    from meganeura_b200 import ops
+    m, k, n = 33, 320, 65
+    w, x = _inputs(O.FMT_Q4, m, k, n)
+    for dtype in (torch.float32, torch.bfloat16):
+        buf = torch.zeros(m * k + 1, device="cuda", dtype=dtype)
+        a = buf[1:].reshape(m, k)
+        a.copy_(torch.from_numpy(x))
+        got = ops.matmul(O.FMT_Q4, a, to_dev(w), k, n, route="gemm").cpu().numpy()
+        assert O.rel_l2(got, a.float().cpu().numpy().astype(np.float64) @ _dense(O.FMT_Q4, w, k, n)) <= 1e-6
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+def test_ranges_of_rows(fmt):
+    # rows of very different magnitude, and one whose chunks differ by 10^20: each keeps its own relative accuracy
+    m, k, n = 20, 512, 130
+    w, x = _inputs(fmt, m, k, n)
+    x *= (10.0 ** np.linspace(-30, 30, m)).astype(np.float32)[:, None]
+    x[7, :] = x[8, :]
+    x[7, 128:] *= np.float32(1e-20)
+    x[3] = 0
+    got = run_matmul(fmt, x, w, k, n, route="gemm")
+    want = x.astype(np.float64) @ _dense(fmt, w, k, n)
+    for r in range(m):
+        assert np.linalg.norm(got[r] - want[r]) <= 1e-6 * np.linalg.norm(want[r])
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+def test_not_finite_and_large_scales_as_in_plain_f32(fmt):
+    import torch
+    from meganeura_b200 import ops
+    m, k, n = 40, 384, 140
+    w, x = _inputs(fmt, m, k, n)
+    w = w.copy()
+    x[3, 17], x[5, 200], x[9, 300] = np.inf, -np.inf, np.nan
+    x[11, 5], x[11, 6] = np.inf, -np.inf
+    x[13] = 3e38
+    scales = w[:4 * (k // 32) * n].view(np.float16)[0::2] if fmt == O.FMT_Q4 else w.reshape(-1, 36)[:, :2].copy().view(np.float16)[:, 0]
+    big = {4: 60000.0, 70: np.inf, 139: 700.0}                # columns
+    for col, value in big.items():
+        scales[col * (k // 32) + 2] = value
+    if fmt == O.FMT_Q8:
+        w.reshape(-1, 36)[:, :2] = scales[:, None].view(np.uint8).reshape(-1, 2)
+    xd, wd = to_dev(x), to_dev(w)
+    got = ops.matmul(fmt, xd, wd, k, n, route="gemm")
+    ops.set_option("gemm.force_tiled", 1)
+    try:
+        plain = ops.matmul(fmt, xd, wd, k, n, route="gemm")
+    finally:
+        ops.set_option("gemm.force_tiled", 0)
+    got, plain = got.cpu().numpy(), plain.cpu().numpy()
+    finite = np.isfinite(plain)
+    assert np.array_equal(np.isnan(got), np.isnan(plain)) and np.array_equal(np.isposinf(got), np.isposinf(plain)) and np.array_equal(np.isneginf(got), np.isneginf(plain))
+    assert (np.abs(got[finite] - plain[finite]) <= 1e-4 * np.abs(plain[finite]).max(initial=0.0)).all()
+    ordinary = [r for r in range(m) if r not in (3, 5, 9, 11, 13)]
+    cols = [c for c in range(n) if c not in big]
+    assert O.rel_l2(got[np.ix_(ordinary, cols)], plain[np.ix_(ordinary, cols)]) <= 2e-6
+
+
+def test_two_streams_at_once():
+    import torch
+    from meganeura_b200 import ops
+    shapes = [(O.FMT_Q4, 300, 1536, 2048), (O.FMT_Q8, 60, 4096, 512)]
+    work = []
+    for i, (fmt, m, k, n) in enumerate(shapes):
+        w, x = _inputs(fmt, m, k, n, seed=i)
+        xd, wd = to_dev(x), to_dev(w)
+        work.append((fmt, xd, wd, k, n, ops.matmul(fmt, xd, wd, k, n, route="gemm"), torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    outs = []
+    for _ in range(10):
+        for fmt, xd, wd, k, n, want, stream in work:
+            with torch.cuda.stream(stream):
+                outs.append((ops.matmul(fmt, xd, wd, k, n, route="gemm", stream=stream), want))
+    torch.cuda.synchronize()
+    assert all(torch.equal(got, want) for got, want in outs)          # sums do not depend on timing
+
+
+def test_captured_in_a_graph():
+    import torch
+    from meganeura_b200 import ops
+    fmt, m, k, n = O.FMT_Q4, 50, 1024, 300
+    w, x = _inputs(fmt, m, k, n)
+    xd, wd, out = to_dev(x), to_dev(w), torch.zeros((m, n), device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.matmul(fmt, xd, wd, k, n, out=out, route="gemm")
+    for seed in range(3):
+        xd.copy_(torch.from_numpy(_inputs(fmt, m, k, n, seed=seed)[1]))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, ops.matmul(fmt, xd, wd, k, n, route="gemm"))

@@ -1,4 +1,4 @@
-"""The tcgen05/TMEM GEMM (bf16 activations, M >= 64, K % 128 == 0) against the oracle."""
+"""The tcgen05/TMEM GEMM with bf16 activations against the oracle."""
 import numpy as np
 import pytest
 
