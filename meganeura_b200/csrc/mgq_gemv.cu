@@ -631,7 +631,10 @@ int launch_all_gather(const float *slice, const void *push_dev, const void *loca
 bool gemv_streamable(const void *x, uint32_t k, uint32_t n)
 {
     const uint32_t bpc = k / 32;
-    return bpc >= 8 && bpc <= 1024 && (((unsigned long long)bpc * n) % 4 == 0) && (reinterpret_cast<uintptr_t>(x) % 16 == 0);
+    if (bpc < 8 || bpc > 1024) return false;
+    // a group of columns has to fit a CTA; with block counts that are not multiples of 4 groups of 2 or 4 columns are needed
+    if (columns_for(bpc <= 256 ? 256u : (bpc + 31u) & ~31u, bpc) == 0) return false;
+    return ((unsigned long long)bpc * n) % 4 == 0 && (reinterpret_cast<uintptr_t>(x) % 16 == 0);
 }
 
 int launch_gemv(int fmt, const float *x, const void *w, const float *addend, float *y,

@@ -155,3 +155,14 @@ def test_subnormal_scales_follow_cpu_dequantize(coracle):
     got = run_matmul(O.FMT_Q8, x, w, k, n, route="gemv")
     check_against_oracle(coracle, O.FMT_Q8, x, w, k, n, got)
     assert np.abs(got).max() > 0
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+@pytest.mark.parametrize("route", ["gemv", "auto"])
+# block counts that are not multiples of 4 and so large that no group of 2 or 4 columns fits a CTA (65, 130, 275), and the last ones that do
+@pytest.mark.parametrize("m,k,n", [(1, 2080, 12), (2, 2016, 36), (1, 4160, 66), (2, 4096 - 64, 34), (4, 8800, 40), (3, 2080, 7)])
+def test_block_counts_that_no_column_group_fits(coracle, fmt, route, m, k, n):
+    w = O.synth_weights(fmt, k, n, seed=k + n)
+    x = _x(m, k, k * 7 + n)
+    got = run_matmul(fmt, x, w, k, n, route=route)
+    check_against_oracle(coracle, fmt, x, w, k, n, got)
