@@ -7,8 +7,8 @@
 //
 //   linear_gemv_kernel   M <= 8: HBM-bound, a warp streams R weight rows with 16-byte loads for all M
 //                        activation rows at once (every weight byte is read once per 8 rows).
-//   linear_tiled_kernel  general: 64x64 register tiles in true f32 (f32 activations, sizes the tensor
-//                        cores cannot take).
+//   linear_tiled_kernel  general: 64x64 register tiles in true f32, K split over clusters (f32 activations, sizes
+//                        the tensor cores cannot take).
 //   mgq_linear_tc.cu     M > 8, bf16 activations: tcgen05.
 #include "mgq_linear.cuh"
 
@@ -154,92 +154,222 @@ int launch_gemv_typed(const LinearGroup &g, bool vec, cudaStream_t stream)
 }
 
 // ---------------------------------------------------------------- general tiled kernel (CUDA cores, f32)
-constexpr int BM = 64, BN = 64, BK = 16;
+// A tile of 8 RM rows x 64 columns per CTA, RM x 4 values per thread, true f32 products and sums.  Few rows make few tiles (100 x 1024
+// outputs are 32), so K is shared out over a cluster of up to 8 CTAs whose partial sums meet in rank order through distributed
+// shared memory; a rank finishes the rows of its share.  The next 32 k are requested while the current ones are multiplied.
+// Bound by the issue of multiply-adds (two per instruction) once the SMs are full.
+// A prompt of 100 tokens and 3 single ones of a 2-layer f32 Tobovik of width 1024: 2829 us with one CTA per tile and 16 k per
+// step, 1160 us so.
+constexpr int BN = 64, BK = 32;
 
-template <typename XT, bool GLU>
-__global__ void __launch_bounds__(256) linear_tiled_kernel(const __grid_constant__ LinearGroup g)
+__device__ __forceinline__ float4 cluster_load4(const float *p, uint32_t rank)
 {
-    __shared__ float s_a[BK][BM + 4], s_w[GLU ? 2 : 1][BK][BN + 4];
+    uint32_t addr;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
+// (c0, c1) += a * (w0, w1), each rounded as by fmaf.
+__device__ __forceinline__ void fma_pair(float &c0, float &c1, float a, float w0, float w1)
+{
+    asm("{\n\t.reg .b64 c, a, w;\n\t"
+        "mov.b64 c, {%0, %1};\n\tmov.b64 a, {%2, %2};\n\tmov.b64 w, {%3, %4};\n\t"
+        "fma.rn.f32x2 c, a, w, c;\n\t"
+        "mov.b64 {%0, %1}, c;\n\t}"
+        : "+f"(c0), "+f"(c1) : "f"(a), "f"(w0), "f"(w1));
+}
+
+__device__ __forceinline__ void load4(const float *p, float (&v)[4])
+{
+    const float4 q = *reinterpret_cast<const float4 *>(p);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+}
+__device__ __forceinline__ void load4(const __nv_bfloat16 *p, float (&v)[4])
+{
+    const uint2 q = *reinterpret_cast<const uint2 *>(p);
+    v[0] = __uint_as_float(q.x << 16); v[1] = __uint_as_float(q.x & 0xFFFF0000u);
+    v[2] = __uint_as_float(q.y << 16); v[3] = __uint_as_float(q.y & 0xFFFF0000u);
+}
+
+template <bool GLU>
+__device__ __forceinline__ void finish_value(const LinearGroup &g, const LinearSegment &s, uint32_t row, uint32_t n, float y, float up)
+{
+    if (row >= g.m || n >= s.n) return;
+    const size_t o = (size_t)row * s.n + n;
+    if (GLU) {
+        y = glu_f(y + (s.bias ? s.bias[n] : 0.f), up + (s.bias ? s.bias2[n] : 0.f), g.act);
+        if (g.out_bf16) static_cast<__nv_bfloat16 *>(s.out)[o] = __float2bfloat16_rn(y);
+        else            static_cast<float *>(s.out)[o] = y;
+        return;
+    }
+    if (s.bias) y += s.bias[n];
+    if (s.addend) y += s.addend[o];
+    static_cast<float *>(s.out)[o] = y;
+}
+
+// grid: column tiles of all layers x (row tiles * splits); a cluster is the splits of a tile.
+template <typename XT, bool GLU, int RM>
+__global__ void __launch_bounds__(128) linear_tiled_kernel(const __grid_constant__ LinearGroup g, uint32_t splits, bool vec)
+{
+    constexpr int BM = 8 * RM, U = GLU ? 2 : 1, LA = BM + 4, LW = BN + 4;
+    constexpr int kStage = BK * LA + U * BK * LW, kPart = U * BM * LW;
+    __shared__ __align__(16) float buf[kStage > kPart ? kStage : kPart];
+    float *s_a = buf, *s_w = buf + BK * LA;                    // [k][row], [weight][k][column]
     uint32_t tile = blockIdx.x, si = 0;
     pdl_launch_dependents();
-    while (si < g.count) {
+    while (si + 1 < g.count) {
         const uint32_t tiles = (g.seg[si].n + BN - 1) / BN;
         if (tile < tiles) break;
         tile -= tiles;
         si++;
     }
-    if (si >= g.count) return;
     const LinearSegment &s = g.seg[si];
-    const uint32_t n0 = tile * BN, m0 = blockIdx.y * BM, k = s.k, t = threadIdx.x;
+    const uint32_t rank = blockIdx.y % splits;
+    const uint32_t n0 = tile * BN, m0 = blockIdx.y / splits * BM, k = s.k, t = threadIdx.x;
     const uint32_t tx = t & 15u, ty = t >> 4;
+    const uint32_t share = (k + splits * BK - 1) / (splits * BK) * BK, k_begin = min(k, rank * share), k_end = min(k, k_begin + share);
     const XT *a = static_cast<const XT *>(s.a);
-    const __nv_bfloat16 *w = static_cast<const __nv_bfloat16 *>(s.w), *w2 = static_cast<const __nv_bfloat16 *>(s.w2);
-    float acc[GLU ? 2 : 1][4][4];
+    const __nv_bfloat16 *w[U] = {};
+    w[0] = static_cast<const __nv_bfloat16 *>(s.w);
+    if (GLU) w[U - 1] = static_cast<const __nv_bfloat16 *>(s.w2);
+    constexpr int NA = BM * (BK / 4) / 128, NW = BN * (BK / 8) / 128;
+    float ra[NA][4];
+    uint4 rw[U][NW];
+    auto fetch = [&](uint32_t k0) {                            // zeros beyond the matrix and beyond this rank's share
 #pragma unroll
-    for (int u = 0; u < (GLU ? 2 : 1); u++)
+        for (int i = 0; i < NA; i++) {
+            const uint32_t e = t + 128u * i, row = m0 + e % BM, kk = k0 + e / BM * 4;
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+            for (int x = 0; x < 4; x++) ra[i][x] = 0.f;
+            if (row < g.m && kk < k_end) {
+                const XT *p = a + (size_t)row * k + kk;
+                if (vec) load4(p, ra[i]);
+                else
+#pragma unroll
+                    for (int x = 0; x < 4; x++)
+                        if (kk + x < k_end) ra[i][x] = to_f32(p[x]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int i = 0; i < NW; i++) {
+                const uint32_t e = t + 128u * i, n = n0 + e % BN, kk = k0 + e / BN * 8;
+                rw[u][i] = make_uint4(0, 0, 0, 0);
+                if (n < s.n && kk < k_end) {
+                    const __nv_bfloat16 *p = w[u] + (size_t)n * k + kk;
+                    if (vec) rw[u][i] = __ldg(reinterpret_cast<const uint4 *>(p));
+                    else {
+                        uint32_t v[8];
+#pragma unroll
+                        for (int x = 0; x < 8; x++) v[x] = kk + x < k_end ? (uint32_t)__bfloat16_as_ushort(p[x]) : 0u;
+                        rw[u][i] = make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16);
+                    }
+                }
+            }
+    };
+    float acc[U][RM][4];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+        for (int i = 0; i < RM; i++)
 #pragma unroll
             for (int j = 0; j < 4; j++) acc[u][i][j] = 0.f;
     pdl_wait();
-    for (uint32_t k0 = 0; k0 < k; k0 += BK) {
+    fetch(k_begin);
+    for (uint32_t k0 = k_begin; k0 < k_end; k0 += BK) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint32_t e = t + 256u * i, row = e / BK, kk = e % BK;
-            const bool in_k = k0 + kk < k;
-            s_a[kk][row] = in_k && m0 + row < g.m ? to_f32(a[(size_t)(m0 + row) * k + k0 + kk]) : 0.f;
-            const bool in_w = in_k && n0 + row < s.n;
-            s_w[0][kk][row] = in_w ? __bfloat162float(w[(size_t)(n0 + row) * k + k0 + kk]) : 0.f;
-            if (GLU) s_w[GLU ? 1 : 0][kk][row] = in_w ? __bfloat162float(w2[(size_t)(n0 + row) * k + k0 + kk]) : 0.f;
+        for (int i = 0; i < NA; i++) {
+            const uint32_t e = t + 128u * i;
+#pragma unroll
+            for (int x = 0; x < 4; x++) s_a[(e / BM * 4 + x) * LA + e % BM] = ra[i][x];
         }
-        __syncthreads();
 #pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int i = 0; i < NW; i++) {
+                const uint32_t e = t + 128u * i;
+                float v[8];
+                unpack8(rw[u][i], v);
+#pragma unroll
+                for (int x = 0; x < 8; x++) s_w[(u * BK + e / BN * 8 + x) * LW + e % BN] = v[x];
+            }
+        __syncthreads();
+        if (k0 + BK < k_end) fetch(k0 + BK);
+#pragma unroll 8
         for (int kk = 0; kk < BK; kk++) {
-            const float4 av = *reinterpret_cast<const float4 *>(&s_a[kk][ty * 4]);
-            const float ar[4] = {av.x, av.y, av.z, av.w};
+            float ar[RM];
 #pragma unroll
-            for (int u = 0; u < (GLU ? 2 : 1); u++) {
-                const float4 wv = *reinterpret_cast<const float4 *>(&s_w[u][kk][tx * 4]);
-                const float wr[4] = {wv.x, wv.y, wv.z, wv.w};
+            for (int i = 0; i < RM; i += 4) {
+                const float4 v = *reinterpret_cast<const float4 *>(s_a + kk * LA + ty * RM + i);
+                ar[i] = v.x; ar[i + 1] = v.y; ar[i + 2] = v.z; ar[i + 3] = v.w;
+            }
 #pragma unroll
-                for (int i = 0; i < 4; i++)
+            for (int u = 0; u < U; u++) {
+                const float4 v = *reinterpret_cast<const float4 *>(s_w + (u * BK + kk) * LW + tx * 4);
 #pragma unroll
-                    for (int j = 0; j < 4; j++) acc[u][i][j] = fmaf(ar[i], wr[j], acc[u][i][j]);
+                for (int i = 0; i < RM; i++) {
+                    fma_pair(acc[u][i][0], acc[u][i][1], ar[i], v.x, v.y);
+                    fma_pair(acc[u][i][2], acc[u][i][3], ar[i], v.z, v.w);
+                }
             }
         }
         __syncthreads();
     }
+    if (splits == 1) {
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const uint32_t row = m0 + ty * 4 + i;
-        if (row >= g.m) break;
+        for (int i = 0; i < RM; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint32_t n = n0 + tx * 4 + j;
-            if (n >= s.n) break;
-            const size_t o = (size_t)row * s.n + n;
-            float y = acc[0][i][j];
-            if (GLU) {
-                y = glu_f(y + (s.bias ? s.bias[n] : 0.f), acc[GLU ? 1 : 0][i][j] + (s.bias ? s.bias2[n] : 0.f), g.act);
-                if (g.out_bf16) static_cast<__nv_bfloat16 *>(s.out)[o] = __float2bfloat16_rn(y);
-                else            static_cast<float *>(s.out)[o] = y;
-                continue;
-            }
-            if (s.bias) y += s.bias[n];
-            if (s.addend) y += s.addend[o];
-            static_cast<float *>(s.out)[o] = y;
-        }
+            for (int j = 0; j < 4; j++) finish_value<GLU>(g, s, m0 + ty * RM + i, n0 + tx * 4 + j, acc[0][i][j], acc[U - 1][i][j]);
+        return;
     }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+        for (int i = 0; i < RM; i++) *reinterpret_cast<float4 *>(buf + (u * BM + ty * RM + i) * LW + tx * 4) = make_float4(acc[u][i][0], acc[u][i][1], acc[u][i][2], acc[u][i][3]);
+    cluster_sync();
+    const uint32_t rows = BM / splits;
+    for (uint32_t e = t; e < rows * 16; e += 128) {
+        const uint32_t row = rank * rows + e / 16, col = e % 16 * 4;
+        float4 sum[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            sum[u] = cluster_load4(buf + (u * BM + row) * LW + col, 0);
+            for (uint32_t r = 1; r < splits; r++) {
+                const float4 v = cluster_load4(buf + (u * BM + row) * LW + col, r);
+                sum[u].x += v.x; sum[u].y += v.y; sum[u].z += v.z; sum[u].w += v.w;
+            }
+        }
+        finish_value<GLU>(g, s, m0 + row, n0 + col, sum[0].x, sum[U - 1].x);
+        finish_value<GLU>(g, s, m0 + row, n0 + col + 1, sum[0].y, sum[U - 1].y);
+        finish_value<GLU>(g, s, m0 + row, n0 + col + 2, sum[0].z, sum[U - 1].z);
+        finish_value<GLU>(g, s, m0 + row, n0 + col + 3, sum[0].w, sum[U - 1].w);
+    }
+    cluster_sync();                                            // the others may still read this CTA's sums
+}
+
+template <typename XT, bool GLU, int RM>
+int launch_tiled_rows(const LinearGroup &g, bool vec, cudaStream_t stream)
+{
+    uint32_t tiles = 0, k = 0;
+    for (uint32_t i = 0; i < g.count; i++) {
+        tiles += (g.seg[i].n + BN - 1) / BN;
+        k = max(k, g.seg[i].k);
+    }
+    const uint32_t row_tiles = (g.m + 8 * RM - 1) / (8 * RM);
+    // four CTAs per SM, as long as each has 128 k left to sum
+    uint32_t splits = 1;
+    while (splits < 8 && tiles * row_tiles * splits * 2 <= 4 * 148 && k / (splits * 2) >= 128) splits *= 2;
+    return launch_clustered(linear_tiled_kernel<XT, GLU, RM>, dim3(tiles, row_tiles * splits), dim3(128), splits, 0, stream, g, splits, vec);
 }
 
 template <typename XT>
-int launch_tiled_typed(const LinearGroup &g, cudaStream_t stream)
+int launch_tiled_typed(const LinearGroup &g, bool vec, cudaStream_t stream)
 {
-    uint32_t tiles = 0;
-    for (uint32_t i = 0; i < g.count; i++) tiles += (g.seg[i].n + BN - 1) / BN;
-    const dim3 grid(tiles, (g.m + BM - 1) / BM);
-    if (g.glu) return launch(linear_tiled_kernel<XT, true>, grid, dim3(256), 0, stream, g);
-    return launch(linear_tiled_kernel<XT, false>, grid, dim3(256), 0, stream, g);
+    if (g.m <= 32) return g.glu ? launch_tiled_rows<XT, true, 4>(g, vec, stream) : launch_tiled_rows<XT, false, 4>(g, vec, stream);
+    return g.glu ? launch_tiled_rows<XT, true, 8>(g, vec, stream) : launch_tiled_rows<XT, false, 8>(g, vec, stream);
 }
 
 int g_linear_force_tiled = 0;      // "linear.force_tiled"
@@ -270,7 +400,7 @@ int launch_linear_group(const LinearGroup &g, void *stream_v)
     }
     if (g.m <= 8) return g.a_bf16 ? launch_gemv_typed<__nv_bfloat16>(g, vec, stream) : launch_gemv_typed<float>(g, vec, stream);
     if (g.a_bf16 && vec && !g_linear_force_tiled) return launch_linear_tc(g, stream_v);
-    return g.a_bf16 ? launch_tiled_typed<__nv_bfloat16>(g, stream) : launch_tiled_typed<float>(g, stream);
+    return g.a_bf16 ? launch_tiled_typed<__nv_bfloat16>(g, vec, stream) : launch_tiled_typed<float>(g, vec, stream);
 }
 
 }  // namespace mgq
