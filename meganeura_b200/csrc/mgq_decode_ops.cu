@@ -183,12 +183,16 @@ __global__ void swiglu_kernel(const float *gate, const float *up, float *out, ui
 // last merges the partials -- the same online-softmax algebra, applied across chunks.
 constexpr int kChunk = 64;
 constexpr int kMaxGroup = 8;          // query heads per KV head
+// Latency bounds a CTA's chunk: 8 warps (4 before) halve the scores' and the weighted sums' chains, and four weights come with one
+// load.  A decode step of 8 layers with 32 / 8 heads of 128 behind 2048 positions: 581 -> 513 us, SmolLM2-135M behind 128: 1118 -> 1006 us.
+constexpr int kAttThreads = 256;
+constexpr int kAttWarps = kAttThreads / 32;
 
 // The last CTA of a KV head merges the chunk partials: out[g, d] = sum_c w_c acc_c[g, d] / sum_c w_c l_c
 // with w_c = exp(m_c - max_c m_c).  Every global round trip costs ~1 us here (the partials sit in
 // L2, written by other SMs), so the loads are arranged to need few of them: the first batch of
 // accumulator loads is issued before the maxima and sums are even known, and each thread keeps
-// NOUT x BATCH independent loads in flight (thread t owns outputs t + 128 j).
+// NOUT x BATCH independent loads in flight (thread t owns outputs t + kAttThreads j).
 template <int D, int NOUT, int BATCH>
 __device__ __forceinline__ void merge_partials(const float *base, uint32_t live, uint32_t group, float *s_w, float *out)
 {
@@ -199,7 +203,7 @@ __device__ __forceinline__ void merge_partials(const float *base, uint32_t live,
     auto fetch = [&](uint32_t c0) {
 #pragma unroll
         for (int j = 0; j < NOUT; j++) {
-            const uint32_t i = t + 128u * j;
+            const uint32_t i = t + (uint32_t)kAttThreads * j;
             const float *col = base + (size_t)(i / D) * (D + 2) + i % D;
 #pragma unroll
             for (int u = 0; u < BATCH; u++) v[j][u] = (i < total && c0 + u < live) ? __ldcg(col + (c0 + u) * cstride) : 0.f;
@@ -209,7 +213,7 @@ __device__ __forceinline__ void merge_partials(const float *base, uint32_t live,
     for (int j = 0; j < NOUT; j++) acc[j] = 0.f;
     fetch(0);
     // chunk weights into shared memory ([group][kChunk]; at most kChunk chunks, checked at launch)
-    for (uint32_t g = warp; g < group; g += 4) {
+    for (uint32_t g = warp; g < group; g += kAttWarps) {
         float mc[2], lc[2];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
@@ -236,14 +240,14 @@ __device__ __forceinline__ void merge_partials(const float *base, uint32_t live,
         if (c0) fetch(c0);
 #pragma unroll
         for (int j = 0; j < NOUT; j++) {
-            const uint32_t g = min((t + 128u * j) / D, (uint32_t)kMaxGroup - 1u);
+            const uint32_t g = min((t + (uint32_t)kAttThreads * j) / D, (uint32_t)kMaxGroup - 1u);
 #pragma unroll
             for (int u = 0; u < BATCH; u++) acc[j] = fmaf(v[j][u], c0 + u < live ? s_w[g * kChunk + c0 + u] : 0.f, acc[j]);
         }
     }
 #pragma unroll
     for (int j = 0; j < NOUT; j++) {
-        const uint32_t i = t + 128u * j;
+        const uint32_t i = t + (uint32_t)kAttThreads * j;
         if (i < total) out[i] = acc[j] * s_inv[i / D];
     }
 }
@@ -260,8 +264,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // Dynamic shared memory: the chunk's K rows, then its V rows ([kChunk][D] floats each).  Both tiles
 // are requested with cp.async up front, so a CTA has its whole 64 KB (D = 128) in flight at once
 // instead of paying a memory round trip per position.
-template <int D, int G2>              // head_dim: 64 or 128; G2: query heads per KV head rounded up to 4 or 8; blockDim.x == 128
-__global__ void __launch_bounds__(128) cached_attention_kernel(const float *q, const float *k_cache, const float *v_cache,
+template <int D, int G2>              // head_dim: 64 or 128; G2: query heads per KV head rounded up to 4 or 8
+__global__ void __launch_bounds__(kAttThreads) cached_attention_kernel(const float *q, const float *k_cache, const float *v_cache,
                                                                const uint32_t *kv_pos, float *out, uint32_t num_heads,
                                                                uint32_t num_kv_heads, uint32_t max_seq, float *workspace,
                                                                unsigned int *counters)
@@ -270,9 +274,9 @@ __global__ void __launch_bounds__(128) cached_attention_kernel(const float *q, c
     constexpr int PPW = 32 / LPP;                 // positions per warp step
     extern __shared__ __align__(16) float s_tiles[];
     float *s_k = s_tiles, *s_v = s_tiles + kChunk * D;
-    __shared__ float s_score[kMaxGroup][kChunk];
+    __shared__ __align__(16) float s_score[kMaxGroup][kChunk];
     __shared__ float s_q[kMaxGroup][D];
-    __shared__ float s_acc[128 / D][kMaxGroup][D];
+    __shared__ float s_acc[kAttThreads / D][kMaxGroup][D];
     __shared__ bool s_last;
     const uint32_t kvh = blockIdx.x, chunk = blockIdx.y, splits = gridDim.y;
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
@@ -286,17 +290,17 @@ __global__ void __launch_bounds__(128) cached_attention_kernel(const float *q, c
 
     if (p0 < kv_len) {
         const uint32_t rows = p1 - p0;
-        for (uint32_t i = t; i < rows * LPP; i += 128) {
+        for (uint32_t i = t; i < rows * LPP; i += kAttThreads) {
             const uint32_t r = i / LPP, c = i % LPP;
             cp_async16(s_k + r * D + c * 4, k_cache + (size_t)(p0 + r) * kv_dim + kvh * D + c * 4);
         }
         cp_async_commit();
-        for (uint32_t i = t; i < rows * LPP; i += 128) {
+        for (uint32_t i = t; i < rows * LPP; i += kAttThreads) {
             const uint32_t r = i / LPP, c = i % LPP;
             cp_async16(s_v + r * D + c * 4, v_cache + (size_t)(p0 + r) * kv_dim + kvh * D + c * 4);
         }
         cp_async_commit();
-        for (uint32_t i = t; i < group * D; i += 128) s_q[i / D][i % D] = q[(size_t)kvh * group * D + i];
+        for (uint32_t i = t; i < group * D; i += kAttThreads) s_q[i / D][i % D] = q[(size_t)kvh * group * D + i];
         cp_async_wait<1>();
         __syncthreads();
         // scores: PPW positions per warp step, LPP lanes per position.  The query slices stay in
@@ -312,7 +316,7 @@ __global__ void __launch_bounds__(128) cached_attention_kernel(const float *q, c
         uint32_t my_head = 0;
 #pragma unroll
         for (int keep = G2 / 2, off = LPP / 2; keep >= 1; keep >>= 1, off >>= 1) my_head = my_head * 2u + ((li & off) ? 1u : 0u);
-        for (uint32_t r = warp * PPW + sub; r < (uint32_t)kChunk; r += 4 * PPW) {
+        for (uint32_t r = warp * PPW + sub; r < (uint32_t)kChunk; r += kAttWarps * PPW) {
             float v[G2];
             if (r < rows) {
                 const float4 kv = *reinterpret_cast<const float4 *>(s_k + r * D + li * 4);
@@ -337,8 +341,8 @@ __global__ void __launch_bounds__(128) cached_attention_kernel(const float *q, c
             if ((li & (LPP / G2 - 1)) == 0 && my_head < group) s_score[my_head][r] = r < rows ? v[0] * scale : -FLT_MAX;
         }
         __syncthreads();
-        // per head: chunk maximum and exponentials (warp w takes heads w, w+4)
-        for (uint32_t g = warp; g < group; g += 4) {
+        // per head: chunk maximum and exponentials (a warp per head)
+        for (uint32_t g = warp; g < group; g += kAttWarps) {
             float m = fmaxf(s_score[g][lane], s_score[g][lane + 32]);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -351,28 +355,34 @@ __global__ void __launch_bounds__(128) cached_attention_kernel(const float *q, c
         }
         cp_async_wait<0>();
         __syncthreads();
-        // weighted V: thread <-> (position slice, dim); 128 / D slices
-        const uint32_t d = t % D, slice = t / D;
-        constexpr uint32_t SL = 128 / D;
-        float acc[kMaxGroup];
+        // weighted V: thread <-> (position slice, dim).  A slice is a run of positions, so that four weights of a head come
+        // with one load; rows beyond the chunk's end have weight 0 and are not read.
+        constexpr uint32_t SL = kAttThreads / D, RUN = kChunk / SL;
+        const uint32_t d = t % D, slice = t / D, r0 = slice * RUN;
+        float acc[G2];
 #pragma unroll
-        for (int g = 0; g < kMaxGroup; g++) acc[g] = 0.f;
-        for (uint32_t r = slice; r < rows; r += SL) {
-            const float v = s_v[r * D + d];
+        for (int g = 0; g < G2; g++) acc[g] = 0.f;
+#pragma unroll 2
+        for (uint32_t r = r0; r < min(rows, r0 + RUN); r += 4) {
+            float v[4];
 #pragma unroll
-            for (int g = 0; g < kMaxGroup; g++)
-                if (g < (int)group) acc[g] = fmaf(s_score[g][r], v, acc[g]);
+            for (int e = 0; e < 4; e++) v[e] = r + e < rows ? s_v[(r + e) * D + d] : 0.f;
+#pragma unroll
+            for (int g = 0; g < G2; g++)
+                if (g < (int)group) {
+                    const float4 w = *reinterpret_cast<const float4 *>(&s_score[g][r]);
+                    acc[g] = fmaf(w.w, v[3], fmaf(w.z, v[2], fmaf(w.y, v[1], fmaf(w.x, v[0], acc[g]))));
+                }
         }
 #pragma unroll
-        for (int g = 0; g < kMaxGroup; g++)
+        for (int g = 0; g < G2; g++)
             if (g < (int)group) s_acc[slice][g][d] = acc[g];
         __syncthreads();
-        if (slice == 0) {
-            for (uint32_t g = 0; g < group; g++) {
-                float a = s_acc[0][g][d];
-                if (SL > 1) a += s_acc[SL - 1][g][d];
-                part[g * (D + 2) + d] = a;
-            }
+        for (uint32_t i = t; i < group * D; i += kAttThreads) {
+            float a = s_acc[0][i / D][i % D];
+#pragma unroll
+            for (uint32_t x = 1; x < SL; x++) a += s_acc[x][i / D][i % D];
+            part[i / D * (D + 2) + i % D] = a;
         }
     }
     // the last CTA of this KV head merges
@@ -388,8 +398,8 @@ __global__ void __launch_bounds__(128) cached_attention_kernel(const float *q, c
     __threadfence();
     const uint32_t live = (kv_len + kChunk - 1) / kChunk;
     const float *base = workspace + (size_t)kvh * splits * kMaxGroup * (D + 2);
-    if (group * D <= 4 * 128) merge_partials<D, 4, 16>(base, live, group, &s_score[0][0], out + (size_t)kvh * group * D);
-    else                      merge_partials<D, kMaxGroup, 8>(base, live, group, &s_score[0][0], out + (size_t)kvh * group * D);
+    if (group * D <= 2 * kAttThreads) merge_partials<D, 2, 16>(base, live, group, &s_score[0][0], out + (size_t)kvh * group * D);
+    else                             merge_partials<D, kMaxGroup * D / kAttThreads, 16>(base, live, group, &s_score[0][0], out + (size_t)kvh * group * D);
 }
 
 // ---------------------------------------------------------------- greedy pick
@@ -523,7 +533,7 @@ int launch_cached_attention(const float *q, const float *k_cache, const float *v
     const size_t tiles = (size_t)2 * kChunk * head_dim * sizeof(float);
     const bool small_group = num_heads / num_kv_heads <= 4;
     if (head_dim == 64)
-        return launch(small_group ? cached_attention_kernel<64, 4> : cached_attention_kernel<64, 8>, grid, dim3(128), tiles, st, q, k_cache,
+        return launch(small_group ? cached_attention_kernel<64, 4> : cached_attention_kernel<64, 8>, grid, dim3(kAttThreads), tiles, st, q, k_cache,
                       v_cache, kv_pos, out, num_heads, num_kv_heads, max_seq, partials, counters);
     if (head_dim == 128) {
         static bool opted_in[64] = {};
@@ -534,7 +544,7 @@ int launch_cached_attention(const float *q, const float *k_cache, const float *v
             MGQ_CUDA(cudaFuncSetAttribute(cached_attention_kernel<128, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiles));
             opted_in[dev] = true;
         }
-        return launch(small_group ? cached_attention_kernel<128, 4> : cached_attention_kernel<128, 8>, grid, dim3(128), tiles, st, q, k_cache,
+        return launch(small_group ? cached_attention_kernel<128, 4> : cached_attention_kernel<128, 8>, grid, dim3(kAttThreads), tiles, st, q, k_cache,
                       v_cache, kv_pos, out, num_heads, num_kv_heads, max_seq, partials, counters);
     }
     return fail(MGQ_ERR_SHAPE, "attention: head_dim %u (64 and 128 are built)", head_dim);
