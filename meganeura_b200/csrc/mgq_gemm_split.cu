@@ -223,19 +223,13 @@ __device__ __forceinline__ void copy4(uint32_t dst, const void *src, bool live)
 
 // D[128 lanes, N] (+)= A (f16 pairs in TMEM, 8 columns) . B (shared memory)
 template <bool ACC>
-__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint64_t desc_b, uint32_t instr)
+__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint32_t b16, uint32_t instr)
 {
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "setp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-                 ::"r"(d), "r"(a), "l"(desc_b), "r"(instr), "n"(ACC ? 1 : 0) : "memory");
-}
-// One lane of a converged warp.
-__device__ __forceinline__ bool elect_one()
-{
-    uint32_t is;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
-    return is != 0;
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+                 "setp.ne.b32 p, %5, 0;\n\t"
+                 "mov.b64 db, {%2, %4};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "r"(b16 | 0x10000u), "r"(instr), "r"(kDescHigh), "n"(ACC ? 1 : 0) : "memory");
 }
 // A converged warp waits for several barriers at once, a lane (with `mine` set) for each: the try_waits share one latency.
 __device__ __forceinline__ bool mbar_wait_lanes(unsigned long long *bar, uint32_t parity, bool mine, volatile int *failed)
@@ -483,7 +477,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
             const uint32_t instr = split_instr(p.tok);
             const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), count = __shfl_sync(0xffffffffu, u_end - u_begin, 0);
             const bool leader = elect_one();
-            const uint64_t ring_desc = umma_desc(smem_u32(ring));
+            const uint32_t ring16 = smem_u32(ring) >> 4;
             const uint32_t sub16 = sub >> 4;
             bool ok = true;
             for (uint32_t i = 0; i < count; i++) {
@@ -496,7 +490,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                 if (!ok) break;
                 tc_fence_after();
                 if (leader) {
-                    const uint64_t x_lo = ring_desc + s * kParts * sub16, x_hi = x_lo + (kParts - 2) * sub16;
+                    const uint32_t x_lo = ring16 + s * kParts * sub16, x_hi = x_lo + (kParts - 2) * sub16;
                     if (FMT == MGQ_FMT_Q4)
                         umma_f16(d, plain_desc(smem_u32(minima + b * kMinBytes)), plain_desc(smem_u32(side_ring + (i % kScaleSlots) * side + p.tok * 4u)), instr, 0u);
                     if (FMT == MGQ_FMT_Q4) umma_f16_ts<true>(d, w_lo, x_hi, instr);

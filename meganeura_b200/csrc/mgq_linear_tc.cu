@@ -5,10 +5,13 @@
 //
 // Persistent: one CTA per SM walks the output tiles (128 rows x TN columns) of all layers of the
 // group, rows fastest, so that consecutive CTAs share a weight tile in L2.
-//   warp 0      TMA producer: 128B-swizzled boxes [128 x 64] of x and [TN x 64] of W per stage
-//               (no multicast), completing on full[s].
-//   warp 1      allocates TMEM, issues 4 tcgen05.mma (M=128, N=TN, K=16) per stage, commits the stage
-//               to empty[s] and the tile to acc_full[b].
+//   warp 0      TMA producer: 128B-swizzled boxes [128 x 64] of x and [TN x 64] of W (no multicast), one or two per stage,
+//               a lane for each, completing on full[s].
+//   warp 1      allocates TMEM, issues 4 or 8 tcgen05.mma (M=128, N=TN, K=16) per stage, commits the stage
+//               to empty[s] and the tile to acc_full[b].  The whole warp runs the loop and an elected lane issues, so that
+//               descriptors stay in uniform registers.
+// A stage's wait and commit take the issuing warp about 300 cycles, as long as 4 MMAs of 128 columns run: TN of 128 and
+// 64 therefore take 128 k per stage.
 //   warps 2-5   epilogue of one accumulator while the other is being filled (2 x TN TMEM columns).
 // Every mbarrier wait is bounded; when one runs out the device-wide error word is raised (mgq_device_status) and the roles end.
 #include <cuda_fp16.h>
@@ -21,7 +24,7 @@
 namespace mgq {
 namespace {
 
-constexpr uint32_t TM = 128, TK = 64;
+constexpr uint32_t TM = 128, TK = 64;                // rows of a tile, k of a box
 constexpr uint32_t kBytesA = TM * TK * 2;
 constexpr int kThreads = 192;
 
@@ -31,8 +34,9 @@ struct LinearMaps {
     CUtensorMap a[kMaxSegments], w[kMaxSegments];        // a GLU group has one layer: w[1] is its second weight
 };
 
-template <int TN> __host__ __device__ constexpr uint32_t stage_bytes() { return kBytesA + TN * TK * 2; }
-template <int TN> __host__ __device__ constexpr int stages() { return TN == 256 ? 4 : TN == 128 ? 6 : 8; }
+template <int TN> __host__ __device__ constexpr uint32_t boxes() { return TN == 256 ? 1 : 2; }             // of 64 k per stage
+template <int TN> __host__ __device__ constexpr uint32_t stage_bytes() { return boxes<TN>() * (kBytesA + TN * TK * 2); }
+template <int TN> __host__ __device__ constexpr int stages() { return TN == 128 ? 3 : 4; }
 
 template <int S>
 struct __align__(8) LinearShared {
@@ -110,23 +114,27 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc_kernel(const __grid_con
         tiles = tiles / all * mt;
     }
 
+    constexpr uint32_t kBoxes = boxes<TN>(), kBytesW = TN * TK * 2;
     if (warp == 0) {
-        if (lane == 0) {
+        // lane = box of the stage * kLoads + operand
+        constexpr uint32_t kLoads = GLU ? 3 : 2;
+        if (lane < kBoxes * kLoads) {
+            const uint32_t box = lane / kLoads, what = lane % kLoads;
+            const uint32_t offset = what == 0 ? box * kBytesA : kBoxes * kBytesA + box * kBytesW + (what == 2 ? COLS * TK * 2 : 0);
             uint32_t it = 0;
             int armed = -1;
             bool ok = true;
             for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
                 const Tile tl = find_tile<COLS>(g, tile, mt);
-                const uint32_t nk = (g.seg[tl.si].k + TK - 1) / TK;
+                const uint32_t nk = (g.seg[tl.si].k + TK * kBoxes - 1) / (TK * kBoxes);
+                const CUtensorMap *map = what == 0 ? &maps.a[tl.si] : what == 1 ? &maps.w[tl.si] : &maps.w[1];
+                const int y = (int)(what == 0 ? tl.m0 : tl.n0);
                 for (uint32_t kc = 0; kc < nk; kc++, it++) {
                     const uint32_t s = it % S, ph = (it / S) & 1u;
                     ok = mbar_wait(&sh.empty[s], ph ^ 1u, &sh.failed, &g_linear_tc_error);
                     if (!ok) break;
-                    uint8_t *st = ring + s * kStage;
-                    mbar_arrive_expect_tx(&sh.full[s], kStage);
-                    tma_load_2d(st, &maps.a[tl.si], (int)(kc * TK), (int)tl.m0, &sh.full[s]);
-                    tma_load_2d(st + kBytesA, &maps.w[tl.si], (int)(kc * TK), (int)tl.n0, &sh.full[s]);
-                    if (GLU) tma_load_2d(st + kBytesA + COLS * TK * 2, &maps.w[1], (int)(kc * TK), (int)tl.n0, &sh.full[s]);
+                    if (lane == 0) mbar_arrive_expect_tx(&sh.full[s], kStage);      // the phase stays open for this arrival
+                    tma_load_2d(ring + s * kStage + offset, map, (int)((kc * kBoxes + box) * TK), y, &sh.full[s]);
                     armed = (int)it;
                 }
             }
@@ -136,29 +144,34 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc_kernel(const __grid_con
                     for (uint32_t w = 0; w < kWaitLimit && !mbar_try_wait(&sh.full[i % S], ((uint32_t)i / S) & 1u); w++) { }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            uint32_t it = 0, at = 0;
-            bool ok = true;
-            for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, at++) {
-                const uint32_t b = at & 1u;
-                ok = mbar_wait(&sh.acc_empty[b], ((at >> 1) & 1u) ^ 1u, &sh.failed, &g_linear_tc_error);
+        const bool leader = elect_one();
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), base16 = smem_u32(ring) >> 4;
+        uint32_t it = 0, at = 0;
+        bool ok = true;
+        for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, at++) {
+            const uint32_t b = at & 1u;
+            ok = __all_sync(0xffffffffu, mbar_wait(&sh.acc_empty[b], ((at >> 1) & 1u) ^ 1u, &sh.failed, &g_linear_tc_error));
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t nk = (g.seg[find_tile<COLS>(g, tile, mt).si].k + TK * kBoxes - 1) / (TK * kBoxes);
+            for (uint32_t kc = 0; kc < nk; kc++, it++) {
+                const uint32_t s = it % S, ph = (it / S) & 1u;
+                ok = __all_sync(0xffffffffu, mbar_wait(&sh.full[s], ph, &sh.failed, &g_linear_tc_error));
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t nk = (g.seg[find_tile<COLS>(g, tile, mt).si].k + TK - 1) / TK;
-                for (uint32_t kc = 0; kc < nk; kc++, it++) {
-                    const uint32_t s = it % S, ph = (it / S) & 1u;
-                    ok = mbar_wait(&sh.full[s], ph, &sh.failed, &g_linear_tc_error);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t base = smem_u32(ring + s * kStage);
+                if (leader) {
+                    const uint32_t a = base16 + s * (kStage / 16), w = a + kBoxes * (kBytesA / 16);
+                    if (kc == 0) umma_step<false>(tm + b * TN, a, w, umma_instr(TM, TN));
+                    else         umma_step<true>(tm + b * TN, a, w, umma_instr(TM, TN));
 #pragma unroll
-                    for (uint32_t j = 0; j < TK / 16; j++)
-                        umma_f16(tmem + b * TN, umma_desc(base + j * 32u), umma_desc(base + kBytesA + j * 32u), umma_instr(TM, TN),
-                                 (kc | j) != 0 ? 1u : 0u);
+                    for (uint32_t j = 1; j < kBoxes * TK / 16; j++)
+                        umma_step<true>(tm + b * TN, a + (j / 4) * (kBytesA / 16) + (j % 4) * 2u, w + (j / 4) * (kBytesW / 16) + (j % 4) * 2u, umma_instr(TM, TN));
                     umma_commit(&sh.empty[s]);
                 }
-                if (ok) umma_commit(&sh.acc_full[b]);
+                __syncwarp();
             }
+            if (ok && leader) umma_commit(&sh.acc_full[b]);
+            __syncwarp();
         }
     } else {
         const uint32_t quad = warp & 3u;                 // TMEM lanes this warp may read

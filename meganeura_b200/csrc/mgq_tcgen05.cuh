@@ -75,6 +75,25 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint6
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
                  ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(instr), "r"(accumulate), "r"(0u) : "memory");
 }
+// The same for operands in the layout of umma_desc, from the low words of their descriptors (address / 16, rest fixed): the
+// high words are constants, so that a step costs one add per operand.
+constexpr uint32_t kDescHigh = (1024 >> 4) | (1u << 14) | (2u << 29);
+template <bool ACC>
+__device__ __forceinline__ void umma_step(uint32_t tmem_d, uint32_t a16, uint32_t b16, uint32_t instr)
+{
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+                 "setp.ne.b32 p, %5, 0;\n\t"
+                 "mov.b64 da, {%1, %4};\n\tmov.b64 db, {%2, %4};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
+                 ::"r"(tmem_d), "r"(a16 | 0x10000u), "r"(b16 | 0x10000u), "r"(instr), "r"(kDescHigh), "n"(ACC ? 1 : 0) : "memory");
+}
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t is;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(is));
+    return is != 0;
+}
 __device__ __forceinline__ void umma_commit(unsigned long long *bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
