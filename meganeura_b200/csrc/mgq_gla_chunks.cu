@@ -1,10 +1,13 @@
-// Gated linear attention over many tokens in chunks of 16 on the tensor cores.
+// Recurrences over many tokens in chunks of 16 on the tensor cores: gated linear attention, RWKV-style time mixing, mLSTM.
 //
 // Inside a chunk, with a_t the decays per key channel, L_t = a_1 .. a_t, G_s = a_(s+1) .. a_16 and the
 // state S in front of the chunk:
 //     o_t = S^T (L_t q_t) + sum_(s <= t) A_ts v_s,      A_ts = sum_d q_t k_s a_(s+1) .. a_t
 //     S'  = diag(L_16) S + sum_s (G_s k_s) v_s^T
 // Only products of decays appear, never a quotient, so nothing overflows however strong the decay is.
+// Time mixing reads the state before a token's decay and update: L_t = a_1 .. a_(t-1), A_ts = sum_d q_t k_s a_(s+1) .. a_(t-1)
+// for s < t and A_tt = sum_d q_t u k_t.  mLSTM: with the maxima m_t (a scan over the gates, mlstm_gates_kernel) all channels of a head decay by
+// exp(f_t + m_(t-1) - m_t), keys count exp(i_t - m_t), and the normaliser is one more value column that holds ones.
 //   gla_prepare_kernel  CTA = chunk x head: the decays from their low-rank projection, then A, L q, G k and L_16
 //                       into a record that the next kernel copies as it is
 //   gla_chunks_kernel   a warp keeps S^T for 16 value columns and all keys in registers, as f32 accumulators of
@@ -12,9 +15,11 @@
 //                       the records come through a ring of cp.async copies
 // State, decays and sums are f32.  Where the state is read it enters as the sum of three bf16, i.e. with all its
 // bits; the decayed queries and keys, A and the values as sums of two, three products each: 16 to 17 significant bits
-// of numbers whose factors are projections, with the range of f32.  A long portion is cut into segments:
+// of numbers whose factors are projections, with the range of f32.  Time mixing and mLSTM take sums of three everywhere (six
+// products each, 24 bits) and add a chunk's update to the state in f32.  A long portion is cut into segments:
 // a first pass leaves the end state of every segment but the last, each started from nothing, gla_combine_kernel
 // turns them into the segments' start states, and a second pass runs all segments with outputs.
+// 2048 tokens, all launches: mLSTM 8 x 128 x 256 190 us against 311 token by token, time mixing 32 x 64 x 64 about 100 against 138.
 #include <algorithm>
 
 #include "mgq_mixer.cuh"
@@ -24,22 +29,39 @@ namespace {
 
 constexpr uint32_t kChunk = 16, kStages = 3, kMaxWarps = 8, kMaxSegs = 16;
 
-// Record of a chunk of a head: G k (high, low parts), L_16, L q (high, low), A (high, low); rows padded for ldmatrix.
-template <int D> struct Record {
+enum { kGla = 0, kWkv = 1, kMlstm = 2 };
+__host__ __device__ constexpr int parts_of(int mode) { return mode == kGla ? 2 : 3; }
+
+// Record of a chunk of a head: G k (parts, the highest first), L_16, L q (parts), A (parts); rows padded for ldmatrix.
+template <int D, int PARTS> struct Record {
     static constexpr uint32_t pitch = D + 8, matrix = kChunk * pitch * 2;
-    static constexpr uint32_t lam = 2 * matrix, ql = lam + D * 4, a = ql + 2 * matrix, bytes = a + 2 * kChunk * kChunk * 2;
+    static constexpr uint32_t lam = PARTS * matrix, ql = lam + D * 4, a = ql + PARTS * matrix, bytes = a + PARTS * kChunk * kChunk * 2;
     static constexpr uint32_t state_part = ql;           // what a pass without outputs needs
 };
 
 struct Chunks {
     const float *q, *k, *v, *w;                          // w: decays, or null: from d
     Decay d;
+    const float *u;                                      // time mixing: bonus [heads, dim]
+    const float *gi, *gf;                                // mLSTM: gate pre-activations [rows, heads]
+    float4 *gates;                                       // mLSTM: decay, key weight, exp(-m) [heads][rows]
+    float *den;                                          // mLSTM: normaliser . q [rows, heads]
+    float *shift_state;
     float *o, *state, *segments, *products;              // products: of a segment's decays, [segment][heads][D]
     uint8_t *records;
     uint32_t rows, heads, dim, vdim, chunks;
+    uint32_t cols;                                       // value columns with the normaliser's
+    uint32_t blocks, norm_pitch, shift_width;            // mLSTM: copies of n and m behind the state, floats from one to the next
     uint32_t seg_len, segs, states_only;                 // chunks per segment; the first pass leaves end states only
-    float qscale;
+    float qscale, cap;
 };
+
+// Normaliser of a head (n, then m), copy b: behind the heads' states.
+__device__ __forceinline__ float *normalizer(const Chunks &p, uint32_t head, uint32_t b)
+{
+    const uint32_t kp = (p.dim + 3u) & ~3u;
+    return p.state + (size_t)p.heads * p.vdim * kp + (size_t)(head * p.blocks + b) * p.norm_pitch;
+}
 
 __device__ __forceinline__ void split2(float x, float y, uint32_t &hi, uint32_t &lo)
 {
@@ -57,16 +79,64 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t &hi, uint32_t 
     split2(x - f.x, y - f.y, mid, lo);
 }
 
-template <int D>
+// The parts of two neighbours, the highest first.
+template <int PARTS>
+__device__ __forceinline__ void split_parts(float x, float y, uint32_t (&part)[3])
+{
+    if (PARTS == 3) split3(x, y, part[0], part[1], part[2]);
+    else            split2(x, y, part[0], part[1]);
+}
+
+// m_t = max(f_t + m_(t-1), i_t) is a scan of (sum of f, max) pairs.  CTA = head; 1024 tokens at a time.
+__global__ void __launch_bounds__(1024) mlstm_gates_kernel(const __grid_constant__ Chunks p)
+{
+    __shared__ float s_f[32], s_m[32], s_last;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, head = blockIdx.x, kp = (p.dim + 3u) & ~3u;
+    pdl_launch_dependents();
+    pdl_wait();
+    float m = normalizer(p, head, 0)[kp];
+    __syncthreads();                                     // read by all before it is replaced below
+    for (uint32_t r0 = 0; r0 < p.rows; r0 += 1024) {
+        const uint32_t row = r0 + t;
+        const bool in = row < p.rows;
+        const size_t at = (size_t)row * p.heads + head;
+        const float li = in ? p.cap * tanhf(p.gi[at] / p.cap) : -INFINITY, lf = in ? log_sigmoid(p.cap * tanhf(p.gf[at] / p.cap)) : 0.f;
+        float F = lf, M = li;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const float Fp = __shfl_up_sync(0xffffffffu, F, off), Mp = __shfl_up_sync(0xffffffffu, M, off);
+            if (lane >= (uint32_t)off) { M = fmaxf(M, F + Mp); F += Fp; }
+        }
+        if (lane == 31) { s_f[warp] = F; s_m[warp] = M; }
+        __syncthreads();
+        float before = m;                                // m in front of this warp
+        for (uint32_t w = 0; w < warp; w++) before = fmaxf(s_f[w] + before, s_m[w]);
+        const float mt = fmaxf(F + before, M);
+        float prev = __shfl_up_sync(0xffffffffu, mt, 1);
+        if (lane == 0) prev = before;
+        if (in) p.gates[(size_t)head * p.rows + row] = make_float4(expf(lf + (prev - mt)), expf(li - mt), expf(-mt), 0.f);
+        if (t == 1023) s_last = mt;                      // tokens beyond the portion leave it as it is
+        __syncthreads();
+        m = s_last;
+        __syncthreads();
+    }
+    if (t < p.blocks) normalizer(p, head, t)[kp] = m;
+}
+
+template <int D, int MODE>
 __global__ void __launch_bounds__(256) gla_prepare_kernel(const __grid_constant__ Chunks p)
 {
     constexpr uint32_t P = D + 4, SLICES = D / 4 < 16 ? D / 4 : 16;
-    using R = Record<D>;
+    constexpr int PARTS = parts_of(MODE);
+    using R = Record<D, PARTS>;
     extern __shared__ __align__(16) float smem[];        // q, k, w [16][P], partial sums of A [SLICES][16 t][16 s]
     float *sq = smem, *sk = sq + kChunk * P, *sw = sk + kChunk * P, *sa = sw + kChunk * P;
     const uint32_t t = threadIdx.x, chunk = blockIdx.x, head = blockIdx.y, row0 = chunk * kChunk, kpitch = p.heads * p.dim;
     pdl_launch_dependents();
     pdl_wait();
+    if (MODE == kWkv && p.shift_state && chunk == 0)     // what token shift has left for the next step
+        for (uint32_t j = head * 256 + t; j < p.shift_width; j += p.heads * 256) p.shift_state[j] = p.shift_state[p.shift_width + j];
+    const float4 *gates = MODE == kMlstm ? p.gates + (size_t)head * p.rows + row0 : nullptr;
     // beyond the portion and beyond the head's channels: nothing decays and nothing is added
     if (p.dim % 4 == 0) {
 #pragma unroll
@@ -77,6 +147,10 @@ __global__ void __launch_bounds__(256) gla_prepare_kernel(const __grid_constant_
             const size_t at = (size_t)(row0 + r) * kpitch + head * p.dim + d;
             float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
             if (in) { q = *reinterpret_cast<const float4 *>(p.q + at); k = *reinterpret_cast<const float4 *>(p.k + at); }
+            if (MODE == kMlstm && in) {
+                const float b = gates[r].y;
+                k.x *= b; k.y *= b; k.z *= b; k.w *= b;
+            }
             *reinterpret_cast<float4 *>(sq + r * P + d) = make_float4(q.x * p.qscale, q.y * p.qscale, q.z * p.qscale, q.w * p.qscale);
             *reinterpret_cast<float4 *>(sk + r * P + d) = k;
         }
@@ -87,10 +161,15 @@ __global__ void __launch_bounds__(256) gla_prepare_kernel(const __grid_constant_
             const bool in = row0 + r < p.rows && d < p.dim;
             const size_t at = (size_t)(row0 + r) * kpitch + head * p.dim + d;
             sq[r * P + d] = in ? p.q[at] * p.qscale : 0.f;
-            sk[r * P + d] = in ? p.k[at] : 0.f;
+            sk[r * P + d] = in ? p.k[at] * (MODE == kMlstm ? gates[r].y : 1.f) : 0.f;
         }
     }
-    if (p.w) {
+    if (MODE == kMlstm) {
+        for (uint32_t i = t; i < kChunk * D; i += 256) {
+            const uint32_t r = i / D, d = i % D;
+            sw[r * P + d] = row0 + r < p.rows ? gates[r].x : 1.f;
+        }
+    } else if (p.w) {
 #pragma unroll 4
         for (uint32_t i = t; i < kChunk * D; i += 256) {
             const uint32_t r = i / D, d = i % D;
@@ -115,11 +194,25 @@ __global__ void __launch_bounds__(256) gla_prepare_kernel(const __grid_constant_
 #pragma unroll
                     for (int i = 0; i < (int)PER; i++) z[i] = p.d.w0[head * p.dim + d];
                 const __nv_bfloat16 *w2 = static_cast<const __nv_bfloat16 *>(p.d.w2) + (size_t)(head * p.dim + d) * ranks + j0;
-#pragma unroll 8
-                for (uint32_t j = 0; j < nj; j++) {
-                    const float x = __bfloat162float(w2[j]);
+                if (ranks % 8 == 0 && reinterpret_cast<uintptr_t>(p.d.w2) % 16 == 0) {      // eight ranks per load: 288 -> 89 us for the whole kernel with 32 x 64 channels, rank 64, 2048 tokens
+#pragma unroll 2
+                    for (uint32_t j = 0; j < nj; j += 8) {
+                        float x[8];
+                        unpack8(__ldg(reinterpret_cast<const uint4 *>(w2 + j)), x);
 #pragma unroll
-                    for (int i = 0; i < (int)PER; i++) z[i] = fmaf(x, sa[(r0 + i) * 128 + j], z[i]);
+                        for (int i = 0; i < (int)PER; i++) {
+                            const float4 a = *reinterpret_cast<const float4 *>(sa + (r0 + i) * 128 + j), b = *reinterpret_cast<const float4 *>(sa + (r0 + i) * 128 + j + 4);
+                            z[i] = fmaf(x[3], a.w, fmaf(x[2], a.z, fmaf(x[1], a.y, fmaf(x[0], a.x, z[i]))));
+                            z[i] = fmaf(x[7], b.w, fmaf(x[6], b.z, fmaf(x[5], b.y, fmaf(x[4], b.x, z[i]))));
+                        }
+                    }
+                } else {
+#pragma unroll 8
+                    for (uint32_t j = 0; j < nj; j++) {
+                        const float x = __bfloat162float(w2[j]);
+#pragma unroll
+                        for (int i = 0; i < (int)PER; i++) z[i] = fmaf(x, sa[(r0 + i) * 128 + j], z[i]);
+                    }
                 }
             }
         }
@@ -136,13 +229,24 @@ __global__ void __launch_bounds__(256) gla_prepare_kernel(const __grid_constant_
         for (int i = 0; i < (int)kChunk; i++) acc[i] = 0.f;
         for (uint32_t d = slice * 4; d < (uint32_t)D; d += 64) {
             const float4 k4 = *reinterpret_cast<const float4 *>(sk + s * P + d);
+            float4 u4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (MODE == kWkv) {
+                const float *u = p.u + head * p.dim + d;
+                u4 = make_float4(d < p.dim ? u[0] * k4.x : 0.f, d + 1 < p.dim ? u[1] * k4.y : 0.f, d + 2 < p.dim ? u[2] * k4.z : 0.f, d + 3 < p.dim ? u[3] * k4.w : 0.f);
+            }
             float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int i = 0; i < (int)kChunk; i++) {
                 const float4 w4 = *reinterpret_cast<const float4 *>(sw + i * P + d), q4 = *reinterpret_cast<const float4 *>(sq + i * P + d);
                 const bool own = (uint32_t)i == s;
+                if (MODE == kWkv) {                      // the state before this token, and the bonus
+                    const float4 x = own ? u4 : r;
+                    acc[i] = fmaf(x.x, q4.x, acc[i]); acc[i] = fmaf(x.y, q4.y, acc[i]); acc[i] = fmaf(x.z, q4.z, acc[i]); acc[i] = fmaf(x.w, q4.w, acc[i]);
+                }
                 r.x = own ? k4.x : r.x * w4.x; r.y = own ? k4.y : r.y * w4.y; r.z = own ? k4.z : r.z * w4.z; r.w = own ? k4.w : r.w * w4.w;
-                acc[i] = fmaf(r.x, q4.x, acc[i]); acc[i] = fmaf(r.y, q4.y, acc[i]); acc[i] = fmaf(r.z, q4.z, acc[i]); acc[i] = fmaf(r.w, q4.w, acc[i]);
+                if (MODE != kWkv) {
+                    acc[i] = fmaf(r.x, q4.x, acc[i]); acc[i] = fmaf(r.y, q4.y, acc[i]); acc[i] = fmaf(r.z, q4.z, acc[i]); acc[i] = fmaf(r.w, q4.w, acc[i]);
+                }
             }
         }
         if (slice < SLICES)
@@ -158,20 +262,21 @@ __global__ void __launch_bounds__(256) gla_prepare_kernel(const __grid_constant_
 #pragma unroll
                 for (int i = 0; i < (int)kChunk; i++) {
                     const float2 w2 = *reinterpret_cast<const float2 *>(sw + i * P + d), x = *reinterpret_cast<const float2 *>(sq + i * P + d);
-                    f.x *= w2.x; f.y *= w2.y;
-                    uint32_t hi, lo;
-                    split2(x.x * f.x, x.y * f.y, hi, lo);
-                    *reinterpret_cast<uint32_t *>(rec + R::ql + (i * R::pitch + d) * 2) = hi;
-                    *reinterpret_cast<uint32_t *>(rec + R::ql + R::matrix + (i * R::pitch + d) * 2) = lo;
+                    if (MODE != kWkv) { f.x *= w2.x; f.y *= w2.y; }
+                    uint32_t part[3];
+                    split_parts<PARTS>(x.x * f.x, x.y * f.y, part);
+#pragma unroll
+                    for (int h = 0; h < PARTS; h++) *reinterpret_cast<uint32_t *>(rec + R::ql + h * R::matrix + (i * R::pitch + d) * 2) = part[h];
+                    if (MODE == kWkv) { f.x *= w2.x; f.y *= w2.y; }
                 }
             } else {
 #pragma unroll
                 for (int i = (int)kChunk - 1; i >= 0; i--) {
                     const float2 w2 = *reinterpret_cast<const float2 *>(sw + i * P + d), x = *reinterpret_cast<const float2 *>(sk + i * P + d);
-                    uint32_t hi, lo;
-                    split2(x.x * f.x, x.y * f.y, hi, lo);
-                    *reinterpret_cast<uint32_t *>(rec + (i * R::pitch + d) * 2) = hi;
-                    *reinterpret_cast<uint32_t *>(rec + R::matrix + (i * R::pitch + d) * 2) = lo;
+                    uint32_t part[3];
+                    split_parts<PARTS>(x.x * f.x, x.y * f.y, part);
+#pragma unroll
+                    for (int h = 0; h < PARTS; h++) *reinterpret_cast<uint32_t *>(rec + h * R::matrix + (i * R::pitch + d) * 2) = part[h];
                     f.x *= w2.x; f.y *= w2.y;
                 }
                 *reinterpret_cast<float2 *>(rec + R::lam + d * 4) = f;
@@ -186,10 +291,10 @@ __global__ void __launch_bounds__(256) gla_prepare_kernel(const __grid_constant_
             const float2 y = *reinterpret_cast<const float2 *>(sa + i * kChunk * kChunk + 2 * t);
             x.x += y.x; x.y += y.y;
         }
-        uint32_t hi, lo;
-        split2(x.x, x.y, hi, lo);
-        *reinterpret_cast<uint32_t *>(rec + R::a + 4 * t) = hi;
-        *reinterpret_cast<uint32_t *>(rec + R::a + kChunk * kChunk * 2 + 4 * t) = lo;
+        uint32_t part[3];
+        split_parts<PARTS>(x.x, x.y, part);
+#pragma unroll
+        for (int h = 0; h < PARTS; h++) *reinterpret_cast<uint32_t *>(rec + R::a + h * kChunk * kChunk * 2 + 4 * t) = part[h];
     }
 }
 
@@ -208,10 +313,11 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 // CTA = head (x) x value columns (y), 16 per warp, x segment (z).
-template <int D>
+template <int D, int MODE>
 __global__ void __launch_bounds__(256, 1) gla_chunks_kernel(const __grid_constant__ Chunks p)
 {
-    using R = Record<D>;
+    constexpr int PARTS = parts_of(MODE);
+    using R = Record<D, PARTS>;
     extern __shared__ __align__(16) uint8_t ring[];      // kStages records
     __shared__ float s_f[D];                             // product of the decays so far (first pass)
     const uint32_t t = threadIdx.x, threads = blockDim.x, lane = t & 31u, warp = t >> 5, g = lane >> 2, tq = lane & 3u;
@@ -219,7 +325,8 @@ __global__ void __launch_bounds__(256, 1) gla_chunks_kernel(const __grid_constan
     const uint32_t seg = blockIdx.z, c0 = seg * p.seg_len, c1 = min(c0 + p.seg_len, p.chunks);
     const bool outputs = !p.states_only;
     const uint32_t vr[2] = {v0 + g, v0 + g + 8};         // this thread's value columns
-    const bool live[2] = {vr[0] < p.vdim, vr[1] < p.vdim};
+    const bool live[2] = {vr[0] < p.cols, vr[1] < p.cols};
+    const bool ones[2] = {MODE == kMlstm && vr[0] == p.vdim, MODE == kMlstm && vr[1] == p.vdim};      // the normaliser's column
     pdl_launch_dependents();
     pdl_wait();
     const uint8_t *records = p.records + (size_t)head * p.chunks * R::bytes;
@@ -244,7 +351,7 @@ __global__ void __launch_bounds__(256, 1) gla_chunks_kernel(const __grid_constan
 #pragma unroll
                 for (int e = 0; e < 2; e++) {
                     const uint32_t row = c * kChunk + h * 8 + tq * 2 + e;
-                    v[(h * 2 + i) * 2 + e] = c < c1 && row < p.rows && live[i] ? vbase[(size_t)row * vpitch + vr[i]] : 0.f;
+                    v[(h * 2 + i) * 2 + e] = c < c1 && row < p.rows && live[i] ? ones[i] ? 1.f : vbase[(size_t)row * vpitch + vr[i]] : 0.f;
                 }
     };
     load_values(c0);
@@ -258,14 +365,14 @@ __global__ void __launch_bounds__(256, 1) gla_chunks_kernel(const __grid_constan
     if (seg == 0 || outputs) {                           // start state: the sequence's, or what the combination left
         const bool own = seg == 0 && (p.segs == 1 || !outputs);
         const uint32_t slot = seg == 0 ? p.segs - 1 : seg - 1, pitch = own ? kp : D;
-        const float *start = own ? p.state + (size_t)head * p.vdim * kp : p.segments + ((size_t)slot * p.heads + head) * p.vdim * D;
+        const float *start = own ? p.state + (size_t)head * p.vdim * kp : p.segments + ((size_t)slot * p.heads + head) * p.cols * D;
 #pragma unroll
         for (int n = 0; n < D / 8; n++)
 #pragma unroll
             for (int i = 0; i < 2; i++) {
                 const uint32_t d = n * 8 + tq * 2;
                 if (d < pitch && live[i]) {
-                    const float2 x = *reinterpret_cast<const float2 *>(start + (size_t)vr[i] * pitch + d);
+                    const float2 x = *reinterpret_cast<const float2 *>((own && ones[i] ? normalizer(p, head, 0) : start + (size_t)vr[i] * pitch) + d);
                     S[n][2 * i] = x.x; S[n][2 * i + 1] = x.y;
                 }
             }
@@ -282,43 +389,54 @@ __global__ void __launch_bounds__(256, 1) gla_chunks_kernel(const __grid_constan
         stage(c + 2);
         const uint8_t *rec = ring + (c - c0) % kStages * R::bytes;
         const uint32_t base = smem_addr(rec);
-        uint32_t vh[4], vl[4];                           // V^T as left operand: rows value columns, columns tokens
+        uint32_t vp[3][4];                               // V^T as left operand: rows value columns, columns tokens
 #pragma unroll
-        for (int i = 0; i < 4; i++) split2(v[2 * i], v[2 * i + 1], vh[i], vl[i]);
+        for (int i = 0; i < 4; i++) {
+            uint32_t part[3];
+            split_parts<PARTS>(v[2 * i], v[2 * i + 1], part);
+#pragma unroll
+            for (int h = 0; h < PARTS; h++) vp[h][i] = part[h];
+        }
         load_values(c + 1);
         float o[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};          // o^T: rows value columns, columns tokens
 #pragma unroll
         for (int j = 0; j < D / 16; j++) {
-            uint32_t sh[4], sm[4], sl[4], qh[4], ql[4], kh[4], kl[4];
+            uint32_t sp[3][4], qp[3][4], kq[3][4];
             if (outputs) {
-                split3(S[2 * j][0], S[2 * j][1], sh[0], sm[0], sl[0]);
-                split3(S[2 * j][2], S[2 * j][3], sh[1], sm[1], sl[1]);
-                split3(S[2 * j + 1][0], S[2 * j + 1][1], sh[2], sm[2], sl[2]);
-                split3(S[2 * j + 1][2], S[2 * j + 1][3], sh[3], sm[3], sl[3]);
-                ldmatrix4(base + q_off + j * 32, qh);
-                ldmatrix4(base + q_off + R::matrix + j * 32, ql);
+#pragma unroll
+                for (int i = 0; i < 4; i++) split3(S[2 * j + i / 2][i % 2 * 2], S[2 * j + i / 2][i % 2 * 2 + 1], sp[0][i], sp[1][i], sp[2][i]);
+#pragma unroll
+                for (int h = 0; h < PARTS; h++) ldmatrix4(base + q_off + h * R::matrix + j * 32, qp[h]);
             }
-            ldmatrix4_t(base + k_off + j * 32, kh);
-            ldmatrix4_t(base + k_off + R::matrix + j * 32, kl);
+#pragma unroll
+            for (int h = 0; h < PARTS; h++) ldmatrix4_t(base + k_off + h * R::matrix + j * 32, kq[h]);
+            float add[2][4] = {};                        // three parts: the update by itself, added in f32
 #pragma unroll
             for (int n = 0; n < 2; n++) {
                 const float2 f = *reinterpret_cast<const float2 *>(rec + R::lam + (j * 16 + n * 8 + tq * 2) * 4);
                 float (&x)[4] = S[2 * j + n];
                 x[0] *= f.x; x[1] *= f.y; x[2] *= f.x; x[3] *= f.y;
             }
-            // small products first; the sums are independent of each other
+            // small products first (the two factors' parts count 2^-8 each); the sums are independent of each other
 #pragma unroll
-            for (int part = 0; part < 5; part++) {
-                const uint32_t (&sa)[4] = part == 0 ? sl : part == 1 || part == 3 ? sm : sh, (&qb)[4] = part == 1 || part == 2 ? ql : qh;
-                if (outputs) {
-                    mma16816(o[0], sa, qb[0], qb[1]);
-                    mma16816(o[1], sa, qb[2], qb[3]);
+            for (int order = 2; order >= 0; order--)
+#pragma unroll
+                for (int x = 0; x <= order; x++) {       // part x of the left operand, order - x of the right
+                    const int y = order - x;
+                    if (y >= PARTS) continue;
+                    if (outputs) {
+                        mma16816(o[0], sp[x], qp[y][0], qp[y][1]);
+                        mma16816(o[1], sp[x], qp[y][2], qp[y][3]);
+                    }
+                    if (PARTS == 2 && (order == 2 || x >= PARTS)) continue;
+                    mma16816(PARTS == 3 ? add[0] : S[2 * j], vp[x], kq[y][0], kq[y][1]);
+                    mma16816(PARTS == 3 ? add[1] : S[2 * j + 1], vp[x], kq[y][2], kq[y][3]);
                 }
-                if (part >= 3) continue;
-                const uint32_t (&va)[4] = part == 1 ? vl : vh, (&kb)[4] = part == 0 ? kl : kh;
-                mma16816(S[2 * j], va, kb[0], kb[1]);
-                mma16816(S[2 * j + 1], va, kb[2], kb[3]);
-            }
+            if (PARTS == 3)
+#pragma unroll
+                for (int n = 0; n < 2; n++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) S[2 * j + n][e] += add[n][e];
         }
         if (product)
             for (uint32_t d = t; d < (uint32_t)D; d += threads) s_f[d] *= *reinterpret_cast<const float *>(rec + R::lam + d * 4);
@@ -326,15 +444,22 @@ __global__ void __launch_bounds__(256, 1) gla_chunks_kernel(const __grid_constan
 #pragma unroll
         for (int n = 0; n < 2; n++) {                    // tokens n * 8 + g as columns, keys of the chunk as the sum
             const uint8_t *a = rec + R::a + ((n * 8 + g) * kChunk + tq * 2) * 2;
-            const uint32_t ah0 = *reinterpret_cast<const uint32_t *>(a), ah1 = *reinterpret_cast<const uint32_t *>(a + 16);
-            const uint32_t al0 = *reinterpret_cast<const uint32_t *>(a + kChunk * kChunk * 2), al1 = *reinterpret_cast<const uint32_t *>(a + kChunk * kChunk * 2 + 16);
-            mma16816(o[n], vh, al0, al1);
-            mma16816(o[n], vl, ah0, ah1);
-            mma16816(o[n], vh, ah0, ah1);
+            uint32_t ap[3][2];
+#pragma unroll
+            for (int h = 0; h < PARTS; h++) {
+                ap[h][0] = *reinterpret_cast<const uint32_t *>(a + h * kChunk * kChunk * 2);
+                ap[h][1] = *reinterpret_cast<const uint32_t *>(a + h * kChunk * kChunk * 2 + 16);
+            }
+#pragma unroll
+            for (int order = PARTS - 1; order >= 0; order--)
+#pragma unroll
+                for (int x = 0; x <= order; x++) mma16816(o[n], vp[x], ap[order - x][0], ap[order - x][1]);
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 const uint32_t row = c * kChunk + n * 8 + tq * 2 + (e & 1);
-                if (row < p.rows && live[e >> 1]) p.o[(size_t)row * vpitch + head * p.vdim + vr[e >> 1]] = o[n][e];
+                if (row >= p.rows || !live[e >> 1]) continue;
+                if (ones[e >> 1]) p.den[(size_t)row * p.heads + head] = o[n][e];
+                else              p.o[(size_t)row * vpitch + head * p.vdim + vr[e >> 1]] = o[n][e];
             }
         }
     }
@@ -348,7 +473,10 @@ __global__ void __launch_bounds__(256, 1) gla_chunks_kernel(const __grid_constan
             const uint32_t d = n * 8 + tq * 2;
             if (!live[i]) continue;
             const float2 x = make_float2(S[n][2 * i], S[n][2 * i + 1]);
-            if (!outputs)    *reinterpret_cast<float2 *>(p.segments + (((size_t)seg * p.heads + head) * p.vdim + vr[i]) * D + d) = x;
+            if (!outputs)    *reinterpret_cast<float2 *>(p.segments + (((size_t)seg * p.heads + head) * p.cols + vr[i]) * D + d) = x;
+            else if (ones[i]) {
+                for (uint32_t b = 0; d < kp && b < p.blocks; b++) *reinterpret_cast<float2 *>(normalizer(p, head, b) + d) = x;
+            }
             else if (d < kp) *reinterpret_cast<float2 *>(p.state + ((size_t)head * p.vdim + vr[i]) * kp + d) = x;
         }
 }
@@ -363,15 +491,15 @@ __global__ void __launch_bounds__(256) gla_combine_kernel(const __grid_constant_
     const uint32_t t = threadIdx.x, head = blockIdx.x, v0 = blockIdx.y * kCombineCols;
     pdl_launch_dependents();
     pdl_wait();
-    const size_t step = (size_t)p.heads * p.vdim * D;
+    const size_t step = (size_t)p.heads * p.cols * D;
     const uint32_t kp = (p.dim + 3u) & ~3u;
     for (uint32_t i = t; i < kCombineCols * D / 4; i += 256) {
         const uint32_t v = v0 + i / (D / 4), d = i % (D / 4) * 4;
-        if (v >= p.vdim) break;
-        float *at = p.segments + ((size_t)head * p.vdim + v) * D + d;
+        if (v >= p.cols) break;
+        float *at = p.segments + ((size_t)head * p.cols + v) * D + d;
         float4 S = *reinterpret_cast<const float4 *>(at);
         *reinterpret_cast<float4 *>(at + (p.segs - 1) * step) =
-            d < kp ? *reinterpret_cast<const float4 *>(p.state + ((size_t)head * p.vdim + v) * kp + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+            d < kp ? *reinterpret_cast<const float4 *>((v < p.vdim ? p.state + ((size_t)head * p.vdim + v) * kp : normalizer(p, head, 0)) + d) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
         for (uint32_t s = 1; s + 1 < p.segs; s++) {
             const float4 x = *reinterpret_cast<const float4 *>(at + s * step), f = *reinterpret_cast<const float4 *>(p.products + ((size_t)s * p.heads + head) * D + d);
@@ -381,72 +509,132 @@ __global__ void __launch_bounds__(256) gla_combine_kernel(const __grid_constant_
     }
 }
 
-uint32_t padded(uint32_t dim) { return dim <= 32 ? 32 : dim <= 64 ? 64 : dim <= 128 ? 128 : 256; }
-uint32_t warps_for(uint32_t vdim) { return std::min(kMaxWarps, (vdim + 15) / 16); }
-size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
-size_t record_bytes(uint32_t dim)
+// o = o / (max(|n . q|, exp(-m)) + 1e-6): a thread per four columns.
+__global__ void __launch_bounds__(256) mlstm_divide_kernel(const __grid_constant__ Chunks p)
 {
-    const uint32_t d = padded(dim);
-    return d == 32 ? Record<32>::bytes : d == 64 ? Record<64>::bytes : d == 128 ? Record<128>::bytes : Record<256>::bytes;
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t row = blockIdx.x;
+    for (uint32_t i = threadIdx.x; i < p.heads * p.vdim; i += 256) {
+        const uint32_t head = i / p.vdim;
+        const float d = fmaxf(fabsf(p.den[(size_t)row * p.heads + head]), p.gates[(size_t)head * p.rows + row].z) + 1e-6f;
+        p.o[(size_t)row * p.heads * p.vdim + i] /= d;
+    }
 }
 
-// Chunks per segment; all of them: one pass.  Two passes pay from three segments on.
-uint32_t segment_chunks(uint32_t chunks, uint32_t heads, uint32_t vdim)
+uint32_t padded(uint32_t dim) { return dim <= 32 ? 32 : dim <= 64 ? 64 : dim <= 128 ? 128 : 256; }
+// Two CTAs of up to 5 warps fit an SM where the state of a warp is no more than 128 keys wide.  More and shorter segments pay for
+// time mixing (32 x 64 x 64, 2048 tokens, both passes: 59 against 85 us), not for mLSTM, whose 17 blocks then need a fourth CTA
+// (8 x 128 x 256: 182 against 135 us).
+uint32_t ctas_per_sm(int mode, uint32_t dim) { return mode == kWkv && padded(dim) <= 128 ? 2 : 1; }
+// Blocks of 16 value columns, shared out evenly over as few CTAs as can take them.
+uint32_t warps_for(int mode, uint32_t dim, uint32_t cols)
 {
-    const uint32_t w = warps_for(vdim), ctas = heads * ((vdim + 16 * w - 1) / (16 * w)), want = std::min(kMaxSegs, 148u / ctas);
+    const uint32_t most = ctas_per_sm(mode, dim) == 2 ? 5 : kMaxWarps, blocks = (cols + 15) / 16, ctas = (blocks + most - 1) / most;
+    return (blocks + ctas - 1) / ctas;
+}
+size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
+template <int PARTS> size_t record_bytes_of(uint32_t dim)
+{
+    const uint32_t d = padded(dim);
+    return d == 32 ? Record<32, PARTS>::bytes : d == 64 ? Record<64, PARTS>::bytes : d == 128 ? Record<128, PARTS>::bytes : Record<256, PARTS>::bytes;
+}
+size_t record_bytes(int mode, uint32_t dim) { return parts_of(mode) == 2 ? record_bytes_of<2>(dim) : record_bytes_of<3>(dim); }
+
+// Chunks per segment; all of them: one pass.  Two passes pay from three segments on.
+uint32_t segment_chunks(int mode, uint32_t chunks, uint32_t heads, uint32_t dim, uint32_t cols)
+{
+    const uint32_t w = warps_for(mode, dim, cols), ctas = heads * ((cols + 16 * w - 1) / (16 * w)), want = std::min(kMaxSegs, 148u * ctas_per_sm(mode, dim) / ctas);
     if (want < 3 || chunks < 12) return chunks;
     const uint32_t len = std::max(4u, (chunks + want - 1) / want);
     return (chunks + len - 1) / len < 3 ? chunks : len;
 }
 
-template <int D>
+template <int D, int MODE>
 int launch_sized(Chunks p, cudaStream_t st)
 {
-    const size_t prep = (size_t)(3 * kChunk * (D + 4) + std::max(std::min(D / 4, 16) * kChunk * kChunk, kChunk * 128)) * 4, smem = (size_t)kStages * Record<D>::bytes;
-    if (int rc = allow_smem(gla_prepare_kernel<D>, prep)) return rc;
-    if (int rc = allow_smem(gla_chunks_kernel<D>, smem)) return rc;
-    if (int rc = launch(gla_prepare_kernel<D>, dim3(p.chunks, p.heads), dim3(256), prep, st, p)) return rc;
-    const uint32_t w = warps_for(p.vdim);
-    dim3 grid(p.heads, (p.vdim + 16 * w - 1) / (16 * w), p.segs);
+    const size_t prep = (size_t)(3 * kChunk * (D + 4) + std::max(std::min(D / 4, 16) * kChunk * kChunk, kChunk * 128)) * 4, smem = (size_t)kStages * Record<D, parts_of(MODE)>::bytes;
+    if (int rc = allow_smem(gla_prepare_kernel<D, MODE>, prep)) return rc;
+    if (int rc = allow_smem(gla_chunks_kernel<D, MODE>, smem)) return rc;
+    if (MODE == kMlstm)
+        if (int rc = launch(mlstm_gates_kernel, dim3(p.heads), dim3(1024), 0, st, p)) return rc;
+    if (int rc = launch(gla_prepare_kernel<D, MODE>, dim3(p.chunks, p.heads), dim3(256), prep, st, p)) return rc;
+    const uint32_t w = warps_for(MODE, p.dim, p.cols);
+    dim3 grid(p.heads, (p.cols + 16 * w - 1) / (16 * w), p.segs);
     if (p.segs > 1) {
         grid.z = p.segs - 1;
         p.states_only = 1;
-        if (int rc = launch(gla_chunks_kernel<D>, grid, dim3(w * 32), smem, st, p)) return rc;
-        if (int rc = launch(gla_combine_kernel<D>, dim3(p.heads, (p.vdim + kCombineCols - 1) / kCombineCols), dim3(256), 0, st, p)) return rc;
+        if (int rc = launch(gla_chunks_kernel<D, MODE>, grid, dim3(w * 32), smem, st, p)) return rc;
+        if (int rc = launch(gla_combine_kernel<D>, dim3(p.heads, (p.cols + kCombineCols - 1) / kCombineCols), dim3(256), 0, st, p)) return rc;
         grid.z = p.segs;
         p.states_only = 0;
     }
-    return launch(gla_chunks_kernel<D>, grid, dim3(w * 32), smem, st, p);
+    if (int rc = launch(gla_chunks_kernel<D, MODE>, grid, dim3(w * 32), smem, st, p)) return rc;
+    return MODE == kMlstm ? launch(mlstm_divide_kernel, dim3(p.rows), dim3(256), 0, st, p) : MGQ_OK;
+}
+
+template <int MODE>
+int launch_chunks(Chunks p, void *workspace, cudaStream_t st)
+{
+    p.cols = p.vdim + (MODE == kMlstm ? 1 : 0);
+    p.chunks = (p.rows + kChunk - 1) / kChunk;
+    uint8_t *ws = static_cast<uint8_t *>(workspace);
+    p.records = ws;
+    ws += align256((size_t)p.chunks * p.heads * record_bytes(MODE, p.dim));
+    if (MODE == kMlstm) {
+        p.gates = reinterpret_cast<float4 *>(ws);
+        ws += align256((size_t)p.rows * p.heads * 16);
+        p.den = reinterpret_cast<float *>(ws);
+        ws += align256((size_t)p.rows * p.heads * 4);
+    }
+    p.segments = reinterpret_cast<float *>(ws);
+    p.products = p.segments + (size_t)kMaxSegs * p.heads * p.cols * padded(p.dim);
+    p.seg_len = segment_chunks(MODE, p.chunks, p.heads, p.dim, p.cols);
+    p.segs = (p.chunks + p.seg_len - 1) / p.seg_len;
+    switch (padded(p.dim)) {
+        case 32: return launch_sized<32, MODE>(p, st);
+        case 64: return launch_sized<64, MODE>(p, st);
+        case 128: return launch_sized<128, MODE>(p, st);
+        default: return launch_sized<256, MODE>(p, st);
+    }
+}
+
+size_t chunks_workspace(int mode, uint32_t max_rows, uint32_t heads, uint32_t dim, uint32_t vdim)
+{
+    if (max_rows < kPrefillRows) return 0;
+    const size_t chunks = (max_rows + kChunk - 1) / kChunk, cols = vdim + (mode == kMlstm ? 1 : 0);
+    return align256(chunks * heads * record_bytes(mode, dim)) + (mode == kMlstm ? align256((size_t)max_rows * heads * 16) + align256((size_t)max_rows * heads * 4) : 0) +
+           (size_t)kMaxSegs * heads * (cols + 1) * padded(dim) * 4;
 }
 
 }  // namespace
 
-size_t gla_chunks_workspace(uint32_t max_rows, uint32_t heads, uint32_t dim, uint32_t vdim)
+size_t gla_chunks_workspace(uint32_t max_rows, uint32_t heads, uint32_t dim, uint32_t vdim) { return chunks_workspace(kGla, max_rows, heads, dim, vdim); }
+size_t wkv_chunks_workspace(uint32_t max_rows, uint32_t heads, uint32_t dim, uint32_t vdim) { return chunks_workspace(kWkv, max_rows, heads, dim, vdim); }
+size_t mlstm_chunks_workspace(uint32_t max_rows, uint32_t heads, uint32_t dim, uint32_t vdim) { return chunks_workspace(kMlstm, max_rows, heads, dim, vdim); }
+
+int launch_channel_decay_chunks(const ChannelDecay &a, void *stream)
 {
-    if (max_rows < kPrefillRows) return 0;
-    const size_t chunks = (max_rows + kChunk - 1) / kChunk;
-    return align256(chunks * heads * record_bytes(dim)) + (size_t)kMaxSegs * heads * (vdim + 1) * padded(dim) * 4;
+    if (a.dim > kMaxStateDim || !a.workspace) return fail(MGQ_ERR_STATE, "recurrence in chunks: no workspace");
+    Chunks p{};
+    p.q = a.q; p.k = a.k; p.v = a.v; p.w = a.decay_pending ? nullptr : a.d.out; p.d = a.d; p.u = a.u; p.o = a.o; p.state = a.state;
+    p.shift_state = a.shift_state; p.shift_width = a.shift_width;
+    p.rows = a.rows; p.heads = a.heads; p.dim = a.dim; p.vdim = a.vdim;
+    p.qscale = a.u ? 1.f : (float)(1.0 / sqrt((double)a.dim));
+    return a.u ? launch_chunks<kWkv>(p, a.workspace, static_cast<cudaStream_t>(stream)) : launch_chunks<kGla>(p, a.workspace, static_cast<cudaStream_t>(stream));
 }
 
-int launch_gla_chunks(const ChannelDecay &a, void *stream)
+int launch_mlstm_chunks(const Mlstm &a, uint32_t blocks, void *stream)
 {
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (a.u || a.dim > kMaxStateDim || !a.workspace) return fail(MGQ_ERR_STATE, "gla chunks: not this recurrence");
+    if (a.dim > kMaxStateDim || !a.workspace) return fail(MGQ_ERR_STATE, "recurrence in chunks: no workspace");
     Chunks p{};
-    p.q = a.q; p.k = a.k; p.v = a.v; p.w = a.decay_pending ? nullptr : a.d.out; p.d = a.d; p.o = a.o; p.state = a.state;
-    p.rows = a.rows; p.heads = a.heads; p.dim = a.dim; p.vdim = a.vdim; p.chunks = (a.rows + kChunk - 1) / kChunk;
-    p.records = static_cast<uint8_t *>(a.workspace);
-    p.segments = reinterpret_cast<float *>(p.records + align256((size_t)p.chunks * a.heads * record_bytes(a.dim)));
-    p.products = p.segments + (size_t)kMaxSegs * a.heads * a.vdim * padded(a.dim);
-    p.seg_len = segment_chunks(p.chunks, a.heads, a.vdim);
-    p.segs = (p.chunks + p.seg_len - 1) / p.seg_len;
+    p.q = a.q; p.k = a.k; p.v = a.v; p.gi = a.gi; p.gf = a.gf; p.o = a.o; p.state = a.state;
+    p.rows = a.rows; p.heads = a.heads; p.dim = a.dim; p.vdim = a.vdim;
+    p.blocks = blocks;
+    p.norm_pitch = ((a.dim + 3u) & ~3u) + 4u;
+    p.cap = a.cap;
     p.qscale = (float)(1.0 / sqrt((double)a.dim));
-    switch (padded(a.dim)) {
-        case 32: return launch_sized<32>(p, st);
-        case 64: return launch_sized<64>(p, st);
-        case 128: return launch_sized<128>(p, st);
-        default: return launch_sized<256>(p, st);
-    }
+    return launch_chunks<kMlstm>(p, a.workspace, static_cast<cudaStream_t>(stream));
 }
 
 }  // namespace mgq

@@ -98,14 +98,15 @@ struct ChannelDecay {
     float *o, *state, *shift_state;
     uint32_t rows, heads, dim, vdim, shift_width;
     void *workspace;                       // scan_workspace bytes, or null (long portions then run in one piece)
-    bool split_products;                   // gated linear, kPrefillRows or more rows: chunks on the tensor cores (mgq_gla_chunks.cu),
-                                           // whose workspace is gla_chunks_workspace bytes
+    bool split_products;                   // kPrefillRows or more rows: chunks on the tensor cores (mgq_gla_chunks.cu), whose
+                                           // workspace is gla_chunks_workspace (u set: wkv_chunks_workspace) bytes
     bool decay_pending;                    // d.out is not computed yet (only with that form, which computes the decay itself)
 };
 size_t channel_decay_state_elements(uint32_t heads, uint32_t dim, uint32_t vdim);
 int launch_channel_decay_scan(const ChannelDecay &a, void *stream);
 size_t gla_chunks_workspace(uint32_t max_rows, uint32_t heads, uint32_t dim, uint32_t vdim);
-int launch_gla_chunks(const ChannelDecay &a, void *stream);
+size_t wkv_chunks_workspace(uint32_t max_rows, uint32_t heads, uint32_t dim, uint32_t vdim);
+int launch_channel_decay_chunks(const ChannelDecay &a, void *stream);
 int launch_channel_decay_step(const ChannelDecay &a, const HeadGate &hg, void *stream);      // rows == 1: decay, recurrence, head gate in one launch
 
 // mLSTM recurrence.  q, k [rows, heads * dim], v, o [rows, heads * vdim], gate pre-activations
@@ -115,11 +116,14 @@ struct Mlstm {
     float *o, *state;
     uint32_t rows, heads, dim, vdim;
     float cap;
-    void *workspace;                       // as in ChannelDecay
+    void *workspace;                       // as in ChannelDecay, or mlstm_chunks_workspace bytes
+    bool split_products;                   // as in ChannelDecay
 };
 size_t scan_workspace(uint32_t max_rows, uint32_t heads, uint32_t dim, uint32_t vdim);
 size_t mlstm_state_elements(uint32_t heads, uint32_t dim, uint32_t vdim);
 int launch_mlstm_scan(const Mlstm &a, void *stream);
+size_t mlstm_chunks_workspace(uint32_t max_rows, uint32_t heads, uint32_t dim, uint32_t vdim);
+int launch_mlstm_chunks(const Mlstm &a, uint32_t blocks, void *stream);      // blocks: copies of n and m in the state
 int launch_mlstm_step(const Mlstm &a, const HeadGate &hg, void *stream);
 
 // Latent attention.  The cache is a ring of `slots` rows of rank + rot_dim elements (position p lives

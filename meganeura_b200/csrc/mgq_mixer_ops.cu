@@ -1165,10 +1165,14 @@ int launch_channel_decay_scan(const ChannelDecay &a, void *stream)
 {
     const Scan p = channel_decay_args(a);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (a.split_products && a.rows >= kPrefillRows) return launch_gla_chunks(a, stream);
+    if (a.split_products && a.rows >= kPrefillRows) return launch_channel_decay_chunks(a, stream);
     return a.u ? launch_scan<kWkv>(p, a.workspace, st) : launch_scan<kGla>(p, a.workspace, st);
 }
-int launch_mlstm_scan(const Mlstm &a, void *stream) { return launch_scan<kMlstm>(mlstm_args(a), a.workspace, static_cast<cudaStream_t>(stream)); }
+int launch_mlstm_scan(const Mlstm &a, void *stream)
+{
+    if (a.split_products && a.rows >= kPrefillRows) return launch_mlstm_chunks(a, value_blocks(a.dim, a.vdim), stream);
+    return launch_scan<kMlstm>(mlstm_args(a), a.workspace, static_cast<cudaStream_t>(stream));
+}
 int launch_channel_decay_step(const ChannelDecay &a, const HeadGate &hg, void *stream)
 {
     const Scan p = channel_decay_args(a);

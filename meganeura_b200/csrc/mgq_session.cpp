@@ -1139,10 +1139,19 @@ int attention_scratch(mgq_session *s, const Node &nd, Dispatch &d)
     return MGQ_OK;
 }
 
+// Long portions run in chunks on the tensor cores: gated linear attention where the graph says so, time mixing and mLSTM where
+// their gated output is rounded to bf16 by the same dispatch.
+bool recurrence_in_chunks(const mgq_session *s, const Node &nd, int out)
+{
+    if (nd.op == Op::Gla) return nd.at[3];
+    return s->nodes[out].op == Op::HeadGate && s->bf16(out);
+}
+
 int recurrence_workspace(mgq_session *s, const Node &nd, Dispatch &d)
 {
-    if (nd.op == Op::Gla && nd.at[3]) {
-        shared_scratch(s, mgq::gla_chunks_workspace((uint32_t)nd.shape[0], nd.at[0], nd.at[1], nd.at[2]), d);
+    if (recurrence_in_chunks(s, nd, d.out)) {
+        const auto bytes = nd.op == Op::Gla ? mgq::gla_chunks_workspace : nd.op == Op::Wkv ? mgq::wkv_chunks_workspace : mgq::mlstm_chunks_workspace;
+        shared_scratch(s, bytes((uint32_t)nd.shape[0], nd.at[0], nd.at[1], nd.at[2]), d);
         return MGQ_OK;
     }
     const size_t bytes = mgq::scan_workspace((uint32_t)nd.shape[0], nd.at[0], nd.at[1], nd.at[2]);
@@ -1874,7 +1883,7 @@ static int run_mixer(mgq_session *s, const Dispatch &d)
         const Node &dn = s->nodes[did];
         a.rows = a.d.rows = rows;
         a.workspace = d.workspace;
-        a.split_products = o.op == Op::Gla && o.at[3];
+        a.split_products = o.op != Op::Decay && recurrence_in_chunks(s, o, d.out);
         a.d.out = f(did);
         if (dn.op == Op::Decay) {
             a.d.low = f(dn.inputs[0]); a.d.w2 = s->ptr(dn.inputs[1]); a.d.w0 = f(dn.inputs[2]);
@@ -1889,7 +1898,8 @@ static int run_mixer(mgq_session *s, const Dispatch &d)
         a.shift_width = o.inputs[6] >= 0 ? (uint32_t)(s->nodes[o.inputs[6]].elements() / 2) : 0;
         if (!fused) return mgq::launch_channel_decay_scan(a, s->stream);
         if (rows == 1) return mgq::launch_channel_decay_step(a, hg, s->stream);
-        a.decay_pending = a.split_products && rows >= mgq::kPrefillRows;
+        // the preparation computes gated linear attention's decays itself (rank 16); time mixing's (rank 64) are 30 us cheaper in a kernel of their own
+        a.decay_pending = a.split_products && rows >= mgq::kPrefillRows && o.op == Op::Gla;
         if (!a.decay_pending)
             if (int rc = mgq::launch_decay(a.d, s->stream)) return rc;
         if (int rc = mgq::launch_channel_decay_scan(a, s->stream)) return rc;
@@ -1911,6 +1921,7 @@ static int run_mixer(mgq_session *s, const Dispatch &d)
         a.state = f(o.inputs[5]); a.o = f(oid);
         a.rows = rows; a.heads = o.at[0]; a.dim = o.at[1]; a.vdim = o.at[2]; a.cap = o.f0;
         a.workspace = d.workspace;
+        a.split_products = recurrence_in_chunks(s, o, d.out);
         if (!fused) return mgq::launch_mlstm_scan(a, s->stream);
         if (rows == 1) return mgq::launch_mlstm_step(a, hg, s->stream);
         if (int rc = mgq::launch_mlstm_scan(a, s->stream)) return rc;

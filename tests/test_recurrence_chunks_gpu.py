@@ -1,0 +1,90 @@
+"""Time mixing and mLSTM in chunks on the tensor cores: portions of 64 and more tokens whose gated output is rounded to bf16.
+
+The output is read through a linear layer with an identity matrix, so it is bf16: half an ulp is 2^-9 of the value; the rest of
+the tolerance of 2^-8 of the largest value is far above what three-part products leave.
+"""
+import numpy as np
+import pytest
+
+from oracle import petotar_oracle as P
+from graph_util import close, rng_of, run, session
+from petotar_util import bf16_round
+
+pytestmark = pytest.mark.gpu
+
+# chunks of 16: a multiple, one more, one less; several segments; short portions in between take the token-by-token kernels
+PORTIONS = (64, 1, 65, 30, 700, 79, 2)
+
+
+def _identity(g, x, n, params):
+    params["eye"] = np.eye(n, dtype=np.float32)
+    return g.matmul_bt(x, g.parameter_bf16("eye", [n, n]))
+
+
+@pytest.mark.parametrize("heads,dim,vdim,cap", [(2, 32, 48, 12.0), (3, 24, 8, 2.0), (1, 128, 256, 15.0), (2, 64, 100, 4.0), (1, 256, 16, 8.0), (2, 10, 128, 6.0)])
+def test_mlstm(heads, dim, vdim, cap):
+    import meganeura_b200 as mg
+    from meganeura_b200._lib import FMT_BF16, GATE_SIGMOID, ROWS_TOKENS, lib
+    r = rng_of(heads, dim, vdim)
+    n, nv, rows = heads * dim, heads * vdim, max(PORTIONS)
+    tabs = {"q": r.standard_normal((90, n)), "k": r.standard_normal((90, n)), "v": r.standard_normal((90, nv)), "g": r.standard_normal((90, nv)),
+              "i": r.standard_normal((90, heads)) * 6 - 2, "f": r.standard_normal((90, heads)) * 6 + 3}
+    tabs = {c: a.astype(np.float32) for c, a in tabs.items()}
+    hw = r.standard_normal(nv).astype(np.float32)
+    g = mg.Graph()
+    ids = g.input_u32_rows("ids", rows, ROWS_TOKENS)
+    e = {c: g.embedding_scaled(ids, g.parameter(c, list(a.shape)), 1.0) for c, a in tabs.items()}
+    state = g.parameter("state", [lib.mgq_mlstm_state_elements(heads, dim, vdim)])
+    o = g.mlstm(e["q"], e["k"], e["v"], e["i"], e["f"], state, heads, cap)
+    params = {**tabs, "hw": hw}
+    y = _identity(g, g.head_gate(o, e["g"], heads, g.parameter("hw", [nv]), 1e-5, GATE_SIGMOID, FMT_BF16), nv, params)
+    s = session(g, [y], params)
+    S, nn, m, at = np.zeros((heads, dim, vdim)), np.zeros((heads, dim)), np.zeros(heads), 0
+    for cnt in PORTIONS:
+        toks = (np.arange(at, at + cnt) * 11) % 90
+        at += cnt
+        s.set_rows(ROWS_TOKENS, cnt)
+        s.set_input_u32("ids", toks)
+        got = run(s, (cnt, nv))
+        li, lf = P.mlstm_gates(tabs["i"][toks].astype(np.float64), tabs["f"][toks].astype(np.float64), cap)
+        oo = P.mlstm_scan(tabs["q"][toks].reshape(cnt, heads, dim) * dim ** -0.5, tabs["k"][toks].reshape(cnt, heads, dim).astype(np.float64),
+                          tabs["v"][toks].reshape(cnt, heads, vdim).astype(np.float64), li, lf, S, nn, m)
+        close(got, P.unit_rms(oo, 1e-5).reshape(cnt, nv) * hw * P.sigmoid(tabs["g"][toks]), 2 ** -8)
+
+
+@pytest.mark.parametrize("heads,dim,rank", [(2, 32, 8), (3, 24, 5), (1, 64, 200), (2, 128, 4), (4, 8, 16), (1, 256, 3)])
+def test_wkv(heads, dim, rank):
+    import meganeura_b200 as mg
+    from meganeura_b200._lib import FMT_BF16, GATE_SILU, ROWS_TOKENS, lib
+    r = rng_of(heads, dim, rank)
+    n, rows, width = heads * dim, max(PORTIONS), 64
+    tabs = {c: r.standard_normal((90, n)).astype(np.float32) for c in "rkvg"}
+    tabs["low"] = r.standard_normal((90, width)).astype(np.float32)
+    mus = r.uniform(0, 1, (1, width)).astype(np.float32)
+    w1 = bf16_round(r.standard_normal((rank, width)).astype(np.float32) * width ** -0.5 * 2)
+    w2 = bf16_round(r.standard_normal((n, rank)).astype(np.float32) * min(1.0, (5 / rank) ** 0.5))
+    w0, u, hw = r.uniform(-5, 0, n).astype(np.float32), r.standard_normal(n).astype(np.float32), r.standard_normal(n).astype(np.float32)
+    g = mg.Graph()
+    ids = g.input_u32_rows("ids", rows, ROWS_TOKENS)
+    e = {c: g.embedding_scaled(ids, g.parameter(c, list(a.shape)), 1.0) for c, a in tabs.items()}
+    shift = g.parameter("shift", [2, width])
+    mix = g.token_shift(e["low"], [g.parameter("mu", [width])], shift)
+    decay = g.lora_decay(g.matmul_bt(g.slot(mix, 0), g.parameter_bf16("w1", [rank, width])), g.parameter_bf16("w2", [n, rank]), g.parameter("w0", [n]))
+    o = g.wkv(e["r"], e["k"], e["v"], decay, g.parameter("u", [n]), g.parameter("state", [lib.mgq_wkv_state_elements(heads, dim)]), heads, shift)
+    params = {**tabs, "mu": mus[0], "w1": w1, "w2": w2, "w0": w0, "u": u, "hw": hw}
+    y = _identity(g, g.head_gate(o, e["g"], heads, g.parameter("hw", [n]), 1e-4, GATE_SILU, FMT_BF16), n, params)
+    s = session(g, [y], params)
+    prev, S, at = np.zeros(width), np.zeros((heads, dim, dim)), 0
+    for cnt in PORTIONS:
+        toks = (np.arange(at, at + cnt) * 7) % 90
+        at += cnt
+        s.set_rows(ROWS_TOKENS, cnt)
+        s.set_input_u32("ids", toks)
+        got = run(s, (cnt, n))
+        h = tabs["low"][toks].astype(np.float64)
+        low = P.token_shift(h, prev, mus[0])
+        prev = h[-1]
+        ro, ko, vo, go = (tabs[c][toks].astype(np.float64) for c in "rkvg")
+        oo = P.wkv_scan(*(a.reshape(cnt, heads, dim) for a in (ro, ko, vo)), P.wkv_decay(low, w1, w2, w0).reshape(cnt, heads, dim), u.reshape(heads, dim), S)
+        close(got, P.unit_rms(oo, 1e-4).reshape(cnt, n) * hw * go * P.sigmoid(go), 2 ** -8)
+
