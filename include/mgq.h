@@ -246,7 +246,8 @@ size_t mgq_argmax_workspace(void);
 int mgq_argmax(const float *logits, uint32_t n, void *workspace, uint32_t *out_token, uint32_t *next_token, uint32_t *kv_pos,
                uint32_t *history, uint32_t history_cap, void *stream);
 
-/* Routing wrapper: mgq_gemv when m <= MGQ_GEMV_MAX_M (f32 activations), else mgq_gemm. */
+/* Routing wrapper: mgq_gemv when m <= MGQ_GEMV_MAX_M (f32 activations) and no pass over the weights beyond the second
+ * would be needed, else mgq_gemm. */
 int mgq_matmul(int fmt, const void *a, int a_dtype, const void *w, const float *addend, float *c,
                uint32_t m, uint32_t k, uint32_t n, void *stream);
 

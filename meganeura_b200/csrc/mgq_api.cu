@@ -228,7 +228,7 @@ int mgq_gemm(int fmt, const void *a, int a_dtype, const void *w, const float *ad
 int mgq_matmul(int fmt, const void *a, int a_dtype, const void *w, const float *addend, float *c,
                uint32_t m, uint32_t k, uint32_t n, void *stream)
 {
-    if (a_dtype == MGQ_A_F32 && m <= MGQ_GEMV_MAX_M)
+    if (a_dtype == MGQ_A_F32 && m <= MGQ_GEMV_MAX_M && (m == 0 || k == 0 || k % 32 != 0 || !gemv_prefers_gemm(fmt, m, k, n, a, w)))
         return mgq_gemv(fmt, static_cast<const float *>(a), w, addend, c, m, k, n, stream);
     return mgq_gemm(fmt, a, a_dtype, w, addend, c, m, k, n, stream);
 }

@@ -376,6 +376,18 @@ Config choose_config(int fmt, uint32_t bpc, uint32_t n, int mt, int sms)
         c.threads = (bpc + 31u) & ~31u;
     }
     c.cpi = columns_for(c.threads, bpc);
+    if (c.cpi == 0 && fmt == MGQ_FMT_Q4) {
+        // a Q4 thread copies its own 16 + 4 bytes, so columns need not come in groups; what counts is how many threads are left over
+        double best_u = -1.0;
+        for (uint32_t t = bpc <= 256 ? 128u : c.threads; t <= (bpc <= 256 ? 256u : c.threads); t += 32) {
+            const double util = (double)(t / bpc * bpc) / t;
+            if (util > best_u + 1e-9) { best_u = util; c.threads = t; }
+        }
+        c.cpi = c.threads / bpc;
+    } else if (c.cpi == 0) {
+        c.cpi = bpc % 2 == 0 ? 2u : 4u;                  // the smallest group that keeps Q8 warps on 16-byte boundaries
+        c.threads = (c.cpi * bpc + 31u) & ~31u;
+    }
     const uint32_t groups = (n + c.cpi - 1) / c.cpi;
     // columns per thread and stage: as many as keep every CTA of a two-per-SM grid busy, fit
     // in ~100 KB of shared memory and leave one finishing lane per column of a round
@@ -628,13 +640,31 @@ int launch_all_gather(const float *slice, const void *push_dev, const void *loca
     return MGQ_OK;
 }
 
-bool gemv_streamable(const void *x, uint32_t k, uint32_t n)
+bool gemv_streamable(int fmt, const void *x, uint32_t k, uint32_t n)
 {
     const uint32_t bpc = k / 32;
     if (bpc < 8 || bpc > 1024) return false;
-    // a group of columns has to fit a CTA; with block counts that are not multiples of 4 groups of 2 or 4 columns are needed
-    if (columns_for(bpc <= 256 ? 256u : (bpc + 31u) & ~31u, bpc) == 0) return false;
+    if (fmt == MGQ_FMT_Q8 && bpc % 4 != 0 && (bpc % 2 == 0 ? 2u : 4u) * bpc > 1024) return false;       // no group of columns fits a CTA
     return ((unsigned long long)bpc * n) % 4 == 0 && (reinterpret_cast<uintptr_t>(x) % 16 == 0);
+}
+
+// Up to 16 f32 rows for which the tensor-core GEMM is ahead (microseconds, GEMV / GEMM):
+//   8 rows per pass (mma kernel): a second pass over large Q8 weights, 16 x 4096 x 6144 30 / 25, x 24576 70 / 52 (Q4: 25 / 25, 55 / 52; 8 rows: 35 / 52)
+//   2 rows per pass (streaming):  from the third pass on, K = 1056, N = 4096: 4 rows 15 / 19, 6 rows 22 / 19, 16 rows 59 / 19
+//   1 row per pass (streaming with more than 512 threads): from the fourth, 4128 x 4096 Q8 3 rows 22 / 25, 4 rows 29 / 25; large ones
+//   from the third, 4128 x 24576 Q8 47 / 58 and 70 / 58
+//   1 row at a time, 4-byte loads (general kernel): 2080 x 4096 39 / 21 per row, 8800 x 3840 150 / 29; 17 us are the GEMM's two launches
+bool gemv_prefers_gemm(int fmt, uint32_t m, uint32_t k, uint32_t n, const void *x, const void *w)
+{
+    if (k <= 128 || !g_tuning.batch_mma) return false;
+    if (gemv_mma_eligible(m, k, n, x, w)) return fmt == MGQ_FMT_Q8 && m > 8 && (unsigned long long)k * n >= 20000000ull;
+    if (gemv_streamable(fmt, x, k, n)) {
+        const uint32_t bpc = k / 32;
+        const bool single = bpc > 512 || (fmt == MGQ_FMT_Q8 && bpc % 4 != 0 && columns_for(bpc <= 256 ? 256u : (bpc + 31u) & ~31u, bpc) == 0 && (bpc % 2 == 0 ? 2u : 4u) * bpc > 512);
+        if (single) return m >= ((unsigned long long)k * n >= 50000000ull ? 3u : 4u);
+        return m >= 5;
+    }
+    return (unsigned long long)m * k > 1024;
 }
 
 int launch_gemv(int fmt, const float *x, const void *w, const float *addend, float *y,
@@ -656,7 +686,7 @@ int launch_gemv(int fmt, const float *x, const void *w, const float *addend, flo
 
     if (!xchg && g_tuning.batch_mma && gemv_mma_eligible(m, k, n, x, w))
         return launch_gemv_mma(fmt, x, w, addend, y, m, k, n, stream_v);
-    const bool streamable = gemv_streamable(x, k, n);
+    const bool streamable = gemv_streamable(fmt, x, k, n);
     if (!streamable) {
         if (xchg) return fail(MGQ_ERR_SHAPE, "this shape has no exchanging GEMV kernel (K=%u N=%u)", k, n);
         p.x = x; p.addend = addend; p.y = y;
@@ -672,8 +702,12 @@ int launch_gemv(int fmt, const float *x, const void *w, const float *addend, flo
 
     // Rows are processed two at a time (their activations live in registers); more rows re-read W.
     for (uint32_t r0 = 0; r0 < m;) {
-        const int mt = (m - r0 >= 2 && bpc <= 512) ? 2 : 1;
-        const Config cfg = choose_config(fmt, bpc, n, mt, di.sms);
+        int mt = (m - r0 >= 2 && bpc <= 512) ? 2 : 1;
+        Config cfg = choose_config(fmt, bpc, n, mt, di.sms);
+        if (mt == 2 && cfg.threads > 512) {              // CTAs this wide have registers for one row
+            mt = 1;
+            cfg = choose_config(fmt, bpc, n, mt, di.sms);
+        }
         p.cpi = cfg.cpi;
         p.active = cfg.cpi * bpc;
         p.red_shift = cfg.red_shift;

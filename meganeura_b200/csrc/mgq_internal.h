@@ -34,7 +34,8 @@ int launch_gemv_mma(int fmt, const float *x, const void *w, const float *addend,
 // f16-weight GEMV (mgq_gemv_f16.cu).
 int launch_gemv_f16(const float *x, const void *w, const float *addend, float *y, uint32_t m, uint32_t k, uint32_t n, void *stream);
 int launch_gemv_bt(const float *x, const float *b, float *y, uint32_t k, uint32_t n, void *stream);
-bool gemv_streamable(const void *x, uint32_t k, uint32_t n);   // the streaming kernels take this shape (else the generic kernel runs)
+bool gemv_streamable(int fmt, const void *x, uint32_t k, uint32_t n);   // the streaming kernels take this shape (else the generic kernel runs)
+bool gemv_prefers_gemm(int fmt, uint32_t m, uint32_t k, uint32_t n, const void *x, const void *w);     // up to MGQ_GEMV_MAX_M f32 rows
 int launch_exchange_finish(const void *last_vec, uint32_t length, unsigned long long *epoch,
                            unsigned int *error, unsigned int *blocks_done, void *stream);
 int launch_all_gather(const float *slice, const void *push_dev, const void *local_vec, float *out, uint32_t rows, uint32_t cols,
