@@ -16,7 +16,8 @@
 // The tensor core truncates when it adds to its f32 accumulator, which over a long K would cost more than f32 sums do
 // (9e-6 for bf16 activations and K = 4096 in one accumulator).  So one accumulator takes a chunk of 128 k only, the small
 // products first; then it is added to a register sum in f32, times 2^e: 2.2e-7 off the exact product at K = 4096 and 2.0e-7 at
-// K = 512, where f32 sums in order of k are 1.1e-6 and 3.9e-7 off.
+// K = 512, where f32 sums in order of k are 1.1e-6 and 3.9e-7 off.  With bf16 activations and K from 2048 on two chunks share an
+// accumulator and a scale: 5e-7, and half the drains (149 -> 143 us for 512 x 4096 x 14336 in a long run).
 //
 // Weights are the left operand, straight from TMEM: a tile is 128 weight columns (TMEM lanes) by up to 128
 // tokens (any multiple of 16), so that few tokens cost few products and no shared-memory pass for weights.
@@ -57,6 +58,8 @@ namespace {
 constexpr uint32_t kChunk = 128;                   // k per accumulator
 constexpr uint32_t kCols = 128;                    // weight columns of a tile
 constexpr uint32_t kMaxTok = 128;                  // tokens of a tile
+// Chunks that share an accumulator and a scale.  Below 2048 k the f32 sums of the tiled kernel would be as exact as pairs are.
+__host__ __device__ constexpr uint32_t group_of(uint32_t planes, uint32_t k) { return planes == 1 && k >= 2048 ? 2 : 1; }
 constexpr uint32_t kSlots = 8;                     // ring of token sub-tiles (64 k of one plane)
 constexpr uint32_t kScaleSlots = 8;
 constexpr uint32_t kRaw = 4;                       // chunks of packed weights in flight, two per group
@@ -85,7 +88,7 @@ struct SplitParams {
 struct __align__(16) SplitShared {
     unsigned long long slot_full[kSlots], slot_empty[kSlots / 2];      // empty: a chunk's sub-tiles together
     unsigned long long sc_full[kScaleSlots], sc_empty[kScaleSlots];
-    unsigned long long w_full[2], d_empty[2], done[2], flushed;        // done: a chunk's products (its weight stage is free, its accumulator full)
+    unsigned long long w_full[2], w_empty[2], d_empty[2], d_full[2], flushed;
     uint32_t tmem_base;
     volatile int failed;
     uint32_t last;
@@ -141,7 +144,7 @@ __device__ __forceinline__ void store4(uint8_t *block, uint32_t sub, uint32_t pl
     if (planes == 2) *reinterpret_cast<uint2 *>(l + at) = *reinterpret_cast<const uint2 *>(lo);
 }
 
-// A warp per row and chunk.  Bound by the read of the activations (8 MB for 512 x 4096 f32) and as many bytes written,
+// A warp per row and group of chunks.  Bound by the read of the activations (8 MB for 512 x 4096 f32) and as many bytes written,
 // all of which stay in L2 for the GEMM behind it.
 __global__ void __launch_bounds__(256) split_rows_kernel(const void *a, bool bf16, bool vec, uint8_t *planes_out, uint8_t *side_out, unsigned int *counters, uint32_t tiles,
                                                          uint32_t m, uint32_t k, uint32_t tok, uint32_t chunks, uint32_t planes, bool q4)
@@ -149,59 +152,69 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const void *a, bool bf1
     pdl_launch_dependents();
     const uint32_t lane = threadIdx.x & 31u, gid = blockIdx.x * 8 + (threadIdx.x >> 5);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < tiles; i += gridDim.x * blockDim.x) counters[i] = 0;      // the GEMM's tile counters
-    const uint32_t row = gid / chunks, chunk = gid % chunks;
+    const uint32_t span = group_of(planes, k), groups = (chunks + span - 1) / span;
+    const uint32_t row = gid / groups, first_chunk = gid % groups * span;
     if (row >= m) return;
     const uint32_t mt = row / tok, t = row % tok, sub = tok * 128u;
-    float v[4] = {};
-    const uint32_t kk = chunk * kChunk + lane * 4;
-    if (kk < k) {
-        const size_t at = (size_t)row * k + kk;
-        if (vec && !bf16) {
-            const float4 q = *reinterpret_cast<const float4 *>(static_cast<const float *>(a) + at);
-            v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-        } else if (vec) {
-            const uint2 q = *reinterpret_cast<const uint2 *>(static_cast<const __nv_bfloat16 *>(a) + at);
-            v[0] = __uint_as_float(q.x << 16); v[1] = __uint_as_float(q.x & 0xFFFF0000u);
-            v[2] = __uint_as_float(q.y << 16); v[3] = __uint_as_float(q.y & 0xFFFF0000u);
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; i++) v[i] = load_act(a, at + i, bf16);
-        }
-    }
+    float v[2][4] = {}, sum[2] = {};                            // sum: of this lane's block of 32
     uint32_t top = 0;                                           // largest magnitude by its bits: NaN stays the largest
 #pragma unroll
-    for (int i = 0; i < 4; i++) top = max(top, __float_as_uint(v[i]) & 0x7FFFFFFFu);
-    float sum = 0.f;                                            // of this lane's block of 32
-    if (q4) {
-        sum = (v[0] + v[1]) + (v[2] + v[3]);
+    for (uint32_t c = 0; c < 2; c++) {
+        const uint32_t kk = (first_chunk + c) * kChunk + lane * 4;
+        if (c < span && kk < k) {
+            const size_t at = (size_t)row * k + kk;
+            if (vec && !bf16) {
+                const float4 q = *reinterpret_cast<const float4 *>(static_cast<const float *>(a) + at);
+                v[c][0] = q.x; v[c][1] = q.y; v[c][2] = q.z; v[c][3] = q.w;
+            } else if (vec) {
+                const uint2 q = *reinterpret_cast<const uint2 *>(static_cast<const __nv_bfloat16 *>(a) + at);
+                v[c][0] = __uint_as_float(q.x << 16); v[c][1] = __uint_as_float(q.x & 0xFFFF0000u);
+                v[c][2] = __uint_as_float(q.y << 16); v[c][3] = __uint_as_float(q.y & 0xFFFF0000u);
+            } else {
 #pragma unroll
-        for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        top = max(top, __float_as_uint(sum) & 0x7FFFFFFFu);
+                for (int i = 0; i < 4; i++) v[c][i] = load_act(a, at + i, bf16);
+            }
+        }
+    }
+#pragma unroll
+    for (uint32_t c = 0; c < 2; c++) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) top = max(top, __float_as_uint(v[c][i]) & 0x7FFFFFFFu);
+        if (q4) {
+            sum[c] = (v[c][0] + v[c][1]) + (v[c][2] + v[c][3]);
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+            top = max(top, __float_as_uint(sum[c]) & 0x7FFFFFFFu);
+        }
     }
     top = __reduce_max_sync(0xffffffffu, top);
     float down, up;
     pick_scale(__uint_as_float(top), down, up);
-    const size_t block = (size_t)mt * chunks + chunk;
-    uint8_t *side = side_out + block * side_bytes(q4 ? MGQ_FMT_Q4 : MGQ_FMT_Q8, tok);
-    // not finite: a NaN scale makes the row's sums NaN, which the GEMM computes again
-    if (lane == 0) reinterpret_cast<float *>(side)[t] = top >= 0x7F800000u ? __uint_as_float(0x7FC00000u) : up;
-    if (q4) {
-        // Q4 weights unpack as pairs (k, k + 4) of eight: order 0 4 1 5 2 6 3 7
-        const bool odd = lane & 1u;
-        const float r0 = __shfl_xor_sync(0xffffffffu, odd ? v[0] : v[2], 1), r1 = __shfl_xor_sync(0xffffffffu, odd ? v[1] : v[3], 1);
-        if (odd) { v[0] = r0; v[1] = v[2]; v[2] = r1; }
-        else     { v[3] = r1; v[2] = v[1]; v[1] = r0; }
-        // places 0-3 s.hi, 4-7 s.lo, 8-11 s.hi, 12-15 zero, beside the weights' b.hi, b.hi, b.lo, zero
-        if ((lane & 7u) == 0) {
-            const uint32_t b = lane >> 3;
-            const float s = sum * down;
-            const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
-            __half *first = reinterpret_cast<__half *>(side + tok * 4u + sums_at(t, 0)), *second = reinterpret_cast<__half *>(side + tok * 4u + sums_at(t, 1));
-            first[b] = hi; first[4 + b] = lo;
-            second[b] = hi; second[4 + b] = __float2half_rn(0.f);
+#pragma unroll
+    for (uint32_t c = 0; c < 2; c++) {
+        if (c >= span || first_chunk + c >= chunks) break;      // uniform over the warp
+        const size_t block = (size_t)mt * chunks + first_chunk + c;
+        uint8_t *side = side_out + block * side_bytes(q4 ? MGQ_FMT_Q4 : MGQ_FMT_Q8, tok);
+        // not finite: a NaN scale makes the row's sums NaN, which the GEMM computes again
+        if (lane == 0) reinterpret_cast<float *>(side)[t] = top >= 0x7F800000u ? __uint_as_float(0x7FC00000u) : up;
+        if (q4) {
+            // Q4 weights unpack as pairs (k, k + 4) of eight: order 0 4 1 5 2 6 3 7
+            const bool odd = lane & 1u;
+            const float r0 = __shfl_xor_sync(0xffffffffu, odd ? v[c][0] : v[c][2], 1), r1 = __shfl_xor_sync(0xffffffffu, odd ? v[c][1] : v[c][3], 1);
+            if (odd) { v[c][0] = r0; v[c][1] = v[c][2]; v[c][2] = r1; }
+            else     { v[c][3] = r1; v[c][2] = v[c][1]; v[c][1] = r0; }
+            // places 0-3 s.hi, 4-7 s.lo, 8-11 s.hi, 12-15 zero, beside the weights' b.hi, b.hi, b.lo, zero
+            if ((lane & 7u) == 0) {
+                const uint32_t b = lane >> 3;
+                const float s = sum[c] * down;
+                const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
+                __half *first = reinterpret_cast<__half *>(side + tok * 4u + sums_at(t, 0)), *second = reinterpret_cast<__half *>(side + tok * 4u + sums_at(t, 1));
+                first[b] = hi; first[4 + b] = lo;
+                second[b] = hi; second[4 + b] = __float2half_rn(0.f);
+            }
         }
+        store4(planes_out + block * 2 * planes * sub, sub, planes, t, lane * 4, v[c], down);
     }
-    store4(planes_out + block * 2 * planes * sub, sub, planes, t, lane * 4, v, down);
 }
 
 // ------------------------------------------------------------------------------------------ pieces
@@ -412,6 +425,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
     __shared__ SplitShared sh;
     constexpr uint32_t kRawChunk = kCols * raw_bytes(FMT);
     constexpr uint32_t kParts = 2 * PLANES, kDepth = kSlots / kParts;       // sub-tiles of a chunk, chunks in the ring
+    const uint32_t group = PLANES == 1 ? group_of(PLANES, p.k) : 1;
     uint8_t *ring = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sub = p.tok * 128u;                          // bytes of a token sub-tile, a multiple of 2048
     const uint32_t side = side_bytes(FMT, p.tok);               // a multiple of 64
@@ -428,7 +442,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
         for (uint32_t s = 0; s < 2; s++) {
             mbar_init(&sh.w_full[s], 4);
             mbar_init(&sh.d_empty[s], 8);
-            mbar_init(&sh.done[s], 1);
+            mbar_init(&sh.w_empty[s], 1);
+            mbar_init(&sh.d_full[s], 1);
         }
         mbar_init(&sh.flushed, 1);
         sh.failed = 0;
@@ -479,22 +494,24 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
             const bool leader = elect_one();
             const uint32_t ring16 = smem_u32(ring) >> 4;
             const uint32_t sub16 = sub >> 4;
-            bool ok = true;
+            uint32_t chunk = __shfl_sync(0xffffffffu, u_begin % p.chunks, 0), filled = 0;      // accumulators so far
+            bool ok = true, open = false;                       // open: the accumulator holds a chunk already
             for (uint32_t i = 0; i < count; i++) {
-                const uint32_t b = i & 1u, ph = (i >> 1) & 1u, s = i % kDepth;
-                const uint32_t d = tm + b * kMaxTok, w_hi = tm + 2 * kMaxTok + b * 128u, w_lo = w_hi + 64u;
+                const uint32_t stage = i & 1u, ph = (i >> 1) & 1u, s = i % kDepth, b = filled & 1u;
+                const bool close = group == 1 || chunk % group == group - 1 || chunk + 1 == p.chunks || i + 1 == count;
+                const uint32_t d = tm + b * kMaxTok, w_hi = tm + 2 * kMaxTok + stage * 128u, w_lo = w_hi + 64u;
                 // lane 0: accumulator, 1: weights, 2: sums (Q4), 4..: the chunk's sub-tiles
-                unsigned long long *bar = lane == 0 ? &sh.d_empty[b] : lane == 1 ? &sh.w_full[b] : lane == 2 ? &sh.sc_full[i % kScaleSlots] : &sh.slot_full[(s * kParts + lane - 4u) % kSlots];
-                const uint32_t parity = lane == 0 ? ph ^ 1u : lane == 1 ? ph : lane == 2 ? (i / kScaleSlots) & 1u : (i / kDepth) & 1u;
+                unsigned long long *bar = lane == 0 ? &sh.d_empty[b] : lane == 1 ? &sh.w_full[stage] : lane == 2 ? &sh.sc_full[i % kScaleSlots] : &sh.slot_full[(s * kParts + lane - 4u) % kSlots];
+                const uint32_t parity = lane == 0 ? ((filled >> 1) & 1u) ^ 1u : lane == 1 ? ph : lane == 2 ? (i / kScaleSlots) & 1u : (i / kDepth) & 1u;
                 ok = mbar_wait_lanes(bar, parity, lane < 2 || (FMT == MGQ_FMT_Q4 && lane == 2) || (lane >= 4 && lane < 4 + kParts), &sh.failed);
                 if (!ok) break;
                 tc_fence_after();
                 if (leader) {
                     const uint32_t x_lo = ring16 + s * kParts * sub16, x_hi = x_lo + (kParts - 2) * sub16;
                     if (FMT == MGQ_FMT_Q4)
-                        umma_f16(d, plain_desc(smem_u32(minima + b * kMinBytes)), plain_desc(smem_u32(side_ring + (i % kScaleSlots) * side + p.tok * 4u)), instr, 0u);
-                    if (FMT == MGQ_FMT_Q4) umma_f16_ts<true>(d, w_lo, x_hi, instr);
-                    else                   umma_f16_ts<false>(d, w_lo, x_hi, instr);
+                        umma_f16(d, plain_desc(smem_u32(minima + stage * kMinBytes)), plain_desc(smem_u32(side_ring + (i % kScaleSlots) * side + p.tok * 4u)), instr, open ? 1u : 0u);
+                    if (FMT == MGQ_FMT_Q4 || open) umma_f16_ts<true>(d, w_lo, x_hi, instr);
+                    else                           umma_f16_ts<false>(d, w_lo, x_hi, instr);
 #pragma unroll
                     for (uint32_t j = 1; j < 8; j++) umma_f16_ts<true>(d, w_lo + j * 8u, x_hi + (j / 4) * sub16 + (j % 4) * 2u, instr);
                     if (PLANES == 2)
@@ -502,10 +519,14 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                         for (uint32_t j = 0; j < 8; j++) umma_f16_ts<true>(d, w_hi + j * 8u, x_lo + (j / 4) * sub16 + (j % 4) * 2u, instr);
 #pragma unroll
                     for (uint32_t j = 0; j < 8; j++) umma_f16_ts<true>(d, w_hi + j * 8u, x_hi + (j / 4) * sub16 + (j % 4) * 2u, instr);
-                    umma_commit(&sh.done[b]);
+                    umma_commit(&sh.w_empty[stage]);
                     umma_commit(&sh.slot_empty[s]);
+                    if (close) umma_commit(&sh.d_full[b]);
                 }
                 __syncwarp();
+                open = !close;
+                if (close) filled++;
+                if (++chunk == p.chunks) chunk = 0;
             }
             if (!ok && leader) {                                // products in flight end before the CTA does
                 umma_commit(&sh.flushed);
@@ -522,7 +543,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
         const uint32_t first = wg * half * 16, mine = wg ? groups - half : half;
         const uint32_t j = quad * 32 + lane;                    // weight column within the tile
         float acc[4][16];                                       // tokens first + 16 g + e
-        uint32_t i = 0;
+        uint32_t i = 0, filled = 0;                             // chunks, accumulators so far
         for (uint32_t u = u_begin; u < u_end;) {
             const uint32_t tile = u / p.chunks, c0 = u % p.chunks;
             const uint32_t c1 = min(p.chunks, c0 + (u_end - u));
@@ -531,8 +552,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
 #pragma unroll
                 for (int e = 0; e < 16; e++) acc[g][e] = 0.f;
             for (uint32_t c = c0; c < c1; c++, i++) {
-                const uint32_t b = i & 1u, sc = i % kScaleSlots;
-                mbar_wait_lanes(lane == 0 ? &sh.done[b] : &sh.sc_full[sc], lane == 0 ? (i >> 1) & 1u : (i / kScaleSlots) & 1u, lane < 2, &sh.failed);
+                if (group > 1 && c % group != group - 1 && c + 1 != c1) continue;            // the next chunk goes into the same accumulator
+                const uint32_t b = filled & 1u, sc = i % kScaleSlots, span = group > 1 ? min(c % group, c - c0) + 1 : 1;
+                const uint32_t x = i + 1 - lane;                // lane 0: the accumulator, 1..span: scales of its chunks
+                mbar_wait_lanes(lane == 0 ? &sh.d_full[b] : &sh.sc_full[x % kScaleSlots], lane == 0 ? (filled >> 1) & 1u : (x / kScaleSlots) & 1u, lane <= span, &sh.failed);
+                filled++;
                 __syncwarp();                                   // tcgen05.ld is warp-collective
                 tc_fence_after();
                 const uint32_t from = tmem + lane_addr + b * kMaxTok + first;
@@ -545,7 +569,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                 __syncwarp();
                 if (lane == 0) {
                     mbar_arrive(&sh.d_empty[b]);
-                    mbar_arrive(&sh.sc_empty[sc]);
+                    for (uint32_t x = 0; x < span; x++) mbar_arrive(&sh.sc_empty[(i - x) % kScaleSlots]);
                 }
             }
             u += c1 - c0;
@@ -651,7 +675,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
             asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncwarp();
             const uint8_t *src = raw + (i % kRaw) * kRawChunk + (quad * 32 + lane) * raw_bytes(FMT);
-            mbar_wait(&sh.done[group], ((i >> 1) & 1u) ^ 1u, &sh.failed, &g_split_error);
+            mbar_wait(&sh.w_empty[group], ((i >> 1) & 1u) ^ 1u, &sh.failed, &g_split_error);
             __syncwarp();
             tc_fence_after();
             const uint32_t dst = tmem_w + ((quad * 32u) << 16) + group * 128u;
@@ -814,7 +838,7 @@ int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const 
         p.partial = reinterpret_cast<float *>(side_dev + all_side);
         p.counters = reinterpret_cast<unsigned int *>(side_dev + all_side + part_bytes);
         const bool vec = reinterpret_cast<uintptr_t>(p.a) % 16 == 0;
-        const unsigned long long warps = (unsigned long long)p.m * p.chunks;
+        const unsigned long long warps = (unsigned long long)p.m * ((p.chunks + group_of(planes, k) - 1) / group_of(planes, k));
         split_rows_kernel<<<(uint32_t)((warps + 7) / 8), 256, 0, stream>>>(p.a, bf16, vec, ws, side_dev, p.counters, p.tiles, p.m, k, p.tok, p.chunks, planes, q4);
         int rc = cuda_check((int)cudaGetLastError(), "split_rows_kernel", __FILE__, __LINE__);
         if (rc == MGQ_OK)
