@@ -69,6 +69,10 @@ size_t attention_workspace_bytes(uint32_t num_kv_heads, uint32_t head_dim, uint3
 int launch_cached_attention(const float *q, const float *k_cache, const float *v_cache, const uint32_t *kv_pos, float *out,
                             uint32_t num_heads, uint32_t num_kv_heads, uint32_t head_dim, uint32_t max_seq, void *workspace,
                             void *stream);
+// launch_rope_cache and launch_cached_attention in one; the destinations and `out` must not overlap the sources.
+int launch_rope_attention(const float *q_src, float *q_dst, const float *k_src, float *k_dst, const float *v_src, float *k_cache, float *v_cache,
+                          const uint32_t *kv_pos, float *out, uint32_t num_heads, uint32_t num_kv_heads, uint32_t head_dim, float theta,
+                          uint32_t max_seq, void *workspace, void *stream);
 size_t argmax_workspace_bytes();
 int launch_argmax(const float *logits, uint32_t n, void *workspace, uint32_t *out_token, uint32_t *next_token, uint32_t *kv_pos,
                   uint32_t *history, uint32_t history_cap, uint32_t advance, void *stream);

@@ -82,6 +82,8 @@ struct Dispatch {
     bool scratch = false;         // workspace is the session's shared scratch
     std::vector<int> members;     // linear group: the node of each layer
     int exchange = -1;            // all_gather: which exchange; GEMV: the exchange it pushes its columns to (-1: none)
+    int rope = -1;                // cached attention: the rotation and cache write right in front of it, which it runs along
+    bool deferred = false;        // ... and that dispatch: left to the attention
     bool push_done = false;       // all_gather: the producing GEMV has pushed the slice already
     std::string label;
 };
@@ -206,6 +208,7 @@ struct mgq_session {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     uint64_t launches = 0;
+    size_t deferred = 0;               // dispatches that another one runs along
     int device = 0;
     // row-dynamic graphs: capacity and current count per MGQ_ROWS_* index; counts of the captured graph
     uint32_t row_cap[3] = {0, 0, 0}, row_count[3] = {0, 1, 1}, graph_rows[3] = {0, 0, 0};
@@ -946,6 +949,32 @@ void merge_rope_cache(mgq_session *s)
     }
 }
 
+// A rotation and cache write followed by the attention over the same vectors, caches and position runs as one kernel.  Both
+// keep their place in the plan, and all their outputs are written.
+void pair_rope_attention(mgq_session *s)
+{
+    std::vector<Dispatch> &ds = s->dispatches;
+    for (size_t i = 0; i + 1 < ds.size(); i++) {
+        Dispatch &r = ds[i], &a = ds[i + 1];
+        if (r.shader != MGQ_SHADER_ROPE_CACHE_WRITE || a.shader != MGQ_SHADER_CACHED_ATTENTION) continue;
+        const uint32_t dim = r.params[2];
+        if (a.params[3] != dim || (dim != 64 && dim != 128) || a.params[0] != r.params[3]) continue;
+        if ((size_t)a.params[1] * dim != r.params[0] || (size_t)a.params[2] * dim != r.params[1]) continue;
+        auto at = [&](int node) { return static_cast<const char *>(s->ptr(node)); };
+        if (at(a.in[0]) != at(r.out) || at(a.in[1]) != at(r.extra[1]) || at(a.in[2]) != at(r.extra[2]) || at(a.in[3]) != at(r.in[3])) continue;
+        // some CTAs still read the sources while others write: nothing may share memory
+        const size_t q = (size_t)r.params[0] * 4, kv = (size_t)r.params[1] * 4;
+        const std::pair<const char *, size_t> from[3] = {{at(r.in[0]), q}, {at(r.in[1]), kv}, {at(r.in[2]), kv}}, to[3] = {{at(r.out), q}, {at(r.extra[0]), kv}, {at(a.out), q}};
+        bool apart = true;
+        for (const auto &f : from)
+            for (const auto &t : to) apart = apart && (f.first + f.second <= t.first || t.first + t.second <= f.first);
+        if (!apart) continue;
+        r.deferred = true;
+        s->deferred++;
+        a.rope = (int)i;
+    }
+}
+
 // Norm(q), Norm(k), QueryTemperature, CacheAppend(k), CacheAppend(v) in a row, as an attention layer builds
 // them, become one dispatch; the normed q and k have no other reader.
 void merge_attention_inputs(mgq_session *s)
@@ -1524,6 +1553,7 @@ int mgq_build_inference_session(const mgq_graph *g, mgq_session **out)
     if (g_fuse_rope_cache) merge_rope_cache(s);
     if (g_fuse_mixer) merge_attention_inputs(s);
     if (g_fuse_mixer) group_linears(s);
+    if (g_fuse_rope_cache) pair_rope_attention(s);
     for (Dispatch &d : s->dispatches) {
         if (d.shader != MGQ_SHADER_LINEAR) continue;
         uint32_t n = 0;
@@ -1980,10 +2010,17 @@ static int run_dispatch(mgq_session *s, const Dispatch &d)
         case MGQ_SHADER_ROPE_DYNAMIC: return mgq_rope_dynamic(f(0), outp, u(1), d.params[0], d.params[1], d.params[3], d.f0, s->stream);
         case MGQ_SHADER_CACHE_WRITE: return mgq_cache_write(f(0), outp, u(2), d.params[0], d.params[1], s->stream);
         case MGQ_SHADER_ROPE_CACHE_WRITE:
+            if (d.deferred) return MGQ_OK;
             return mgq_rope_cache_write(f(0), outp, f(1), static_cast<float *>(s->ptr(d.extra[0])), f(2), static_cast<float *>(s->ptr(d.extra[1])),
                                         static_cast<float *>(s->ptr(d.extra[2])), u(3), d.params[0], d.params[1], d.params[2], d.f0,
                                         d.params[3], s->stream);
         case MGQ_SHADER_CACHED_ATTENTION:
+            if (d.rope >= 0) {
+                const Dispatch &r = s->dispatches[d.rope];
+                auto rf = [&](int node) { return static_cast<float *>(s->ptr(node)); };
+                return mgq::launch_rope_attention(rf(r.in[0]), rf(r.out), rf(r.in[1]), rf(r.extra[0]), rf(r.in[2]), rf(r.extra[1]), rf(r.extra[2]), u(3), outp, d.params[1],
+                                                  d.params[2], d.params[3], r.f0, d.params[0], d.workspace, s->stream);
+            }
             return mgq_cached_attention(f(0), f(1), f(2), u(3), outp, d.params[1], d.params[2], d.params[3], d.params[0], d.workspace, s->stream);
         case MGQ_SHADER_SWIGLU: return mgq_swiglu(f(0), f(1), outp, d.params[0] / d.params[1], d.params[1], d.params[2], s->stream);
         case MGQ_SHADER_SWIGLU_CONCAT:
@@ -2091,7 +2128,7 @@ int mgq_session_step(mgq_session *s)
     }
     nvtxRangePop();
     if (rc) return rc;
-    s->launches += s->dispatches.size() + (s->greedy ? 1 : 0) + (s->exchanges.empty() ? 0 : 1);
+    s->launches += s->dispatches.size() - s->deferred + (s->greedy ? 1 : 0) + (s->exchanges.empty() ? 0 : 1);
     return MGQ_OK;
 }
 

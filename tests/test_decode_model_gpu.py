@@ -292,3 +292,27 @@ def test_gemv_bt_matches_float64(k, n):
     assert bool((y[n:] == 123.0).all())                       # nothing written past the end
     with pytest.raises(Exception):
         check(lib.mgq_gemv_bt(xd.data_ptr(), bd.data_ptr(), y.data_ptr(), 6, n, None))
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim", [(8, 1, 64), (3, 3, 64), (4, 2, 128), (7, 1, 128)])
+def test_rotation_inside_the_attention_is_the_separate_kernels(heads, kv_heads, head_dim):
+    """Positions at the edges of the attention's chunks of 64, the last rows of the cache and behind it: the same bits, in
+    the step itself and in the steps after it that read its key and value from the cache."""
+    from meganeura_b200 import decode_model as M, ops
+    cfg = M.DecoderConfig("rope", 512, heads * head_dim, 2, heads, kv_heads, head_dim, 512, 1e-5, 1e4, O.FMT_Q8, O.FMT_Q4, O.FMT_Q8)
+    outs = []
+    for merged in (0, 1):
+        ops.set_option("session.fuse_rope_cache", merged)
+        try:
+            s, _ = _build(cfg, seed=5)
+        finally:
+            ops.set_option("session.fuse_rope_cache", 1)
+        got = []
+        for pos in (0, 1, 62, 63, 64, 65, MAX_SEQ - 1, MAX_SEQ, MAX_SEQ + 70, 64):
+            s.set_input_u32("token_ids", [7 * pos % 512])
+            s.set_input_u32("kv_pos", [pos])
+            s.step()
+            s.wait()
+            got.append(s.read_output(512))
+        outs.append(np.stack(got))
+    assert np.isfinite(outs[0]).all() and np.array_equal(outs[0], outs[1])
