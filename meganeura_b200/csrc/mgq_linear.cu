@@ -39,11 +39,11 @@ __global__ void __launch_bounds__(128) linear_gemv_kernel(const __grid_constant_
         const uint32_t n = min(n0 + (uint32_t)(GLU ? r / 2 : r), s.n - 1u);
         w[r] = static_cast<const __nv_bfloat16 *>((GLU && (r & 1)) ? s.w2 : s.w) + (size_t)n * k;
     }
-    // weights are immutable: start moving the first pieces towards L2 before waiting for the activations
-    if (lane * 64u < k) {
+    // weights are immutable: start moving all of the rows towards L2 before waiting for the activations, and keep eight loads of a
+    // lone row in flight (Tobovik, 777 + 12 tokens: 9321 -> 9052 us; only the first 2048 k and four loads before)
+    for (uint32_t c = lane * 64u; c < k; c += 2048u)
 #pragma unroll
-        for (int r = 0; r < R; r++) asm volatile("prefetch.global.L2 [%0];" ::"l"(w[r] + lane * 64u));
-    }
+        for (int r = 0; r < R; r++) asm volatile("prefetch.global.L2 [%0];" ::"l"(w[r] + c));
     pdl_wait();
     const XT *x = static_cast<const XT *>(s.a) + (size_t)row0 * k;
     float acc[M][R];
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(128) linear_gemv_kernel(const __grid_constant_
         for (int r = 0; r < R; r++) acc[i][r] = 0.f;
     if (VEC) {
         const uint32_t chunks = k / 8;
-#pragma unroll(M <= 2 ? 4 : 2)
+#pragma unroll(M <= 2 ? (R == 1 ? 8 : 4) : 2)
         for (uint32_t c = lane; c < chunks; c += 32) {
             uint4 q[R];
 #pragma unroll
