@@ -876,6 +876,11 @@ __global__ void __launch_bounds__(kStepThreads) step_kernel(const __grid_constan
     }
     pdl_launch_dependents();
     pdl_wait();
+    // the first columns' state and values are requested before the decay is worked out
+    float S[1][RPT];
+    const uint32_t first = part * kStepCols + t / 8;
+    load_keys<RPT>(p.state + ((size_t)head * vdim + (first < vdim ? first : 0)) * kp, ks, kp, S[0]);
+    float v[1] = {first < vdim ? p.v[head * vdim + first] : 0.f};
     for (uint32_t i = t; i < (uint32_t)KS; i += kStepThreads) {
         sq[i] = i < dim ? p.q[head * dim + i] : 0.f;
         sk[i] = i < dim ? p.k[head * dim + i] : 0.f;
@@ -916,11 +921,13 @@ __global__ void __launch_bounds__(kStepThreads) step_kernel(const __grid_constan
         const uint32_t col = c0 + t / 8;
         const bool live = col < vdim;
         float *srow = p.state + ((size_t)head * vdim + (live ? col : 0)) * kp;
-        float S[1][RPT], nn[RPT], out1[1], den;
-        load_keys<RPT>(srow, ks, kp, S[0]);
+        float nn[RPT], out1[1], den;
+        if (col != first) {
+            load_keys<RPT>(srow, ks, kp, S[0]);
+            v[0] = live ? p.v[head * vdim + col] : 0.f;
+        }
 #pragma unroll
         for (int i = 0; i < RPT; i++) nn[i] = n[i];
-        const float v[1] = {live ? p.v[head * vdim + col] : 0.f};
         token_update<MODE, RPT, 1, true>(sq + ks * 4, sk + ks * 4, sw + ks * 4, u, v, a, b, S, nn, out1, den);
         float out = sum8(out1[0]);
         if (MODE == kGla) out *= p.qscale;
