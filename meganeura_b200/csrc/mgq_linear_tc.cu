@@ -12,7 +12,10 @@
 //               descriptors stay in uniform registers.
 // A stage's wait and commit take the issuing warp about 300 cycles, as long as 4 MMAs of 128 columns run: TN of 128 and
 // 64 therefore take 128 k per stage.
-//   warps 2-5   epilogue of one accumulator while the other is being filled (2 x TN TMEM columns).
+//   warps 2-9   epilogue of one accumulator while the other is being filled (2 x TN TMEM columns): 32 rows by every other
+//               32 columns each.  A GLU takes a warp about 40 instructions per output; four
+//               warps were slower than the MMAs (2048 x 6144 x 2048: 105 us, with eight 86).  Two blocks of 128 rows per tile
+//               without a second accumulator set were slower still (118 us).
 // Every mbarrier wait is bounded; when one runs out the device-wide error word is raised (mgq_device_status) and the roles end.
 #include <cuda_fp16.h>
 
@@ -26,7 +29,7 @@ namespace {
 
 constexpr uint32_t TM = 128, TK = 64;                // rows of a tile, k of a box
 constexpr uint32_t kBytesA = TM * TK * 2;
-constexpr int kThreads = 192;
+constexpr int kThreads = 320;
 
 __device__ unsigned int g_linear_tc_error = 0;
 
@@ -45,7 +48,7 @@ struct __align__(8) LinearShared {
     volatile int failed;
 };
 
-constexpr uint32_t kStgBytes = 32 * 36 * 4;              // epilogue staging of one warp: 32 rows x 32 columns, padded rows
+constexpr uint32_t kStgBytes = 32 * 20 * 4;              // epilogue staging of one warp: 32 rows x 16 columns, padded rows
 
 // Two values of a 2-byte output: bf16 for a GLU, f16 otherwise.
 template <bool BF16> __device__ __forceinline__ uint32_t pack_pair(float x, float y)
@@ -95,7 +98,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc_kernel(const __grid_con
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(&sh.acc_full[b], 1);
-            mbar_init(&sh.acc_empty[b], 4);
+            mbar_init(&sh.acc_empty[b], 8);
         }
         sh.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -116,33 +119,34 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc_kernel(const __grid_con
 
     constexpr uint32_t kBoxes = boxes<TN>(), kBytesW = TN * TK * 2;
     if (warp == 0) {
-        // lane = box of the stage * kLoads + operand
+        // lane = box of the stage * kLoads + operand; the whole warp stays together, or every lane's wait would run by itself
         constexpr uint32_t kLoads = GLU ? 3 : 2;
-        if (lane < kBoxes * kLoads) {
-            const uint32_t box = lane / kLoads, what = lane % kLoads;
-            const uint32_t offset = what == 0 ? box * kBytesA : kBoxes * kBytesA + box * kBytesW + (what == 2 ? COLS * TK * 2 : 0);
-            uint32_t it = 0;
-            int armed = -1;
-            bool ok = true;
-            for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-                const Tile tl = find_tile<COLS>(g, tile, mt);
-                const uint32_t nk = (g.seg[tl.si].k + TK * kBoxes - 1) / (TK * kBoxes);
-                const CUtensorMap *map = what == 0 ? &maps.a[tl.si] : what == 1 ? &maps.w[tl.si] : &maps.w[1];
-                const int y = (int)(what == 0 ? tl.m0 : tl.n0);
-                for (uint32_t kc = 0; kc < nk; kc++, it++) {
-                    const uint32_t s = it % S, ph = (it / S) & 1u;
-                    ok = mbar_wait(&sh.empty[s], ph ^ 1u, &sh.failed, &g_linear_tc_error);
-                    if (!ok) break;
-                    if (lane == 0) mbar_arrive_expect_tx(&sh.full[s], kStage);      // the phase stays open for this arrival
-                    tma_load_2d(ring + s * kStage + offset, map, (int)((kc * kBoxes + box) * TK), y, &sh.full[s]);
-                    armed = (int)it;
-                }
+        const uint32_t box = lane / kLoads, what = lane % kLoads;
+        const bool mine = lane < kBoxes * kLoads;
+        const uint32_t offset = what == 0 ? box * kBytesA : kBoxes * kBytesA + box * kBytesW + (what == 2 ? COLS * TK * 2 : 0);
+        uint32_t it = 0;
+        int armed = -1;
+        bool ok = true;
+        for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+            const Tile tl = find_tile<COLS>(g, tile, mt);
+            const uint32_t nk = (g.seg[tl.si].k + TK * kBoxes - 1) / (TK * kBoxes);
+            const CUtensorMap *map = what == 0 ? &maps.a[tl.si] : what == 1 ? &maps.w[tl.si] : &maps.w[1];
+            const int y = (int)(what == 0 ? tl.m0 : tl.n0);
+            for (uint32_t kc = 0; kc < nk; kc++, it++) {
+                const uint32_t s = it % S, ph = (it / S) & 1u;
+                ok = __all_sync(0xffffffffu, mbar_wait(&sh.empty[s], ph ^ 1u, &sh.failed, &g_linear_tc_error));
+                if (!ok) break;
+                if (lane == 0) mbar_arrive_expect_tx(&sh.full[s], kStage);          // the phase stays open for this arrival
+                __syncwarp();
+                if (mine) tma_load_2d(ring + s * kStage + offset, map, (int)((kc * kBoxes + box) * TK), y, &sh.full[s]);
+                __syncwarp();
+                armed = (int)it;
             }
-            // after a failure: let the copies in flight land before the CTA exits
-            if (!ok)
-                for (int i = armed; i >= 0 && i > armed - S; i--)
-                    for (uint32_t w = 0; w < kWaitLimit && !mbar_try_wait(&sh.full[i % S], ((uint32_t)i / S) & 1u); w++) { }
         }
+        // after a failure: let the copies in flight land before the CTA exits
+        if (!ok && lane == 0)
+            for (int i = armed; i >= 0 && i > armed - S; i--)
+                for (uint32_t w = 0; w < kWaitLimit && !mbar_try_wait(&sh.full[i % S], ((uint32_t)i / S) & 1u); w++) { }
     } else if (warp == 1) {
         const bool leader = elect_one();
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0), base16 = smem_u32(ring) >> 4;
@@ -174,8 +178,8 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc_kernel(const __grid_con
             __syncwarp();
         }
     } else {
-        const uint32_t quad = warp & 3u;                 // TMEM lanes this warp may read
-        float *stg = reinterpret_cast<float *>(ring + S * kStage) + quad * (kStgBytes / 4);
+        const uint32_t quad = warp & 3u, half = (warp - 2) / 4;      // TMEM lanes this warp may read; every other 32 columns
+        float *stg = reinterpret_cast<float *>(ring + S * kStage) + (warp - 2) * (kStgBytes / 4);
         uint32_t at = 0;
         for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, at++) {
             const uint32_t b = at & 1u;
@@ -189,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc_kernel(const __grid_con
             const uint32_t acc = tmem + ((quad * 32u) << 16) + b * TN;
             const bool narrow = (GLU && g.out_bf16) || (!GLU && g.out_f16);       // 2-byte outputs
 #pragma unroll 1
-            for (uint32_t c0 = 0; c0 < COLS; c0 += 32) {
+            for (uint32_t c0 = half * 32; c0 < COLS; c0 += 64) {
                 const uint32_t col = tl.n0 + c0;
                 if (col >= n) break;                     // uniform over the warp
                 const bool whole = col + 32 <= n && n % (narrow ? 8 : 4) == 0;
@@ -246,25 +250,28 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc_kernel(const __grid_con
                     }
                     __syncwarp();
                 } else if (whole) {
-                    float *mine = stg + lane * 36;
-                    float4 add[8];
+                    float *mine = stg + lane * 20;
+                    float4 add[2][4];
 #pragma unroll
                     for (int i = 0; i < 8; i++) {        // all addends requested before the first one is needed
-                        const uint32_t r = i * 4 + lane / 8;
-                        add[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (!GLU && sg.addend && rbase + r < g.m) add[i] = *reinterpret_cast<const float4 *>(sg.addend + (size_t)(rbase + r) * n + col + (lane & 7u) * 4);
+                        const uint32_t r = i % 4 * 8 + lane / 4;
+                        add[i / 4][i % 4] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (!GLU && sg.addend && rbase + r < g.m) add[i / 4][i % 4] = *reinterpret_cast<const float4 *>(sg.addend + (size_t)(rbase + r) * n + col + i / 4 * 16 + (lane & 3u) * 4);
                     }
 #pragma unroll
-                    for (int e = 0; e < 32; e += 4) *reinterpret_cast<float4 *>(mine + e) = make_float4(y[e], y[e + 1], y[e + 2], y[e + 3]);
-                    __syncwarp();
+                    for (int x = 0; x < 2; x++) {        // 16 columns at a time
 #pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const uint32_t r = i * 4 + lane / 8;
-                        float4 v = *reinterpret_cast<const float4 *>(stg + r * 36 + (lane & 7u) * 4);
-                        v.x += add[i].x; v.y += add[i].y; v.z += add[i].z; v.w += add[i].w;
-                        if (rbase + r < g.m) *reinterpret_cast<float4 *>(static_cast<float *>(sg.out) + (size_t)(rbase + r) * n + col + (lane & 7u) * 4) = v;
+                        for (int e = 0; e < 16; e += 4) *reinterpret_cast<float4 *>(mine + e) = make_float4(y[x * 16 + e], y[x * 16 + e + 1], y[x * 16 + e + 2], y[x * 16 + e + 3]);
+                        __syncwarp();
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            const uint32_t r = i * 8 + lane / 4;
+                            float4 v = *reinterpret_cast<const float4 *>(stg + r * 20 + (lane & 3u) * 4);
+                            v.x += add[x][i].x; v.y += add[x][i].y; v.z += add[x][i].z; v.w += add[x][i].w;
+                            if (rbase + r < g.m) *reinterpret_cast<float4 *>(static_cast<float *>(sg.out) + (size_t)(rbase + r) * n + col + x * 16 + (lane & 3u) * 4) = v;
+                        }
+                        __syncwarp();
                     }
-                    __syncwarp();
                 } else if (rbase + lane < g.m) {         // ragged columns
                     const size_t o = (size_t)(rbase + lane) * n + col;
 #pragma unroll
@@ -317,7 +324,7 @@ int launch_tc(const LinearGroup &g, cudaStream_t stream)
         tiles += (s.n + COLS - 1) / COLS;
     }
     tiles *= (g.m + TM - 1) / TM;
-    const size_t smem = (size_t)stages<TN>() * stage_bytes<TN>() + 4 * kStgBytes + 1024;
+    const size_t smem = (size_t)stages<TN>() * stage_bytes<TN>() + 8 * kStgBytes + 1024;
     if (int rc = allow_smem(linear_tc_kernel<TN, GLU>, smem)) return rc;
     return launch(linear_tc_kernel<TN, GLU>, dim3(min(tiles, 148u)), dim3(kThreads), smem, stream, maps, g, tiles);
 }
