@@ -37,9 +37,10 @@
 // What bounds it: of the 2650 cycles that a chunk of 128 x 128 takes with f32 activations the tensor core needs 1536 (2100 and 1024
 // for bf16), the rest is the hand-over of a weight stage: products of chunk i - 2 done, conversion (1500 cycles, four warps),
 // products of chunk i; 52 % of the issue slots are taken.  Measured and dropped: weight stages of 64 k (147 instead
-// of 112 us for bf16, twice the waits), two issuing warps and both groups on every chunk (no change).
-// 512 x 4096 x 12288 Q4 f32: 138 us against 1991 on the CUDA cores; 512 x 4096 x 14336 Q8 bf16: 127 against 141 us of a
-// kernel with one 112-column strip of bf16 weight pairs per CTA and 512 tokens.
+// of 112 us for bf16, twice the waits), two issuing warps, both groups on every chunk, two token tiles per converted weight (no change).
+// In a long run (the power cap adds a tenth) 512 x 4096 x 12288 Q4 f32 takes 161 us against 1993 on the CUDA cores, 512 x 4096 x 14336 Q8
+// bf16 143 against 147 us of a kernel with one 112-column strip of bf16 weight pairs per CTA and 512 tokens, whose sums were
+// 9.4e-6 off.
 //
 // Every mbarrier wait is bounded; when one runs out the device-wide error word is raised (mgq_device_status reports
 // MGQ_ERR_TIMEOUT), the roles run to their ends without waiting and the CTA frees its TMEM.
