@@ -160,7 +160,9 @@ def test_subnormal_scales_follow_cpu_dequantize(coracle):
 @pytest.mark.parametrize("fmt", FMTS)
 @pytest.mark.parametrize("route", ["gemv", "auto"])
 # block counts that are not multiples of 4 and so large that no group of 2 or 4 columns fits a CTA (65, 130, 275), and the last ones that do
-@pytest.mark.parametrize("m,k,n", [(1, 2080, 12), (2, 2016, 36), (1, 4160, 66), (2, 4096 - 64, 34), (4, 8800, 40), (3, 2080, 7)])
+@pytest.mark.parametrize("m,k,n", [(1, 2080, 12), (2, 2016, 36), (1, 4160, 66), (2, 4096 - 64, 34), (4, 8800, 40), (3, 2080, 7),
+                                   # rows at the lines between GEMV and GEMM
+                                   (4, 1056, 64), (5, 1056, 64), (3, 4160, 34), (4, 4128, 36), (8, 4096, 4896), (9, 4096, 4896), (16, 8192, 2448)])
 def test_block_counts_that_no_column_group_fits(coracle, fmt, route, m, k, n):
     w = O.synth_weights(fmt, k, n, seed=k + n)
     x = _x(m, k, k * 7 + n)
