@@ -8,11 +8,11 @@
 // Operands are sums of f16 values, whose products the tensor cores form exactly:
 //   activations  x = (hi + lo) * 2^e, e per row and 128 k (split_rows_kernel): all 24 bits of an f32 but the last
 //                one or two; a bf16 value fits hi alone, so that case has one plane and two products instead of three.
-//   weights      code * scale has at most 19 bits: hi = rn16(code * d), lo = fma16(code, d, -hi), both exact, two
-//                instructions for two weights.  Every such product is a multiple of 2^-24, so nothing is lost for small
-//                scales.  Q4 codes are centred (q - 8); what is left of the block's minimum, b = m + 8 d, times the
-//                block's sum s of activations takes one more step of K = 16 per chunk: for each of the chunk's four
-//                blocks b.hi s.hi + b.hi s.lo + b.lo s.hi.
+//   weights      Q8: code * d has at most 19 bits, hi = rn16(code * d), lo = fma16(code, d, -hi), both exact, two
+//                instructions for two weights.  Q4: hi = fma16(code, d, m), lo = rn16(code * d + m - hi), the difference
+//                in f32: 2^-23 of the weight at most is left.  Both are multiples of 2^-24 as d and m are, so nothing is
+//                lost for small scales.  The minimum is part of the weight: d * sum(code x) + m * sum(x) would cancel where
+//                a large activation meets a weight near zero (2.2e-5 off for a value of 1000 in every 128, m = -7 d).
 // The tensor core truncates when it adds to its f32 accumulator, which over a long K would cost more than f32 sums do
 // (9e-6 for bf16 activations and K = 4096 in one accumulator).  So one accumulator takes a chunk of 128 k only, the small
 // products first; then it is added to a register sum in f32, times 2^e: 2.2e-7 off the exact product at K = 4096 and 2.0e-7 at
@@ -25,13 +25,13 @@
 // tile is spread over several CTAs, each leaves its partial sums in the workspace and the one that finishes last adds
 // them up in order: results do not depend on timing.
 //   warp 0        token planes, 64 k of one plane per copy (cp.async.bulk of a block that split_rows_kernel has laid
-//                 out in the 128-byte swizzle), ring of 8; scales and (Q4) sums of a chunk, ring of 8.
+//                 out in the 128-byte swizzle), ring of 8; scales of a chunk, ring of 8.
 //   warp 1        MMA issue: tcgen05.mma.kind::f16, M=128 (weight columns), N=tokens, K=16, A in TMEM.
 //   warps 4-11    drain: 32 weight columns by half of the tokens per warp, sums in registers; results.
 //   warps 12-19   weights: two groups of four, chunks in turn; cp.async of a warp's 32 columns two chunks
 //                 of its own ahead, conversion, tcgen05.st.
 // TMEM: two accumulators of 128 columns, two weight stages of 64 (hi) + 64 (lo) columns.
-// Sums that are not finite (non-finite inputs, |code * scale| or |m + 8 d| beyond the f16 range) are computed again
+// Sums that are not finite (non-finite inputs, a weight beyond the f16 range) are computed again
 // element by element on the CUDA cores.
 //
 // What bounds it: of the 2650 cycles that a chunk of 128 x 128 takes with f32 activations the tensor core needs 1536 (2100 and 1024
@@ -75,7 +75,7 @@ struct SplitParams {
     const float *addend;
     float *c;
     const uint8_t *planes;          // [m tile][chunk][slot][tokens * 128 B]
-    const uint8_t *side;            // [m tile][chunk]: scales [tokens] f32 | Q4: sums [tokens][16] f16, see sums_at
+    const float *scales;            // [m tile][chunk][tokens]
     float *partial;                 // [CTA][2][128 tokens][128 columns]
     unsigned int *counters;         // one per tile
     unsigned long long num_blocks;
@@ -96,11 +96,6 @@ struct __align__(16) SplitShared {
 };
 
 __host__ __device__ constexpr uint32_t raw_bytes(int fmt) { return fmt == MGQ_FMT_Q8 ? 144u : 80u; }      // of a column and chunk: Q4 = 16 header bytes | 64 nibble bytes
-
-// K = 16 operands of the minimum step: no swizzle, 8 rows x 16 bytes side by side, the two halves of K 128 bytes apart.
-__host__ __device__ constexpr uint32_t sums_at(uint32_t row, uint32_t half) { return (row >> 3) * 256u + half * 128u + (row & 7u) * 16u; }
-__host__ __device__ constexpr uint32_t side_bytes(int fmt, uint32_t tok) { return tok * (fmt == MGQ_FMT_Q4 ? 36u : 4u); }
-constexpr uint32_t kMinBytes = kCols * 32;         // minima of a chunk
 
 // CTA that owns unit u, and first unit of CTA g, when `units` are shared out over `ctas`.
 __host__ __device__ inline uint32_t unit_owner(uint32_t u, uint32_t units, uint32_t ctas)
@@ -147,7 +142,7 @@ __device__ __forceinline__ void store4(uint8_t *block, uint32_t sub, uint32_t pl
 
 // A warp per row and group of chunks.  Bound by the read of the activations (8 MB for 512 x 4096 f32) and as many bytes written,
 // all of which stay in L2 for the GEMM behind it.
-__global__ void __launch_bounds__(256) split_rows_kernel(const void *a, bool bf16, bool vec, uint8_t *planes_out, uint8_t *side_out, unsigned int *counters, uint32_t tiles,
+__global__ void __launch_bounds__(256) split_rows_kernel(const void *a, bool bf16, bool vec, uint8_t *planes_out, float *scales_out, unsigned int *counters, uint32_t tiles,
                                                          uint32_t m, uint32_t k, uint32_t tok, uint32_t chunks, uint32_t planes, bool q4)
 {
     pdl_launch_dependents();
@@ -157,7 +152,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const void *a, bool bf1
     const uint32_t row = gid / groups, first_chunk = gid % groups * span;
     if (row >= m) return;
     const uint32_t mt = row / tok, t = row % tok, sub = tok * 128u;
-    float v[2][4] = {}, sum[2] = {};                            // sum: of this lane's block of 32
+    float v[2][4] = {};
     uint32_t top = 0;                                           // largest magnitude by its bits: NaN stays the largest
 #pragma unroll
     for (uint32_t c = 0; c < 2; c++) {
@@ -178,16 +173,9 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const void *a, bool bf1
         }
     }
 #pragma unroll
-    for (uint32_t c = 0; c < 2; c++) {
+    for (uint32_t c = 0; c < 2; c++)
 #pragma unroll
         for (int i = 0; i < 4; i++) top = max(top, __float_as_uint(v[c][i]) & 0x7FFFFFFFu);
-        if (q4) {
-            sum[c] = (v[c][0] + v[c][1]) + (v[c][2] + v[c][3]);
-#pragma unroll
-            for (int o = 1; o < 8; o <<= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
-            top = max(top, __float_as_uint(sum[c]) & 0x7FFFFFFFu);
-        }
-    }
     top = __reduce_max_sync(0xffffffffu, top);
     float down, up;
     pick_scale(__uint_as_float(top), down, up);
@@ -195,24 +183,15 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const void *a, bool bf1
     for (uint32_t c = 0; c < 2; c++) {
         if (c >= span || first_chunk + c >= chunks) break;      // uniform over the warp
         const size_t block = (size_t)mt * chunks + first_chunk + c;
-        uint8_t *side = side_out + block * side_bytes(q4 ? MGQ_FMT_Q4 : MGQ_FMT_Q8, tok);
-        // not finite: a NaN scale makes the row's sums NaN, which the GEMM computes again
-        if (lane == 0) reinterpret_cast<float *>(side)[t] = top >= 0x7F800000u ? __uint_as_float(0x7FC00000u) : up;
+        // not finite, or so large (from 2^120 on) that f32 sums overflow on their way: a NaN scale makes the row's sums NaN, which the
+        // GEMM computes again in plain f32
+        if (lane == 0) scales_out[block * tok + t] = top >= (127u + 120u) << 23 ? __uint_as_float(0x7FC00000u) : up;
         if (q4) {
             // Q4 weights unpack as pairs (k, k + 4) of eight: order 0 4 1 5 2 6 3 7
             const bool odd = lane & 1u;
             const float r0 = __shfl_xor_sync(0xffffffffu, odd ? v[c][0] : v[c][2], 1), r1 = __shfl_xor_sync(0xffffffffu, odd ? v[c][1] : v[c][3], 1);
             if (odd) { v[c][0] = r0; v[c][1] = v[c][2]; v[c][2] = r1; }
             else     { v[c][3] = r1; v[c][2] = v[c][1]; v[c][1] = r0; }
-            // places 0-3 s.hi, 4-7 s.lo, 8-11 s.hi, 12-15 zero, beside the weights' b.hi, b.hi, b.lo, zero
-            if ((lane & 7u) == 0) {
-                const uint32_t b = lane >> 3;
-                const float s = sum[c] * down;
-                const __half hi = __float2half_rn(s), lo = __float2half_rn(s - __half2float(hi));
-                __half *first = reinterpret_cast<__half *>(side + tok * 4u + sums_at(t, 0)), *second = reinterpret_cast<__half *>(side + tok * 4u + sums_at(t, 1));
-                first[b] = hi; first[4 + b] = lo;
-                second[b] = hi; second[4 + b] = __float2half_rn(0.f);
-            }
         }
         store4(planes_out + block * 2 * planes * sub, sub, planes, t, lane * 4, v[c], down);
     }
@@ -258,11 +237,6 @@ __device__ __forceinline__ bool mbar_wait_lanes(unsigned long long *bar, uint32_
     atomicExch(&g_split_error, 1u);
     return false;
 }
-// K-major without a swizzle: halves of K 128 bytes apart, groups of 8 rows 256.
-__device__ __forceinline__ uint64_t plain_desc(uint32_t smem_addr)
-{
-    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (uint64_t)(128 >> 4) << 16 | (uint64_t)(256 >> 4) << 32 | (uint64_t)1 << 46;
-}
 // kind::f16 instruction descriptor: D f32, A and B f16, both K-major.
 __device__ __forceinline__ uint32_t split_instr(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((kCols >> 4) << 24); }
 
@@ -284,6 +258,29 @@ __device__ __forceinline__ void split_codes(uint32_t magic, __half2 offset, __ha
     const __half2 h = __hmul2_rn(c, d);                         // never contracted into the fma below
     hi = as_word(h);
     lo = as_word(__hfma2(c, d, __hneg2(h)));
+}
+
+// a - c and a * b + c of f16 values and an f32, rounded once.
+__device__ __forceinline__ float sub_mixed(__half a, float c)
+{
+    float d;
+    asm("sub.rn.f32.f16 %0, %1, %2;" : "=f"(d) : "h"(__half_as_ushort(a)), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float fma_mixed(__half a, __half b, float c)
+{
+    float d;
+    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(d) : "h"(__half_as_ushort(a)), "h"(__half_as_ushort(b)), "f"(c));
+    return d;
+}
+// Two codes as f16 1024 + c in one word -> parts of c * d + m: the first rounded to nearest, the second what is left of it.
+__device__ __forceinline__ void split_affine(uint32_t magic, __half2 d, __half2 m, float m32, uint32_t &hi, uint32_t &lo)
+{
+    const __half2 c = __hsub2(as_half2(magic), __float2half2_rn(1024.f));
+    const __half2 h = __hfma2(c, d, m);
+    hi = as_word(h);
+    lo = as_word(__floats2half2_rn(fma_mixed(__low2half(c), __low2half(d), -sub_mixed(__low2half(h), m32)),
+                                   fma_mixed(__high2half(c), __low2half(d), -sub_mixed(__high2half(h), m32))));
 }
 
 // The element (row, col) in plain f32, the way the tiled kernel sums it.
@@ -429,10 +426,9 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
     const uint32_t group = PLANES == 1 ? group_of(PLANES, p.k) : 1;
     uint8_t *ring = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sub = p.tok * 128u;                          // bytes of a token sub-tile, a multiple of 2048
-    const uint32_t side = side_bytes(FMT, p.tok);               // a multiple of 64
-    uint8_t *side_ring = ring + kSlots * sub;
-    uint8_t *raw = side_ring + kScaleSlots * side;
-    uint8_t *minima = raw + kRaw * kRawChunk;                   // Q4: two stages
+    const uint32_t scale_bytes = p.tok * 4u;                    // a multiple of 64
+    uint8_t *scale_ring = ring + kSlots * sub;
+    uint8_t *raw = scale_ring + kScaleSlots * scale_bytes;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t u_begin = unit_start(blockIdx.x, p.units, gridDim.x), u_end = unit_start(blockIdx.x + 1, p.units, gridDim.x);
 
@@ -461,13 +457,13 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         if (warp == 0) {
             // ------------------------------------------------------------------ token planes and scales
-            // lane x: the x-th sub-tile of every chunk; lane kParts: scales and sums.  One lane for all of them was late: a
+            // lane x: the x-th sub-tile of every chunk; lane kParts: scales.  One lane for all of them was late: a
             // wait, an arrival and a copy take it 300 cycles.
             if (lane <= kParts) {
                 pdl_wait();
                 const uint32_t depth = lane < kParts ? kDepth : kScaleSlots, count = u_end - u_begin;
-                const uint32_t bytes = lane < kParts ? sub : side, pitch = lane < kParts ? kParts * sub : side;
-                const uint8_t *base = lane < kParts ? p.planes + lane * sub : p.side;
+                const uint32_t bytes = lane < kParts ? sub : scale_bytes, pitch = lane < kParts ? kParts * sub : scale_bytes;
+                const uint8_t *base = lane < kParts ? p.planes + lane * sub : reinterpret_cast<const uint8_t *>(p.scales);
                 // [m tile][chunk]: the tiles of a column strip follow one another
                 uint32_t at = u_begin / p.chunks % p.m_tiles * p.chunks + u_begin % p.chunks, armed = 0;
                 const uint32_t wrap = p.m_tiles * p.chunks;
@@ -476,7 +472,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                     unsigned long long *full = lane < kParts ? &sh.slot_full[slot] : &sh.sc_full[s], *empty = lane < kParts ? &sh.slot_empty[s] : &sh.sc_empty[s];
                     if (!mbar_wait(empty, ((i / depth) & 1u) ^ 1u, &sh.failed, &g_split_error)) continue;
                     mbar_arrive_expect_tx(full, bytes);
-                    bulk_load(lane < kParts ? ring + slot * sub : side_ring + s * side, base + (size_t)at * pitch, bytes, full);
+                    bulk_load(lane < kParts ? ring + slot * sub : scale_ring + s * scale_bytes, base + (size_t)at * pitch, bytes, full);
                     armed = i + 1;
                 }
                 if (sh.failed)                                  // let this lane's own copies land before the CTA exits
@@ -501,18 +497,16 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                 const uint32_t stage = i & 1u, ph = (i >> 1) & 1u, s = i % kDepth, b = filled & 1u;
                 const bool close = group == 1 || chunk % group == group - 1 || chunk + 1 == p.chunks || i + 1 == count;
                 const uint32_t d = tm + b * kMaxTok, w_hi = tm + 2 * kMaxTok + stage * 128u, w_lo = w_hi + 64u;
-                // lane 0: accumulator, 1: weights, 2: sums (Q4), 4..: the chunk's sub-tiles
-                unsigned long long *bar = lane == 0 ? &sh.d_empty[b] : lane == 1 ? &sh.w_full[stage] : lane == 2 ? &sh.sc_full[i % kScaleSlots] : &sh.slot_full[(s * kParts + lane - 4u) % kSlots];
-                const uint32_t parity = lane == 0 ? ((filled >> 1) & 1u) ^ 1u : lane == 1 ? ph : lane == 2 ? (i / kScaleSlots) & 1u : (i / kDepth) & 1u;
-                ok = mbar_wait_lanes(bar, parity, lane < 2 || (FMT == MGQ_FMT_Q4 && lane == 2) || (lane >= 4 && lane < 4 + kParts), &sh.failed);
+                // lane 0: accumulator, 1: weights, 4..: the chunk's sub-tiles
+                unsigned long long *bar = lane == 0 ? &sh.d_empty[b] : lane == 1 ? &sh.w_full[stage] : &sh.slot_full[(s * kParts + lane - 4u) % kSlots];
+                const uint32_t parity = lane == 0 ? ((filled >> 1) & 1u) ^ 1u : lane == 1 ? ph : (i / kDepth) & 1u;
+                ok = mbar_wait_lanes(bar, parity, lane < 2 || (lane >= 4 && lane < 4 + kParts), &sh.failed);
                 if (!ok) break;
                 tc_fence_after();
                 if (leader) {
                     const uint32_t x_lo = ring16 + s * kParts * sub16, x_hi = x_lo + (kParts - 2) * sub16;
-                    if (FMT == MGQ_FMT_Q4)
-                        umma_f16(d, plain_desc(smem_u32(minima + stage * kMinBytes)), plain_desc(smem_u32(side_ring + (i % kScaleSlots) * side + p.tok * 4u)), instr, open ? 1u : 0u);
-                    if (FMT == MGQ_FMT_Q4 || open) umma_f16_ts<true>(d, w_lo, x_hi, instr);
-                    else                           umma_f16_ts<false>(d, w_lo, x_hi, instr);
+                    if (open) umma_f16_ts<true>(d, w_lo, x_hi, instr);
+                    else      umma_f16_ts<false>(d, w_lo, x_hi, instr);
 #pragma unroll
                     for (uint32_t j = 1; j < 8; j++) umma_f16_ts<true>(d, w_lo + j * 8u, x_hi + (j / 4) * sub16 + (j % 4) * 2u, instr);
                     if (PLANES == 2)
@@ -561,7 +555,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                 __syncwarp();                                   // tcgen05.ld is warp-collective
                 tc_fence_after();
                 const uint32_t from = tmem + lane_addr + b * kMaxTok + first;
-                const uint8_t *scale = side_ring + sc * side + first * 4u;
+                const uint8_t *scale = scale_ring + sc * scale_bytes + first * 4u;
                 if (mine > 1) drain_part<0, 2>(from, scale, acc);
                 else if (mine > 0) drain_part<0, 1>(from, scale, acc);
                 if (mine > 3) drain_part<2, 2>(from, scale, acc);
@@ -683,31 +677,21 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
             if (FMT == MGQ_FMT_Q4) {
                 const uint4 head = *reinterpret_cast<const uint4 *>(src);
                 const uint32_t h[4] = {head.x, head.y, head.z, head.w};
-                const __half2 offset = __float2half2_rn(1032.f);
-                float b[4];
 #pragma unroll
                 for (int blk = 0; blk < 4; blk++) {
                     uint32_t hi[16], lo[16];
-                    const float2 dm = __half22float2(as_half2(h[blk]));
-                    b[blk] = fmaf(8.f, dm.x, dm.y);
-                    const __half2 d = __half2half2(__low2half(as_half2(h[blk])));
+                    const __half2 d = __half2half2(__low2half(as_half2(h[blk]))), m = __half2half2(__high2half(as_half2(h[blk])));
+                    const float m32 = __high2float(as_half2(h[blk]));
                     const uint4 q4 = *reinterpret_cast<const uint4 *>(src + 16u + blk * 16u);
                     const uint32_t q[4] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
                     for (int e = 0; e < 4; e++)
 #pragma unroll
                         for (int s = 0; s < 4; s++)             // codes s and s + 4 of eight
-                            split_codes(((q[e] >> (4 * s)) & 0x000F000Fu) | 0x64006400u, offset, d, hi[e * 4 + s], lo[e * 4 + s]);
+                            split_affine(((q[e] >> (4 * s)) & 0x000F000Fu) | 0x64006400u, d, m, m32, hi[e * 4 + s], lo[e * 4 + s]);
                     tmem_st16(dst + blk * 16u, hi);
                     tmem_st16(dst + 64u + blk * 16u, lo);
                 }
-                const __half2 h01 = __floats2half2_rn(b[0], b[1]), h23 = __floats2half2_rn(b[2], b[3]);
-                const __half2 l01 = __floats2half2_rn(b[0] - __low2float(h01), b[1] - __high2float(h01));
-                const __half2 l23 = __floats2half2_rn(b[2] - __low2float(h23), b[3] - __high2float(h23));
-                uint8_t *mins = minima + group * kMinBytes;
-                *reinterpret_cast<uint4 *>(mins + sums_at(quad * 32 + lane, 0)) = make_uint4(as_word(h01), as_word(h23), as_word(h01), as_word(h23));
-                *reinterpret_cast<uint4 *>(mins + sums_at(quad * 32 + lane, 1)) = make_uint4(as_word(l01), as_word(l23), 0u, 0u);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             } else {
                 uint32_t words[36];                             // four blocks of 9
 #pragma unroll
@@ -779,8 +763,7 @@ cudaMemPool_t workspace_pool(int dev)
 template <int FMT, int PLANES>
 int launch_split(const SplitParams &p, uint32_t ctas, cudaStream_t stream)
 {
-    const size_t smem = 1024 + (size_t)kSlots * p.tok * 128 + (size_t)kScaleSlots * side_bytes(FMT, p.tok) + (size_t)kRaw * kCols * raw_bytes(FMT) +
-                        (FMT == MGQ_FMT_Q4 ? 2 * kMinBytes : 0);
+    const size_t smem = 1024 + (size_t)kSlots * p.tok * 128 + (size_t)kScaleSlots * p.tok * 4 + (size_t)kRaw * kCols * raw_bytes(FMT);
     if (int rc = allow_smem(gemm_split_kernel<FMT, PLANES>, smem)) return rc;
     return launch(gemm_split_kernel<FMT, PLANES>, dim3(ctas), dim3(kSplitThreads), smem, stream, p);
 }
@@ -826,21 +809,21 @@ int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const 
         const uint32_t ctas = p.units / 2 < 1 ? 1 : p.units / 2 < (uint32_t)sms ? p.units / 2 : (uint32_t)sms;
 
         const size_t plane_bytes = (size_t)p.m_tiles * p.chunks * 2 * planes * p.tok * 128;
-        const size_t all_side = ((size_t)p.m_tiles * p.chunks * side_bytes(fmt, p.tok) + 255) / 256 * 256;
+        const size_t scale_bytes = ((size_t)p.m_tiles * p.chunks * p.tok * 4 + 255) / 256 * 256;
         const size_t part_bytes = (size_t)ctas * 2 * kMaxTok * kCols * 4;
         uint8_t *ws = nullptr;
-        if (cudaMallocFromPoolAsync(reinterpret_cast<void **>(&ws), plane_bytes + all_side + part_bytes + (size_t)p.tiles * 4, pool, stream) != cudaSuccess) {
+        if (cudaMallocFromPoolAsync(reinterpret_cast<void **>(&ws), plane_bytes + scale_bytes + part_bytes + (size_t)p.tiles * 4, pool, stream) != cudaSuccess) {
             cudaGetLastError();
             return MGQ_OK;
         }
-        uint8_t *side_dev = ws + plane_bytes;
+        float *scales = reinterpret_cast<float *>(ws + plane_bytes);
         p.planes = ws;
-        p.side = side_dev;
-        p.partial = reinterpret_cast<float *>(side_dev + all_side);
-        p.counters = reinterpret_cast<unsigned int *>(side_dev + all_side + part_bytes);
+        p.scales = scales;
+        p.partial = reinterpret_cast<float *>(ws + plane_bytes + scale_bytes);
+        p.counters = reinterpret_cast<unsigned int *>(ws + plane_bytes + scale_bytes + part_bytes);
         const bool vec = reinterpret_cast<uintptr_t>(p.a) % 16 == 0;
         const unsigned long long warps = (unsigned long long)p.m * ((p.chunks + group_of(planes, k) - 1) / group_of(planes, k));
-        split_rows_kernel<<<(uint32_t)((warps + 7) / 8), 256, 0, stream>>>(p.a, bf16, vec, ws, side_dev, p.counters, p.tiles, p.m, k, p.tok, p.chunks, planes, q4);
+        split_rows_kernel<<<(uint32_t)((warps + 7) / 8), 256, 0, stream>>>(p.a, bf16, vec, ws, scales, p.counters, p.tiles, p.m, k, p.tok, p.chunks, planes, q4);
         int rc = cuda_check((int)cudaGetLastError(), "split_rows_kernel", __FILE__, __LINE__);
         if (rc == MGQ_OK)
             rc = q4 ? (bf16 ? launch_split<MGQ_FMT_Q4, 1>(p, ctas, stream) : launch_split<MGQ_FMT_Q4, 2>(p, ctas, stream))

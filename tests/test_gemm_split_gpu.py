@@ -137,3 +137,67 @@ def test_captured_in_a_graph():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, ops.matmul(fmt, xd, wd, k, n, route="gemm"))
+
+
+def _bound(act, k):
+    """Truncating steps per accumulator (two or three products of eight, two chunks of bf16 from K = 2048 on), see above."""
+    return (24 if act == "f32" else 32 if k >= 2048 else 16) * 2 / 3 * 2.0 ** -24 + 1e-8
+
+
+def _q4_weights(kind, k, n, seed, zero_at=()):
+    """Minima that have nothing to do with -8 d; rows of W in `zero_at` dequantize to exactly 0 (not for kind "quantized")."""
+    rng = np.random.Generator(np.random.PCG64(seed))
+    if kind == "quantized":
+        from meganeura_b200 import ops
+        return ops.quantize(O.FMT_Q4, rng.standard_normal((k, n)).astype(np.float32) * 0.02)
+    # d of 7 bits, so that its multiples up to 15 are exact in f16
+    d = np.exp(rng.uniform(np.log(1e-3), np.log(1e-1), size=(n, k // 32))).astype(np.float32)
+    d = (d.view(np.uint32) >> 17 << 17).view(np.float32)
+    zero = {"seven": 7, "plus": 0, "above": 15}[kind]
+    codes = rng.integers(0, 16, size=(k, n), dtype=np.uint8)
+    m = -zero * d if zero else d * rng.integers(-20, 21, size=d.shape).astype(np.float32)
+    codes[list(zero_at)] = zero
+    return O.pack_q4_np(codes, d.astype(np.float16).view(np.uint16), m.astype(np.float16).view(np.uint16))
+
+
+@pytest.mark.parametrize("act", ["f32", "bf16"])
+@pytest.mark.parametrize("kind", ["seven", "plus", "above", "quantized"])
+@pytest.mark.parametrize("m,k,n", [(20, 160, 70), (33, 288, 129), (40, 2176, 70), (17, 4128, 200), (130, 2048, 33)])
+def test_q4_minima(kind, act, m, k, n):
+    import torch
+    w, x = _q4_weights(kind, k, n, m + k), _inputs(O.FMT_Q4, m, k, n)[1]
+    xd = to_dev(x)
+    if act == "bf16":
+        xd = xd.to(torch.bfloat16)
+        x = xd.float().cpu().numpy()
+    got = run_matmul(O.FMT_Q4, xd, w, k, n, route="gemm")
+    assert O.rel_l2(got, x.astype(np.float64) @ _dense(O.FMT_Q4, w, k, n)) <= _bound(act, k)
+
+
+@pytest.mark.parametrize("act", ["f32", "bf16"])
+@pytest.mark.parametrize("kind", ["seven", "above", "q8"])
+@pytest.mark.parametrize("size", [1e3, 1e5])
+def test_large_activation_at_a_weight_of_zero(kind, act, size):
+    """It adds nothing to a sum, so it may not add an error either: in every row, relative to the row's own result."""
+    import torch
+    m, k, n = 24, 2176, 150
+    at = range(5, k, 128)
+    fmt = O.FMT_Q8 if kind == "q8" else O.FMT_Q4
+    w, x = _inputs(fmt, m, k, n)
+    if kind == "q8":
+        w = w.copy()
+        blocks = w.reshape(n, k // 32, 36)
+        for kk in at:
+            blocks[:, kk // 32, 4 + kk % 32] = 0
+    else:
+        w = _q4_weights(kind, k, n, 9, at)
+    assert (_dense(fmt, w, k, n)[list(at)] == 0).all()
+    x[:, list(at)] = size * np.where(np.arange(m) % 2, 1, -1)[:, None]
+    xd = to_dev(x)
+    if act == "bf16":
+        xd = xd.to(torch.bfloat16)
+        x = xd.float().cpu().numpy()
+    got = run_matmul(fmt, xd, w, k, n, route="gemm")
+    want = x.astype(np.float64) @ _dense(fmt, w, k, n)
+    for r in range(m):
+        assert O.rel_l2(got[r], want[r]) <= _bound(act, k)
