@@ -31,8 +31,9 @@
 //   warps 12-19   weights: two groups of four, chunks in turn; cp.async of a warp's 32 columns two chunks
 //                 of its own ahead, conversion, tcgen05.st.
 // TMEM: two accumulators of 128 columns, two weight stages of 64 (hi) + 64 (lo) columns.
-// Sums that are not finite (non-finite inputs, a weight beyond the f16 range) are computed again
-// element by element on the CUDA cores.
+// Sums that are not finite (non-finite inputs, a weight beyond the f16 range) are noted in the workspace and computed again
+// element by element on the CUDA cores once the CTA's pipeline has ended, so that no bounded wait depends on how many they are;
+// a row with a NaN is known after one look at it.
 //
 // What bounds it: of the 2650 cycles that a chunk of 128 x 128 takes with f32 activations the tensor core needs 1536 (2100 and 1024
 // for bf16), the rest is the hand-over of a weight stage: products of chunk i - 2 done, conversion (1500 cycles, four warps),
@@ -78,6 +79,8 @@ struct SplitParams {
     const float *scales;            // [m tile][chunk][tokens]
     float *partial;                 // [CTA][2][128 tokens][128 columns]
     unsigned int *counters;         // one per tile
+    unsigned int *odd_by;           // [tile][drain warp]: 1 + the CTA whose warp has left masks, or 0
+    unsigned long long *odd;        // [tile][drain thread]: its tokens whose sums are not finite
     unsigned long long num_blocks;
     uint32_t m, k, n, bpc;
     uint32_t tok, m_tiles, tiles;   // tokens of a tile, tiles
@@ -142,12 +145,12 @@ __device__ __forceinline__ void store4(uint8_t *block, uint32_t sub, uint32_t pl
 
 // A warp per row and group of chunks.  Bound by the read of the activations (8 MB for 512 x 4096 f32) and as many bytes written,
 // all of which stay in L2 for the GEMM behind it.
-__global__ void __launch_bounds__(256) split_rows_kernel(const void *a, bool bf16, bool vec, uint8_t *planes_out, float *scales_out, unsigned int *counters, uint32_t tiles,
+__global__ void __launch_bounds__(256) split_rows_kernel(const void *a, bool bf16, bool vec, uint8_t *planes_out, float *scales_out, unsigned int *counters, uint32_t words,
                                                          uint32_t m, uint32_t k, uint32_t tok, uint32_t chunks, uint32_t planes, bool q4)
 {
     pdl_launch_dependents();
     const uint32_t lane = threadIdx.x & 31u, gid = blockIdx.x * 8 + (threadIdx.x >> 5);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < tiles; i += gridDim.x * blockDim.x) counters[i] = 0;      // the GEMM's tile counters
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x) counters[i] = 0;      // the GEMM's counters and marks
     const uint32_t span = group_of(planes, k), groups = (chunks + span - 1) / span;
     const uint32_t row = gid / groups, first_chunk = gid % groups * span;
     if (row >= m) return;
@@ -308,6 +311,36 @@ __device__ __noinline__ float plain_element(const SplitParams &p, bool bf16, uin
         }
     }
     return acc;
+}
+
+// The sums that a drain warp has noted, tile by tile: a thread its own column, the rows one after another.
+template <int FMT>
+__device__ __noinline__ void redo_odd(const SplitParams &p, bool bf16, uint32_t u_begin, uint32_t u_end, uint32_t warp, uint32_t lane)
+{
+    for (uint32_t tile = u_begin / p.chunks; tile <= (u_end - 1) / p.chunks; tile++) {
+        uint32_t by = lane == 0 ? p.odd_by[tile * 8 + warp] : 0u;
+        if (__shfl_sync(0xffffffffu, by, 0) != blockIdx.x + 1) continue;
+        const unsigned long long odd = p.odd[((size_t)tile * 8 + warp) * 32 + lane];
+        const uint32_t groups = p.tok / 16, m0 = (tile % p.m_tiles) * p.tok + (warp >= 4 ? (groups + 1) / 2 * 16 : 0);
+        const uint32_t col = (tile / p.m_tiles) * kCols + (warp & 3u) * 32 + lane;
+        for (uint32_t r = 0; r < 64; r++) {
+            const bool mine = odd >> r & 1u;
+            if (!__any_sync(0xffffffffu, mine)) continue;
+            const uint32_t row = m0 + r;
+            bool nan = false;                                   // NaN times any weight is NaN, and so is the sum
+            for (uint32_t k0 = 0; k0 < p.k && !nan; k0 += 256) {
+                bool found = false;
+#pragma unroll
+                for (uint32_t x = 0; x < 256; x += 32)
+                    if (k0 + x < p.k) found |= isnan(load_act(p.a, (size_t)row * p.k + k0 + x + lane, bf16));
+                nan = __any_sync(0xffffffffu, found);
+            }
+            if (!mine) continue;
+            const float v = nan ? __uint_as_float(0x7FC00000u) : plain_element<FMT>(p, bf16, row, col);
+            const size_t o = (size_t)row * p.n + col;
+            p.c[o] = p.addend ? v + p.addend[o] : v;
+        }
+    }
 }
 
 // Asynchronous copy of the packed bytes that a warp's 32 columns (from col0) hold of a chunk; neighbouring lanes copy
@@ -539,6 +572,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
         const uint32_t j = quad * 32 + lane;                    // weight column within the tile
         float acc[4][16];                                       // tokens first + 16 g + e
         uint32_t i = 0, filled = 0;                             // chunks, accumulators so far
+        bool redo = false;
         for (uint32_t u = u_begin; u < u_end;) {
             const uint32_t tile = u / p.chunks, c0 = u % p.chunks;
             const uint32_t c1 = min(p.chunks, c0 + (u_end - u));
@@ -637,15 +671,14 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                         if (g * 16 + e < (int)rows && !(odd >> (g * 16 + e) & 1u)) p.c[o0 + (size_t)(g * 16 + e) * p.n] = acc[g][e];
                 }
                 if (rows < 64) odd &= (1ull << rows) - 1;
-                while (odd) {
-                    const uint32_t row = m0 + __ffsll((long long)odd) - 1;
-                    odd &= odd - 1;
-                    const float v = plain_element<FMT>(p, PLANES == 1, row, col);
-                    const size_t o = (size_t)row * p.n + col;
-                    p.c[o] = p.addend ? v + p.addend[o] : v;
+                if (__any_sync(0xffffffffu, odd != 0)) {
+                    p.odd[((size_t)tile * 8 + warp - 4) * 32 + lane] = odd;
+                    if (lane == 0) p.odd_by[tile * 8 + warp - 4] = blockIdx.x + 1;
+                    redo = true;
                 }
             }
         }
+        if (redo) redo_odd<FMT>(p, PLANES == 1, u_begin, u_end, warp - 4, lane);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
         // ---------------------------------------------------------------------- weights
@@ -810,9 +843,9 @@ int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const 
 
         const size_t plane_bytes = (size_t)p.m_tiles * p.chunks * 2 * planes * p.tok * 128;
         const size_t scale_bytes = ((size_t)p.m_tiles * p.chunks * p.tok * 4 + 255) / 256 * 256;
-        const size_t part_bytes = (size_t)ctas * 2 * kMaxTok * kCols * 4;
+        const size_t part_bytes = (size_t)ctas * 2 * kMaxTok * kCols * 4, odd_bytes = (size_t)p.tiles * 256 * 8, words = (size_t)p.tiles * 9;
         uint8_t *ws = nullptr;
-        if (cudaMallocFromPoolAsync(reinterpret_cast<void **>(&ws), plane_bytes + scale_bytes + part_bytes + (size_t)p.tiles * 4, pool, stream) != cudaSuccess) {
+        if (cudaMallocFromPoolAsync(reinterpret_cast<void **>(&ws), plane_bytes + scale_bytes + part_bytes + odd_bytes + words * 4, pool, stream) != cudaSuccess) {
             cudaGetLastError();
             return MGQ_OK;
         }
@@ -820,10 +853,12 @@ int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const 
         p.planes = ws;
         p.scales = scales;
         p.partial = reinterpret_cast<float *>(ws + plane_bytes + scale_bytes);
-        p.counters = reinterpret_cast<unsigned int *>(ws + plane_bytes + scale_bytes + part_bytes);
+        p.odd = reinterpret_cast<unsigned long long *>(ws + plane_bytes + scale_bytes + part_bytes);
+        p.counters = reinterpret_cast<unsigned int *>(ws + plane_bytes + scale_bytes + part_bytes + odd_bytes);
+        p.odd_by = p.counters + p.tiles;
         const bool vec = reinterpret_cast<uintptr_t>(p.a) % 16 == 0;
         const unsigned long long warps = (unsigned long long)p.m * ((p.chunks + group_of(planes, k) - 1) / group_of(planes, k));
-        split_rows_kernel<<<(uint32_t)((warps + 7) / 8), 256, 0, stream>>>(p.a, bf16, vec, ws, scales, p.counters, p.tiles, p.m, k, p.tok, p.chunks, planes, q4);
+        split_rows_kernel<<<(uint32_t)((warps + 7) / 8), 256, 0, stream>>>(p.a, bf16, vec, ws, scales, p.counters, (uint32_t)words, p.m, k, p.tok, p.chunks, planes, q4);
         int rc = cuda_check((int)cudaGetLastError(), "split_rows_kernel", __FILE__, __LINE__);
         if (rc == MGQ_OK)
             rc = q4 ? (bf16 ? launch_split<MGQ_FMT_Q4, 1>(p, ctas, stream) : launch_split<MGQ_FMT_Q4, 2>(p, ctas, stream))

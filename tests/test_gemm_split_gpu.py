@@ -201,3 +201,40 @@ def test_large_activation_at_a_weight_of_zero(kind, act, size):
     want = x.astype(np.float64) @ _dense(fmt, w, k, n)
     for r in range(m):
         assert O.rel_l2(got[r], want[r]) <= _bound(act, k)
+
+
+@pytest.mark.parametrize("act", ["f32", "bf16"])
+@pytest.mark.parametrize("fmt", FMTS)
+def test_nothing_but_nan_and_infinities(fmt, act):
+    """Every sum of a long K takes the way of those that are not finite; no bounded wait may run out meanwhile."""
+    import torch
+    from meganeura_b200 import ops
+    m, k, n = 48, 4096, 300
+    w, x = _inputs(fmt, m, k, n)
+    x[:] = np.nan
+    x[40:44] = np.inf                                         # signs of the weights decide: NaN wherever both come up
+    x[44] = 1.0
+    x[44, k - 1] = np.nan                                     # the last element
+    x[45:] = 0.5                                              # ordinary rows beside them
+    d = np.ones((m, n), dtype=np.float32)
+    xd = to_dev(x).to(torch.bfloat16) if act == "bf16" else to_dev(x)
+    got = run_matmul(fmt, xd, w, k, n, addend=d, route="gemm")
+    ops.device_status()
+    assert np.isnan(got[:45]).all()
+    assert O.rel_l2(got[45:], x[45:].astype(np.float64) @ _dense(fmt, w, k, n) + 1.0) <= _bound(act, k)
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+def test_infinities_in_place(fmt):
+    """The addend is the output: sums that are computed again read it before it is overwritten."""
+    import torch
+    from meganeura_b200 import ops
+    m, k, n = 150, 288, 260
+    w, x = _inputs(fmt, m, k, n)
+    x[7, 3] = x[140, 200] = np.inf
+    xd, wd = to_dev(x), to_dev(w)
+    out = torch.full((m, n), 2.0, device="cuda")
+    want = ops.matmul(fmt, xd, wd, k, n, addend=out.clone(), route="gemm")
+    ops.matmul(fmt, xd, wd, k, n, addend=out, out=out, route="gemm")
+    torch.cuda.synchronize()
+    assert torch.equal(torch.nan_to_num(out, nan=7.0), torch.nan_to_num(want, nan=7.0)) and bool(torch.isinf(out[[7, 140]]).any())
