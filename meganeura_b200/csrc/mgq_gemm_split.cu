@@ -6,8 +6,10 @@
 // dequant_q4 / dequant_q8 as the B-tile load).
 //
 // Operands are sums of f16 values, whose products the tensor cores form exactly:
-//   activations  x = (hi + lo) * 2^e, e per row and 128 k (split_rows_kernel): all 24 bits of an f32 but the last
-//                one or two; a bf16 value fits hi alone, so that case has one plane and two products instead of three.
+//   activations  x = (hi + lo * 2^-12) * 2^e, e per row and 128 k (split_rows_kernel): 22 bits of an f32 at least, down to
+//                2^-29 of the row's largest value in these 128 k (the products with lo come first and the accumulator is scaled
+//                by 2^-12 before the others are added); a bf16 value fits hi alone down to 2^-31, so that case has one plane and
+//                two products instead of three.  Rows with more than 16 values below 2^-29 (bf16: 2^-27) are summed in plain f32.
 //   weights      Q8: code * d has at most 19 bits, hi = rn16(code * d), lo = fma16(code, d, -hi), both exact, two
 //                instructions for two weights.  Q4: hi = fma16(code, d, m), lo = rn16(code * d + m - hi), the difference
 //                in f32: 2^-23 of the weight at most is left.  Both are multiples of 2^-24 as d and m are, so nothing is
@@ -126,6 +128,8 @@ __device__ __forceinline__ void pick_scale(float top, float &down, float &up)
     up = __uint_as_float((uint32_t)(127 - s) << 23);
 }
 
+constexpr uint32_t kLowShift = 12;                 // the low plane is stored 2^12 times as large: |lo| <= 2^3, beside |hi| <= 2^15
+
 // Four consecutive places of one row: f16 parts of v * down into the planes' swizzled sub-tiles.  pos: place within the chunk.
 __device__ __forceinline__ void store4(uint8_t *block, uint32_t sub, uint32_t planes, uint32_t t, uint32_t pos, const float (&v)[4], float down)
 {
@@ -134,7 +138,7 @@ __device__ __forceinline__ void store4(uint8_t *block, uint32_t sub, uint32_t pl
     for (int i = 0; i < 4; i++) {
         const float s = v[i] * down;
         hi[i] = __float2half_rn(s);
-        lo[i] = __float2half_rn(s - __half2float(hi[i]));
+        lo[i] = __float2half_rn((s - __half2float(hi[i])) * (float)(1u << kLowShift));
     }
     const uint32_t half = pos >> 6, byte = (pos & 63u) * 2u;
     uint8_t *h = block + (size_t)((planes == 2 ? 2u : 0u) + half) * sub + t * 128u, *l = block + (size_t)half * sub + t * 128u;      // lo, lo, hi, hi
@@ -182,13 +186,22 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const void *a, bool bf1
     top = __reduce_max_sync(0xffffffffu, top);
     float down, up;
     pick_scale(__uint_as_float(top), down, up);
+    // below it f16 parts of that scale hold less than 22 bits of a value; a lone part holds 8 down to 2^-31, but 256 k with
+    // one value of 10^8 at weights of 0 were 1.1e-5 off (with bf16 operands in their own range 7.5e-6)
+    const float least = __uint_as_float(top) * (planes == 2 ? 0x1p-29f : 0x1p-27f);
+    uint32_t small = 0;
+#pragma unroll
+    for (uint32_t c = 0; c < 2; c++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) small += fabsf(v[c][i]) < least && v[c][i] != 0.f ? 1u : 0u;
+    const bool wide = __reduce_add_sync(0xffffffffu, small) > kChunk / 8;
 #pragma unroll
     for (uint32_t c = 0; c < 2; c++) {
         if (c >= span || first_chunk + c >= chunks) break;      // uniform over the warp
         const size_t block = (size_t)mt * chunks + first_chunk + c;
-        // not finite, or so large (from 2^120 on) that f32 sums overflow on their way: a NaN scale makes the row's sums NaN, which the
+        // too many small values, not finite, or so large (from 2^120 on) that f32 sums overflow on their way: a NaN scale makes the row's sums NaN, which the
         // GEMM computes again in plain f32
-        if (lane == 0) scales_out[block * tok + t] = top >= (127u + 120u) << 23 ? __uint_as_float(0x7FC00000u) : up;
+        if (lane == 0) scales_out[block * tok + t] = wide || top >= (127u + 120u) << 23 ? __uint_as_float(0x7FC00000u) : up;
         if (q4) {
             // Q4 weights unpack as pairs (k, k + 4) of eight: order 0 4 1 5 2 6 3 7
             const bool odd = lane & 1u;
@@ -226,6 +239,15 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint32_t b16
                  "mov.b64 db, {%2, %4};\n\t"
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
                  ::"r"(d), "r"(a), "r"(b16 | 0x10000u), "r"(instr), "r"(kDescHigh), "n"(ACC ? 1 : 0) : "memory");
+}
+// D = A . B + D * 2^-kLowShift
+__device__ __forceinline__ void umma_f16_ts_scaled(uint32_t d, uint32_t a, uint32_t b16, uint32_t instr)
+{
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+                 "setp.ne.b32 p, 1, 0;\n\t"
+                 "mov.b64 db, {%2, %4};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p, %5;\n\t}"
+                 ::"r"(d), "r"(a), "r"(b16 | 0x10000u), "r"(instr), "r"(kDescHigh), "n"(kLowShift) : "memory");
 }
 // A converged warp waits for several barriers at once, a lane (with `mine` set) for each: the try_waits share one latency.
 __device__ __forceinline__ bool mbar_wait_lanes(unsigned long long *bar, uint32_t parity, bool mine, volatile int *failed)
@@ -538,13 +560,15 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                 tc_fence_after();
                 if (leader) {
                     const uint32_t x_lo = ring16 + s * kParts * sub16, x_hi = x_lo + (kParts - 2) * sub16;
-                    if (open) umma_f16_ts<true>(d, w_lo, x_hi, instr);
-                    else      umma_f16_ts<false>(d, w_lo, x_hi, instr);
+                    if (PLANES == 2) {                          // never two chunks per accumulator
+                        umma_f16_ts<false>(d, w_hi, x_lo, instr);
+#pragma unroll
+                        for (uint32_t j = 1; j < 8; j++) umma_f16_ts<true>(d, w_hi + j * 8u, x_lo + (j / 4) * sub16 + (j % 4) * 2u, instr);
+                        umma_f16_ts_scaled(d, w_lo, x_hi, instr);
+                    } else if (open) umma_f16_ts<true>(d, w_lo, x_hi, instr);
+                    else             umma_f16_ts<false>(d, w_lo, x_hi, instr);
 #pragma unroll
                     for (uint32_t j = 1; j < 8; j++) umma_f16_ts<true>(d, w_lo + j * 8u, x_hi + (j / 4) * sub16 + (j % 4) * 2u, instr);
-                    if (PLANES == 2)
-#pragma unroll
-                        for (uint32_t j = 0; j < 8; j++) umma_f16_ts<true>(d, w_hi + j * 8u, x_lo + (j / 4) * sub16 + (j % 4) * 2u, instr);
 #pragma unroll
                     for (uint32_t j = 0; j < 8; j++) umma_f16_ts<true>(d, w_hi + j * 8u, x_hi + (j / 4) * sub16 + (j % 4) * 2u, instr);
                     umma_commit(&sh.w_empty[stage]);

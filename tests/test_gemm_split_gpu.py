@@ -238,3 +238,39 @@ def test_infinities_in_place(fmt):
     ops.matmul(fmt, xd, wd, k, n, addend=out, out=out, route="gemm")
     torch.cuda.synchronize()
     assert torch.equal(torch.nan_to_num(out, nan=7.0), torch.nan_to_num(want, nan=7.0)) and bool(torch.isinf(out[[7, 140]]).any())
+
+
+@pytest.mark.parametrize("act", ["f32", "bf16"])
+@pytest.mark.parametrize("fmt", FMTS)
+# one value per 128 k so much larger than the others; 2^29 (bf16: 2^27) is where plain f32 sums take over
+@pytest.mark.parametrize("size", [2.0 ** 20, 2.0 ** 26, 2.0 ** 28, 2.0 ** 33, 2.0 ** 60, 2.0 ** 100])
+def test_span_of_magnitudes(fmt, act, size):
+    """A large activation at weights of zero leaves the small ones their bits.
+
+    Down to 2^-29 of the largest value an f32 keeps 22 bits, 2^-23 of its value at most; that adds in quadrature to the sums.
+    Plain f32 sums in order of k are sqrt(k / 3) * 2^-24 off."""
+    import torch
+    m, k, n = 24, 2176, 150
+    at = list(range(70, k, 128))
+    if fmt == O.FMT_Q4:
+        w = _q4_weights("seven", k, n, 4, at)
+    else:
+        w = _inputs(fmt, m, k, n)[0].copy()
+        for kk in at:
+            w.reshape(n, k // 32, 36)[:, kk // 32, 4 + kk % 32] = 0
+    x = _inputs(fmt, m, k, n)[1]
+    x = np.sign(x) * np.maximum(np.abs(x), 0.5).astype(np.float32)
+    x[:, at] = size
+    x[1::2, at] = -size
+    x[5] = 0                                                  # nothing but the large ones
+    x[5, at] = size
+    xd = to_dev(x)
+    if act == "bf16":
+        xd = xd.to(torch.bfloat16)
+        x = xd.float().cpu().numpy()
+    got = run_matmul(fmt, xd, w, k, n, route="gemm")
+    want = x.astype(np.float64) @ _dense(fmt, w, k, n)
+    assert (got[5] == 0).all()
+    bound = max(_bound(act, k), 2 * (k / 3) ** 0.5 * 2.0 ** -24)
+    for r in range(m):
+        assert r == 5 or O.rel_l2(got[r], want[r]) <= bound
