@@ -246,8 +246,11 @@ size_t mgq_argmax_workspace(void);
 int mgq_argmax(const float *logits, uint32_t n, void *workspace, uint32_t *out_token, uint32_t *next_token, uint32_t *kv_pos,
                uint32_t *history, uint32_t history_cap, void *stream);
 
-/* Routing wrapper: mgq_gemv when m <= MGQ_GEMV_MAX_M (f32 activations) and no pass over the weights beyond the second
- * would be needed, else mgq_gemm. */
+/* Routing wrapper.  f32 activations with m <= MGQ_GEMV_MAX_M go to mgq_gemv, unless that would need more passes over the
+ * weights than mgq_gemm takes time: from 5 rows on (8 or 12 for few columns) where k % 256 != 0, from 9 rows on for large
+ * Q8 weights, and where no streaming kernel takes the shape (k < 256, k > 32768, Q8 with k / 32 odd and above 256, packed
+ * sizes that are no multiple of 16 bytes) from a few thousand m * k on, single rows among them.  Everything else goes to
+ * mgq_gemm.  A column's bits do not depend on n while the call stays with mgq_gemv. */
 int mgq_matmul(int fmt, const void *a, int a_dtype, const void *w, const float *addend, float *c,
                uint32_t m, uint32_t k, uint32_t n, void *stream);
 

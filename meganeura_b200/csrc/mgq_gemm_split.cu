@@ -21,6 +21,10 @@
 // K = 512, where f32 sums in order of k are 1.1e-6 and 3.9e-7 off.  With bf16 activations and K from 2048 on two chunks share an
 // accumulator and a scale: 5e-7, and half the drains (149 -> 143 us for 512 x 4096 x 14336 in a long run).
 //
+// Up to 16 f32 rows on Q8 weights that no streaming GEMV takes would otherwise be summed in short f32 trees, 1.2e-7 off.  For them an
+// accumulator takes 32 k and its sums are added with what they round away: 1.0e-7 (2.0e-7 with 128 k).  16 x 12320 x 4099: 72 us
+// (45 with 128 k, 3312 with that GEMV).
+//
 // Weights are the left operand, straight from TMEM: a tile is 128 weight columns (TMEM lanes) by up to 128
 // tokens (any multiple of 16), so that few tokens cost few products and no shared-memory pass for weights.
 // Tiles are cut along K into chunks and the chunks of all tiles are shared out evenly over the CTAs (1 per SM); where a
@@ -88,6 +92,7 @@ struct SplitParams {
     uint32_t tok, m_tiles, tiles;   // tokens of a tile, tiles
     uint32_t chunks;                // per tile
     uint32_t units;                 // tiles * chunks
+    uint32_t fine;                  // an accumulator per 32 k, compensated sums; one group of 16 tokens only
     uint32_t wide;                  // packed weights can be copied 16 bytes at a time
 };
 
@@ -248,6 +253,24 @@ __device__ __forceinline__ void umma_f16_ts_scaled(uint32_t d, uint32_t a, uint3
                  "mov.b64 db, {%2, %4};\n\t"
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p, %5;\n\t}"
                  ::"r"(d), "r"(a), "r"(b16 | 0x10000u), "r"(instr), "r"(kDescHigh), "n"(kLowShift) : "memory");
+}
+// Products of the K = 16 steps from .. from + COUNT - 1 of a chunk into one accumulator, the small ones first.  open: it holds a chunk already.
+template <int PLANES, int COUNT>
+__device__ __forceinline__ void issue_products(uint32_t d, uint32_t w_hi, uint32_t w_lo, uint32_t x_hi, uint32_t x_lo, uint32_t sub16, uint32_t instr, uint32_t from, bool open)
+{
+    auto x_at = [&](uint32_t x, uint32_t j) { return x + ((from + j) / 4) * sub16 + ((from + j) % 4) * 2u; };
+    auto w_at = [&](uint32_t w, uint32_t j) { return w + (from + j) * 8u; };
+    if (PLANES == 2) {                                          // never two chunks per accumulator
+        umma_f16_ts<false>(d, w_at(w_hi, 0), x_at(x_lo, 0), instr);
+#pragma unroll
+        for (uint32_t j = 1; j < COUNT; j++) umma_f16_ts<true>(d, w_at(w_hi, j), x_at(x_lo, j), instr);
+        umma_f16_ts_scaled(d, w_at(w_lo, 0), x_at(x_hi, 0), instr);
+    } else if (open) umma_f16_ts<true>(d, w_at(w_lo, 0), x_at(x_hi, 0), instr);
+    else             umma_f16_ts<false>(d, w_at(w_lo, 0), x_at(x_hi, 0), instr);
+#pragma unroll
+    for (uint32_t j = 1; j < COUNT; j++) umma_f16_ts<true>(d, w_at(w_lo, j), x_at(x_hi, j), instr);
+#pragma unroll
+    for (uint32_t j = 0; j < COUNT; j++) umma_f16_ts<true>(d, w_at(w_hi, j), x_at(x_hi, j), instr);
 }
 // A converged warp waits for several barriers at once, a lane (with `mine` set) for each: the try_waits share one latency.
 __device__ __forceinline__ bool mbar_wait_lanes(unsigned long long *bar, uint32_t parity, bool mine, volatile int *failed)
@@ -457,6 +480,23 @@ __device__ __forceinline__ void drain_part(uint32_t from, const uint8_t *scale, 
         }
 }
 
+// sum += x; low collects what the sums round away.
+__device__ __forceinline__ void add_exact(float &sum, float &low, float x)
+{
+    const float s = __fadd_rn(sum, x), b = __fsub_rn(s, sum);
+    low = __fadd_rn(low, __fadd_rn(__fsub_rn(sum, __fsub_rn(s, b)), __fsub_rn(x, b)));
+    sum = s;
+}
+
+// drain_part for one group of 16 tokens; the scales are powers of two, so that the products are exact.
+__device__ __forceinline__ void drain_fine(uint32_t from, const uint8_t *scale, float (&sum)[16], float (&low)[16])
+{
+    uint32_t r[16];
+    tmem_ld16(from, r);
+#pragma unroll
+    for (int e = 0; e < 16; e++) add_exact(sum[e], low[e], __uint_as_float(r[e]) * *reinterpret_cast<const float *>(scale + e * 4));
+}
+
 // acc += the sums that another CTA has left.
 __device__ __forceinline__ void add_part(const float *src, uint32_t groups, float (&acc)[4][16])
 {
@@ -479,6 +519,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
     constexpr uint32_t kRawChunk = kCols * raw_bytes(FMT);
     constexpr uint32_t kParts = 2 * PLANES, kDepth = kSlots / kParts;       // sub-tiles of a chunk, chunks in the ring
     const uint32_t group = PLANES == 1 ? group_of(PLANES, p.k) : 1;
+    const bool fine = FMT == MGQ_FMT_Q8 && PLANES == 2 && p.fine;
     uint8_t *ring = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sub = p.tok * 128u;                          // bytes of a token sub-tile, a multiple of 2048
     const uint32_t scale_bytes = p.tok * 4u;                    // a multiple of 64
@@ -549,28 +590,34 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
             uint32_t chunk = __shfl_sync(0xffffffffu, u_begin % p.chunks, 0), filled = 0;      // accumulators so far
             bool ok = true, open = false;                       // open: the accumulator holds a chunk already
             for (uint32_t i = 0; i < count; i++) {
-                const uint32_t stage = i & 1u, ph = (i >> 1) & 1u, s = i % kDepth, b = filled & 1u;
+                const uint32_t stage = i & 1u, ph = (i >> 1) & 1u, s = i % kDepth;
+                uint32_t b = filled & 1u;
                 const bool close = group == 1 || chunk % group == group - 1 || chunk + 1 == p.chunks || i + 1 == count;
-                const uint32_t d = tm + b * kMaxTok, w_hi = tm + 2 * kMaxTok + stage * 128u, w_lo = w_hi + 64u;
+                const uint32_t w_hi = tm + 2 * kMaxTok + stage * 128u, w_lo = w_hi + 64u;
                 // lane 0: accumulator, 1: weights, 4..: the chunk's sub-tiles
                 unsigned long long *bar = lane == 0 ? &sh.d_empty[b] : lane == 1 ? &sh.w_full[stage] : &sh.slot_full[(s * kParts + lane - 4u) % kSlots];
                 const uint32_t parity = lane == 0 ? ((filled >> 1) & 1u) ^ 1u : lane == 1 ? ph : (i / kDepth) & 1u;
                 ok = mbar_wait_lanes(bar, parity, lane < 2 || (lane >= 4 && lane < 4 + kParts), &sh.failed);
                 if (!ok) break;
                 tc_fence_after();
+                const uint32_t x_lo = ring16 + s * kParts * sub16, x_hi = x_lo + (kParts - 2) * sub16;
+                if (fine) {                                     // all quarters of the chunk but the last
+                    for (uint32_t from = 0; from < 6; from += 2) {
+                        if (leader) {
+                            issue_products<PLANES, 2>(tm + b * kMaxTok, w_hi, w_lo, x_hi, x_lo, sub16, instr, from, false);
+                            umma_commit(&sh.d_full[b]);
+                        }
+                        __syncwarp();
+                        filled++;
+                        b = filled & 1u;
+                        ok = ok && mbar_wait_lanes(&sh.d_empty[b], ((filled >> 1) & 1u) ^ 1u, lane == 0, &sh.failed);
+                        tc_fence_after();
+                    }
+                    if (!ok) break;
+                }
                 if (leader) {
-                    const uint32_t x_lo = ring16 + s * kParts * sub16, x_hi = x_lo + (kParts - 2) * sub16;
-                    if (PLANES == 2) {                          // never two chunks per accumulator
-                        umma_f16_ts<false>(d, w_hi, x_lo, instr);
-#pragma unroll
-                        for (uint32_t j = 1; j < 8; j++) umma_f16_ts<true>(d, w_hi + j * 8u, x_lo + (j / 4) * sub16 + (j % 4) * 2u, instr);
-                        umma_f16_ts_scaled(d, w_lo, x_hi, instr);
-                    } else if (open) umma_f16_ts<true>(d, w_lo, x_hi, instr);
-                    else             umma_f16_ts<false>(d, w_lo, x_hi, instr);
-#pragma unroll
-                    for (uint32_t j = 1; j < 8; j++) umma_f16_ts<true>(d, w_lo + j * 8u, x_hi + (j / 4) * sub16 + (j % 4) * 2u, instr);
-#pragma unroll
-                    for (uint32_t j = 0; j < 8; j++) umma_f16_ts<true>(d, w_hi + j * 8u, x_hi + (j / 4) * sub16 + (j % 4) * 2u, instr);
+                    if (fine) issue_products<PLANES, 2>(tm + b * kMaxTok, w_hi, w_lo, x_hi, x_lo, sub16, instr, 6, false);
+                    else      issue_products<PLANES, 8>(tm + b * kMaxTok, w_hi, w_lo, x_hi, x_lo, sub16, instr, 0, open);
                     umma_commit(&sh.w_empty[stage]);
                     umma_commit(&sh.slot_empty[s]);
                     if (close) umma_commit(&sh.d_full[b]);
@@ -606,26 +653,35 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                 for (int e = 0; e < 16; e++) acc[g][e] = 0.f;
             for (uint32_t c = c0; c < c1; c++, i++) {
                 if (group > 1 && c % group != group - 1 && c + 1 != c1) continue;            // the next chunk goes into the same accumulator
-                const uint32_t b = filled & 1u, sc = i % kScaleSlots, span = group > 1 ? min(c % group, c - c0) + 1 : 1;
+                const uint32_t sc = i % kScaleSlots, span = group > 1 ? min(c % group, c - c0) + 1 : 1;
                 const uint32_t x = i + 1 - lane;                // lane 0: the accumulator, 1..span: scales of its chunks
-                mbar_wait_lanes(lane == 0 ? &sh.d_full[b] : &sh.sc_full[x % kScaleSlots], lane == 0 ? (filled >> 1) & 1u : (x / kScaleSlots) & 1u, lane <= span, &sh.failed);
-                filled++;
-                __syncwarp();                                   // tcgen05.ld is warp-collective
-                tc_fence_after();
-                const uint32_t from = tmem + lane_addr + b * kMaxTok + first;
                 const uint8_t *scale = scale_ring + sc * scale_bytes + first * 4u;
-                if (mine > 1) drain_part<0, 2>(from, scale, acc);
-                else if (mine > 0) drain_part<0, 1>(from, scale, acc);
-                if (mine > 3) drain_part<2, 2>(from, scale, acc);
-                else if (mine > 2) drain_part<2, 1>(from, scale, acc);
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&sh.d_empty[b]);
-                    for (uint32_t x = 0; x < span; x++) mbar_arrive(&sh.sc_empty[(i - x) % kScaleSlots]);
+                for (uint32_t h = fine ? 0 : 3; h < 4; h++) {
+                    const uint32_t b = filled & 1u;
+                    mbar_wait_lanes(lane == 0 ? &sh.d_full[b] : &sh.sc_full[x % kScaleSlots], lane == 0 ? (filled >> 1) & 1u : (x / kScaleSlots) & 1u, lane <= span, &sh.failed);
+                    filled++;
+                    __syncwarp();                               // tcgen05.ld is warp-collective
+                    tc_fence_after();
+                    const uint32_t from = tmem + lane_addr + b * kMaxTok + first;
+                    if (fine) {
+                        if (mine > 0) drain_fine(from, scale, acc[0], acc[1]);
+                    } else {
+                        if (mine > 1) drain_part<0, 2>(from, scale, acc);
+                        else if (mine > 0) drain_part<0, 1>(from, scale, acc);
+                        if (mine > 3) drain_part<2, 2>(from, scale, acc);
+                        else if (mine > 2) drain_part<2, 1>(from, scale, acc);
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sh.d_empty[b]);
                 }
+                if (lane == 0)
+                    for (uint32_t y = 0; y < span; y++) mbar_arrive(&sh.sc_empty[(i - y) % kScaleSlots]);
             }
             u += c1 - c0;
+            if (fine)                                           // before any part is added: the sum of two must not depend on which comes last
+#pragma unroll
+                for (int e = 0; e < 16; e++) acc[0][e] += acc[1][e];
 
             bool finish = true;
             if (c0 != 0 || c1 != p.chunks) {
@@ -669,7 +725,20 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                         for (int g = 0; g < 4; g++)
 #pragma unroll
                             for (int e = 0; e < 16; e++) acc[g][e] = 0.f;
-                        for (uint32_t s = head; s <= tail; s++) add_part(part_of(s), mine, acc);      // this CTA's own part among them
+                        if (fine) {
+                            for (uint32_t s = head; s <= tail && mine > 0; s++) {
+                                const float *part = part_of(s);
+                                float v[16];
+#pragma unroll
+                                for (int e = 0; e < 16; e++) v[e] = __ldcg(part + e * kCols);
+#pragma unroll
+                                for (int e = 0; e < 16; e++) add_exact(acc[0][e], acc[1][e], v[e]);
+                            }
+#pragma unroll
+                            for (int e = 0; e < 16; e++) acc[0][e] += acc[1][e];
+                        } else {
+                            for (uint32_t s = head; s <= tail; s++) add_part(part_of(s), mine, acc);      // this CTA's own part among them
+                        }
                     }
                 }
             }
@@ -863,6 +932,7 @@ int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const 
         p.units = (uint32_t)units;
         // Q8: whole 16-byte pieces of 4 blocks; Q4: nibbles behind num_blocks header words
         p.wide = q4 ? p.num_blocks % 4 == 0 : p.bpc % 4 == 0;
+        p.fine = !q4 && !bf16 && m <= MGQ_GEMV_MAX_M && !gemv_streamable(fmt, a, k, n) && !gemv_mma_eligible(m, k, n, a, w);
         const uint32_t ctas = p.units / 2 < 1 ? 1 : p.units / 2 < (uint32_t)sms ? p.units / 2 : (uint32_t)sms;
 
         const size_t plane_bytes = (size_t)p.m_tiles * p.chunks * 2 * planes * p.tok * 128;

@@ -648,23 +648,28 @@ bool gemv_streamable(int fmt, const void *x, uint32_t k, uint32_t n)
     return ((unsigned long long)bpc * n) % 4 == 0 && (reinterpret_cast<uintptr_t>(x) % 16 == 0);
 }
 
-// Up to 16 f32 rows for which the tensor-core GEMM is ahead (microseconds, GEMV / GEMM):
-//   8 rows per pass (mma kernel): a second pass over large Q8 weights, 16 x 4096 x 6144 30 / 25, x 24576 70 / 52 (Q4: 25 / 25, 55 / 52; 8 rows: 35 / 52)
-//   2 rows per pass (streaming):  from the third pass on, K = 1056, N = 4096: 4 rows 15 / 19, 6 rows 22 / 19, 16 rows 59 / 19
-//   1 row per pass (streaming with more than 512 threads): from the fourth, 4128 x 4096 Q8 3 rows 22 / 25, 4 rows 29 / 25; large ones
-//   from the third, 4128 x 24576 Q8 47 / 58 and 70 / 58
-//   1 row at a time, 4-byte loads (general kernel): 2080 x 4096 39 / 21 per row, 8800 x 3840 150 / 29; 17 us are the GEMM's two launches
+// Up to 16 f32 rows for which the tensor-core GEMM is ahead (microseconds of one call by itself, GEMV / GEMM; the GEMM's two launches alone are 17):
+//   8 rows per pass (mma kernel): a second pass over large Q8 weights, 16 x 4096 x 6144 36 / 29, 9 x 4096 x 24576 75 / 58 (Q4: 32 / 32)
+//   2 rows per pass (streaming): from the third pass on, K = 1056, N = 4096: 4 rows 21 / 21, 5 rows 26 / 21, 16 rows 67 / 21; narrow
+//   weights leave most SMs to the other passes: N = 192, 5 and 8 rows of K = 1056 17 / 21, 24 / 21, of K = 6176 24 / 29, 33 / 29
+//   1 row per pass (streaming with more than 512 threads): from the fourth, 4128 x 4096 Q8 3 rows 30 / 29, 4 rows 38 / 29; large ones
+//   from the third, 4128 x 24576 Q8 85 / 64
+//   1 row at a time, 4-byte loads (general kernel): goes by K for few columns, 193 of K = 608 5 and 6 rows 20 / 21, 23 / 21, of 2080
+//   1 and 2 rows 16 / 25, 25 / 25, one row of 4128 and 6176 25 / 29, 34 / 33; by all of the work for many, 288 x 4099 2 and 3 rows
+//   16 / 20, 22 / 20, one row of 1056 and 2080 x 4099 about 24 / 25, 40 / 29
+// Nothing that goes there comes farther from the exact product than with the GEMV.
 bool gemv_prefers_gemm(int fmt, uint32_t m, uint32_t k, uint32_t n, const void *x, const void *w)
 {
     if (k <= 128 || !g_tuning.batch_mma) return false;
-    if (gemv_mma_eligible(m, k, n, x, w)) return fmt == MGQ_FMT_Q8 && m > 8 && (unsigned long long)k * n >= 20000000ull;
+    const unsigned long long size = (unsigned long long)k * n;
+    if (gemv_mma_eligible(m, k, n, x, w)) return fmt == MGQ_FMT_Q8 && m > 8 && size >= 20000000ull;
     if (gemv_streamable(fmt, x, k, n)) {
         const uint32_t bpc = k / 32;
         const bool single = bpc > 512 || (fmt == MGQ_FMT_Q8 && bpc % 4 != 0 && columns_for(bpc <= 256 ? 256u : (bpc + 31u) & ~31u, bpc) == 0 && (bpc % 2 == 0 ? 2u : 4u) * bpc > 512);
-        if (single) return m >= ((unsigned long long)k * n >= 50000000ull ? 3u : 4u);
-        return m >= 5;
+        if (single) return m >= (size >= 50000000ull ? 3u : 4u);
+        return m >= (n >= 1024 ? 5u : k <= 4096 ? 8u : 12u);
     }
-    return (unsigned long long)m * k > 1024;
+    return (unsigned long long)m * k >= (m == 1 ? 6144u : 3456u) || m * size >= (m == 1 ? 6000000ull : 3500000ull);
 }
 
 int launch_gemv(int fmt, const float *x, const void *w, const float *addend, float *y,

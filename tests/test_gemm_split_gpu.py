@@ -274,3 +274,19 @@ def test_span_of_magnitudes(fmt, act, size):
     bound = max(_bound(act, k), 2 * (k / 3) ** 0.5 * 2.0 ** -24)
     for r in range(m):
         assert r == 5 or O.rel_l2(got[r], want[r]) <= bound
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+# shapes that do not stream and ones that do, each with the rows from which on the GEMM takes them
+@pytest.mark.parametrize("m,k,n", [(16, 288, 193), (16, 576, 1001), (1, 6176, 193), (1, 2912, 2099), (2, 8800, 3841), (3, 12320, 1001), (5, 1056, 4096), (16, 4128, 64), (16, 4096, 4896)])
+def test_few_rows_lose_nothing(fmt, m, k, n):
+    """Up to 16 f32 rows that leave the GEMV for the GEMM come no farther from the exact product."""
+    import torch
+    from meganeura_b200 import ops
+    w, x = _q4_weights("quantized", k, n, 1) if fmt == O.FMT_Q4 else _inputs(fmt, m, k, n)[0], _inputs(fmt, m, k, n)[1]
+    want = x.astype(np.float64) @ _dense(fmt, w, k, n)
+    got = {r: run_matmul(fmt, x, w, k, n, route=r) for r in ("auto", "gemv", "gemm")}
+    again = run_matmul(fmt, x, w, k, n, route="gemm")
+    assert np.array_equal(got["gemm"], again)                 # sums do not depend on which CTA comes last
+    assert O.rel_l2(got["gemm"], want) <= O.rel_l2(got["gemv"], want)
+    assert O.rel_l2(got["auto"], want) <= O.rel_l2(got["gemv"], want)
