@@ -189,7 +189,7 @@ int mgq_exchange_all_gather_rows(const float *slice, uint32_t slice_pitch, uint3
 /* c[m,n] = a[m,k] . dequant(w)[k,n] (+ addend[m,n]); a is f32 or bf16 row-major, c is f32.
  * Stands in for the MatMul / FusedMatMulAdd dispatches with a quantized weight_format
  * (src/compile.rs:1408-1419, 1511-1522; src/shaders/matmul.wgsl:28-109).
- * Calls with k > 128 run on the tensor cores (tcgen05, operands as sums of f16 values, f32 accuracy) with a
+ * Calls with k > 128, and large ones with k = 128 and bf16, run on the tensor cores (tcgen05, operands as sums of f16 values, f32 accuracy) with a
  * stream-ordered workspace from a memory pool of the library (at most 256 MB of it are kept between calls); shorter k, and
  * calls whose workspace cannot be allocated, run the register-tiled CUDA-core kernel. */
 int mgq_gemm(int fmt, const void *a, int a_dtype, const void *w, const float *addend, float *c,

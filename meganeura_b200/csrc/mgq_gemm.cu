@@ -4,7 +4,8 @@
 // (src/compile.rs:1408-1419, 1511-1522; kernel src/shaders/matmul.wgsl:28-109 with
 // dequant_q4 / dequant_q8 as the B-tile load, src/codegen.rs:702-713).
 //
-// The tensor-core kernel of mgq_gemm_split.cu takes every shape with K > 128.  gemm_tiled_kernel is what is left for short K
+// The tensor-core kernel of mgq_gemm_split.cu takes every shape with K > 128, and large ones of K = 128 with bf16
+// activations.  gemm_tiled_kernel is what is left for short K
 // and for calls whose workspace cannot be allocated (any M, any N, f32 or bf16 activations): a 64x64x32
 // register-tiled f32 contraction on the CUDA cores in which each K-tile is exactly one
 // quantization block per column, so a block header is decoded once per 32 weights (the
@@ -124,9 +125,12 @@ int set_gemm_option(const char *name, long value)
 int launch_gemm(int fmt, const void *a, int a_dtype, const void *w, const float *addend, float *c,
                 uint32_t m, uint32_t k, uint32_t n, void *stream_v)
 {
-    // Up to 128 k the tiled kernel is done (4 steps, 14 us with its launch) before the split kernel's two launches and its pipeline
-    // are under way (20 us); from 256 k on the split kernel is ahead (512 x 256 x 2048: 15 against 27 us, 17 x 576 x 192: 17 against 29).
-    if (!force_tiled() && k > 128) {
+    // Up to 128 k a wave of tiles is done (4 steps, 14 us with its launch) before the split kernel's two launches and its pipeline
+    // are under way (17 us); from 256 k on the split kernel is ahead (512 x 256 x 2048: 15 against 27 us, 17 x 576 x 192: 17 against 29).
+    // Many tiles of 128 k and bf16 rows take the split kernel, which is as exact there (f32 rows would lose bits): m x n = 2^20 18 / 18,
+    // 2^21 19 / 31, 2048 x 16384 60 to 72 / 330 us.
+    const bool wide = a_dtype == MGQ_A_BF16 && k == 128 && m >= 64 && (unsigned long long)m * n > 1u << 20;
+    if (!force_tiled() && (k > 128 || wide)) {
         uint32_t done = 0;
         if (int rc = launch_gemm_split(fmt, a, a_dtype, w, addend, c, m, k, n, stream_v, &done)) return rc;
         if (done == m) return MGQ_OK;

@@ -290,3 +290,23 @@ def test_few_rows_lose_nothing(fmt, m, k, n):
     assert np.array_equal(got["gemm"], again)                 # sums do not depend on which CTA comes last
     assert O.rel_l2(got["gemm"], want) <= O.rel_l2(got["gemv"], want)
     assert O.rel_l2(got["auto"], want) <= O.rel_l2(got["gemv"], want)
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+# below, at and above the line where bf16 rows of K = 128 leave the tiled kernel; fewer than 64 rows stay
+@pytest.mark.parametrize("m,n,split", [(64, 16384, False), (64, 16388, True), (200, 5251, True), (1030, 1030, True), (63, 17000, False)])
+def test_one_chunk_of_bf16(fmt, m, n, split):
+    import torch
+    from meganeura_b200 import ops
+    k = 128
+    w = _q4_weights("quantized", k, n, m) if fmt == O.FMT_Q4 else _inputs(fmt, m, k, n)[0]
+    xd, wd = to_dev(_inputs(fmt, m, k, n)[1]).to(torch.bfloat16), to_dev(w)
+    got = ops.matmul(fmt, xd, wd, k, n)
+    ops.set_option("gemm.force_tiled", 1)
+    try:
+        tiled = ops.matmul(fmt, xd, wd, k, n)
+    finally:
+        ops.set_option("gemm.force_tiled", 0)
+    assert torch.equal(got, tiled) != split
+    want = xd.double().cpu().numpy() @ _dense(fmt, w, k, n)
+    assert O.rel_l2(got.cpu().numpy(), want) <= _bound("bf16", k)
