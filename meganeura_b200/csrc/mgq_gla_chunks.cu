@@ -15,8 +15,11 @@
 //                       the records come through a ring of cp.async copies
 // State, decays and sums are f32.  Where the state is read it enters as the sum of three bf16, i.e. with all its
 // bits; the decayed queries and keys, A and the values as sums of two, three products each: 16 to 17 significant bits
-// of numbers whose factors are projections, with the range of f32.  Time mixing and mLSTM take sums of three everywhere (six
-// products each, 24 bits) and add a chunk's update to the state in f32.  A long portion is cut into segments:
+// of numbers whose factors are projections, with the range of f32.  Time mixing and mLSTM take sums of three everywhere and six of
+// the nine products (what is left out is below 2^-26 of a product).  The tensor cores truncate what they accumulate, so there every
+// block of 16 keys is summed by itself and added in f32.  Against 64 bits, this and token by token: time mixing 64 x 64 with
+// decays around 0.95 1.24e-7 / 1.21e-7, 0.999 3.7e-7 / 4.5e-7, mLSTM 128 x 256 6.3e-7 / 8.2e-7 (all blocks in one
+// accumulator: 4.4e-7, 6.9e-7, 1.8e-6).  A long portion is cut into segments:
 // a first pass leaves the end state of every segment but the last, each started from nothing, gla_combine_kernel
 // turns them into the segments' start states, and a second pass runs all segments with outputs.
 // 2048 tokens, all launches: mLSTM 8 x 128 x 256 190 us against 311 token by token, time mixing 32 x 64 x 64 about 100 against 138.
@@ -285,14 +288,15 @@ __global__ void __launch_bounds__(256) gla_prepare_kernel(const __grid_constant_
     }
     __syncthreads();
     if (t < 128) {                                       // two neighbouring keys of one query
-        float2 x = make_float2(0.f, 0.f);
+        float2 sum[4] = {};                              // three parts: four short sums round less than one
 #pragma unroll
         for (int i = 0; i < (int)SLICES; i++) {
             const float2 y = *reinterpret_cast<const float2 *>(sa + i * kChunk * kChunk + 2 * t);
+            float2 &x = sum[PARTS == 3 ? i % 4 : 0];
             x.x += y.x; x.y += y.y;
         }
         uint32_t part[3];
-        split_parts<PARTS>(x.x, x.y, part);
+        split_parts<PARTS>((sum[0].x + sum[1].x) + (sum[2].x + sum[3].x), (sum[0].y + sum[1].y) + (sum[2].y + sum[3].y), part);
 #pragma unroll
         for (int h = 0; h < PARTS; h++) *reinterpret_cast<uint32_t *>(rec + R::a + h * kChunk * kChunk * 2 + 4 * t) = part[h];
     }
@@ -410,12 +414,15 @@ __global__ void __launch_bounds__(256, 1) gla_chunks_kernel(const __grid_constan
             }
 #pragma unroll
             for (int h = 0; h < PARTS; h++) ldmatrix4_t(base + k_off + h * R::matrix + j * 32, kq[h]);
-            float add[2][4] = {};                        // three parts: the update by itself, added in f32
+            float add[2][4] = {}, out[2][4] = {};        // three parts: each block of 16 keys by itself, added in f32
+            float f[2][2];                               // the chunk's decay of this thread's keys
 #pragma unroll
             for (int n = 0; n < 2; n++) {
-                const float2 f = *reinterpret_cast<const float2 *>(rec + R::lam + (j * 16 + n * 8 + tq * 2) * 4);
-                float (&x)[4] = S[2 * j + n];
-                x[0] *= f.x; x[1] *= f.y; x[2] *= f.x; x[3] *= f.y;
+                const float2 l = *reinterpret_cast<const float2 *>(rec + R::lam + (j * 16 + n * 8 + tq * 2) * 4);
+                f[n][0] = l.x; f[n][1] = l.y;
+                if (PARTS == 2)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) S[2 * j + n][e] *= f[n][e & 1];
             }
             // small products first (the two factors' parts count 2^-8 each); the sums are independent of each other
 #pragma unroll
@@ -425,8 +432,8 @@ __global__ void __launch_bounds__(256, 1) gla_chunks_kernel(const __grid_constan
                     const int y = order - x;
                     if (y >= PARTS) continue;
                     if (outputs) {
-                        mma16816(o[0], sp[x], qp[y][0], qp[y][1]);
-                        mma16816(o[1], sp[x], qp[y][2], qp[y][3]);
+                        mma16816(PARTS == 3 ? out[0] : o[0], sp[x], qp[y][0], qp[y][1]);
+                        mma16816(PARTS == 3 ? out[1] : o[1], sp[x], qp[y][2], qp[y][3]);
                     }
                     if (PARTS == 2 && (order == 2 || x >= PARTS)) continue;
                     mma16816(PARTS == 3 ? add[0] : S[2 * j], vp[x], kq[y][0], kq[y][1]);
@@ -436,7 +443,10 @@ __global__ void __launch_bounds__(256, 1) gla_chunks_kernel(const __grid_constan
 #pragma unroll
                 for (int n = 0; n < 2; n++)
 #pragma unroll
-                    for (int e = 0; e < 4; e++) S[2 * j + n][e] += add[n][e];
+                    for (int e = 0; e < 4; e++) {
+                        S[2 * j + n][e] = fmaf(S[2 * j + n][e], f[n][e & 1], add[n][e]);
+                        o[n][e] += out[n][e];
+                    }
         }
         if (product)
             for (uint32_t d = t; d < (uint32_t)D; d += threads) s_f[d] *= *reinterpret_cast<const float *>(rec + R::lam + d * 4);
@@ -450,10 +460,14 @@ __global__ void __launch_bounds__(256, 1) gla_chunks_kernel(const __grid_constan
                 ap[h][0] = *reinterpret_cast<const uint32_t *>(a + h * kChunk * kChunk * 2);
                 ap[h][1] = *reinterpret_cast<const uint32_t *>(a + h * kChunk * kChunk * 2 + 16);
             }
+            float in[4] = {};                            // from inside the chunk
 #pragma unroll
             for (int order = PARTS - 1; order >= 0; order--)
 #pragma unroll
-                for (int x = 0; x <= order; x++) mma16816(o[n], vp[x], ap[order - x][0], ap[order - x][1]);
+                for (int x = 0; x <= order; x++) mma16816(PARTS == 3 ? in : o[n], vp[x], ap[order - x][0], ap[order - x][1]);
+            if (PARTS == 3)
+#pragma unroll
+                for (int e = 0; e < 4; e++) o[n][e] += in[e];
 #pragma unroll
             for (int e = 0; e < 4; e++) {
                 const uint32_t row = c * kChunk + n * 8 + tq * 2 + (e & 1);

@@ -88,3 +88,56 @@ def test_wkv(heads, dim, rank):
         oo = P.wkv_scan(*(a.reshape(cnt, heads, dim) for a in (ro, ko, vo)), P.wkv_decay(low, w1, w2, w0).reshape(cnt, heads, dim), u.reshape(heads, dim), S)
         close(got, P.unit_rms(oo, 1e-4).reshape(cnt, n) * hw * go * P.sigmoid(go), 2 ** -8)
 
+
+
+@pytest.mark.parametrize("kind,heads,dim,vdim", [("wkv", 2, 64, 64), ("wkv", 1, 128, 128), ("wkv", 1, 256, 256), ("mlstm", 2, 64, 100), ("mlstm", 1, 128, 256), ("mlstm", 1, 256, 64)])
+def test_no_farther_from_64_bits_than_token_by_token(kind, heads, dim, vdim):
+    """The second half of every head's keys repeats the first, and the queries of both cancel to 2^-12: what is left of an output
+    shows the last bits of f32 sums through the bf16 rounding.  A long portion may be as far off as the same tokens in short
+    ones, which take the token-by-token kernels; a third part left out, or sums that truncate, are three times as far and more."""
+    import meganeura_b200 as mg
+    from meganeura_b200._lib import FMT_BF16, GATE_SIGMOID, ROWS_TOKENS, lib
+    r = rng_of(heads, dim, vdim, 5)
+    rows, short, half, rank, delta = 512, 32, dim // 2, 4, 2.0 ** -12
+    n, nv = heads * dim, heads * vdim
+
+    def doubled(a):                                           # [.., heads, half] -> [.., heads * dim]
+        return np.concatenate([a, a], -1).reshape(*a.shape[:-2], n).astype(np.float32)
+    q1 = r.standard_normal((rows, heads, half))
+    q = np.concatenate([q1, -q1 * (1 + delta * r.standard_normal(q1.shape))], -1).reshape(rows, n).astype(np.float32)
+    tabs = {"q": q, "k": doubled(r.standard_normal((rows, heads, half))), "v": r.standard_normal((rows, nv)).astype(np.float32), "g": np.zeros((rows, nv), np.float32)}
+    g = mg.Graph()
+    ids = g.input_u32_rows("ids", rows, ROWS_TOKENS)
+    params = {"hw": np.ones(nv, np.float32)}
+    if kind == "mlstm":
+        tabs |= {c: (r.standard_normal((rows, heads)) + b).astype(np.float32) for c, b in (("i", 0), ("f", 3))}
+    else:
+        tabs["low"] = (r.standard_normal((rows, rank)) * 0.3).astype(np.float32)
+        params |= {"w2": bf16_round(doubled(r.standard_normal((rank, heads, half))).T.copy() * np.float32(0.2)), "w0": doubled(r.uniform(-6, -2, (heads, half))),
+                   "u": doubled(r.standard_normal((heads, half)))}
+    e = {c: g.embedding_scaled(ids, g.parameter(c, list(a.shape)), 1.0) for c, a in tabs.items()}
+    if kind == "mlstm":
+        o = g.mlstm(e["q"], e["k"], e["v"], e["i"], e["f"], g.parameter("state", [lib.mgq_mlstm_state_elements(heads, dim, vdim)]), heads, 15.0)
+    else:
+        decay = g.lora_decay(e["low"], g.parameter_bf16("w2", [n, rank]), g.parameter("w0", [n]))
+        o = g.wkv(e["q"], e["k"], e["v"], decay, g.parameter("u", [n]), g.parameter("state", [lib.mgq_wkv_state_elements(heads, dim)]), heads)
+    params |= tabs
+    y = _identity(g, g.head_gate(o, e["g"], heads, g.parameter("hw", [nv]), 1e-20, GATE_SIGMOID, FMT_BF16), nv, params)
+    d = {c: a.astype(np.float64) for c, a in tabs.items()}
+    qq, kk, vv = d["q"].reshape(rows, heads, dim), d["k"].reshape(rows, heads, dim), d["v"].reshape(rows, heads, vdim)
+    if kind == "mlstm":
+        oo = P.mlstm_scan(qq * dim ** -0.5, kk, vv, *P.mlstm_gates(d["i"], d["f"], 15.0), np.zeros((heads, dim, vdim)), np.zeros((heads, dim)), np.zeros(heads))
+    else:
+        w = np.exp(-np.exp(np.tanh(d["low"]) @ params["w2"].astype(np.float64).T + params["w0"])).reshape(rows, heads, dim)
+        oo = P.wkv_scan(qq, kk, vv, w, params["u"].astype(np.float64).reshape(heads, dim), np.zeros((heads, dim, dim)))
+    want = P.unit_rms(oo, 1e-20).reshape(rows, nv) * 0.5
+    off = {}
+    for portion in (rows, short):
+        s = session(g, [y], params)
+        got = []
+        for at in range(0, rows, portion):
+            s.set_rows(ROWS_TOKENS, portion)
+            s.set_input_u32("ids", np.arange(at, at + portion))
+            got.append(run(s, (portion, nv)))
+        off[portion] = np.linalg.norm(np.concatenate(got) - want) / np.linalg.norm(want)
+    assert off[rows] <= 1.5 * off[short] + 2.0 ** -10         # bf16 rounding is in both
