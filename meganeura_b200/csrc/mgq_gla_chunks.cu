@@ -31,6 +31,9 @@ namespace mgq {
 namespace {
 
 constexpr uint32_t kChunk = 16, kStages = 3, kMaxWarps = 8, kMaxSegs = 16;
+// Time mixing and mLSTM take longer portions in pieces, whose records (31 KB per token with 32 heads of 64 channels) then share 64 MB; a
+// piece fills the chip.
+constexpr uint32_t kPieceRows = 2048;
 
 enum { kGla = 0, kWkv = 1, kMlstm = 2 };
 __host__ __device__ constexpr int parts_of(int mode) { return mode == kGla ? 2 : 3; }
@@ -588,7 +591,7 @@ int launch_sized(Chunks p, cudaStream_t st)
 }
 
 template <int MODE>
-int launch_chunks(Chunks p, void *workspace, cudaStream_t st)
+int launch_piece(Chunks p, void *workspace, cudaStream_t st)
 {
     p.cols = p.vdim + (MODE == kMlstm ? 1 : 0);
     p.chunks = (p.rows + kChunk - 1) / kChunk;
@@ -613,9 +616,28 @@ int launch_chunks(Chunks p, void *workspace, cudaStream_t st)
     }
 }
 
+template <int MODE>
+int launch_chunks(const Chunks &all, void *workspace, cudaStream_t st)
+{
+    const uint32_t piece = MODE == kGla ? all.rows : kPieceRows;
+    for (uint32_t r0 = 0; r0 < all.rows; r0 += piece) {
+        Chunks p = all;
+        p.rows = std::min(piece, all.rows - r0);
+        const size_t keys = (size_t)r0 * p.heads * p.dim, values = (size_t)r0 * p.heads * p.vdim, gates = (size_t)r0 * p.heads;
+        p.q += keys; p.k += keys; p.v += values; p.o += values;
+        if (p.w) p.w += keys;
+        if (p.d.low) p.d.low += (size_t)r0 * p.d.rank;
+        if (MODE == kMlstm) { p.gi += gates; p.gf += gates; }
+        if (r0) p.shift_state = nullptr;
+        if (int rc = launch_piece<MODE>(p, workspace, st)) return rc;
+    }
+    return MGQ_OK;
+}
+
 size_t chunks_workspace(int mode, uint32_t max_rows, uint32_t heads, uint32_t dim, uint32_t vdim)
 {
     if (max_rows < kPrefillRows) return 0;
+    if (mode != kGla) max_rows = std::min(max_rows, kPieceRows);
     const size_t chunks = (max_rows + kChunk - 1) / kChunk, cols = vdim + (mode == kMlstm ? 1 : 0);
     return align256(chunks * heads * record_bytes(mode, dim)) + (mode == kMlstm ? align256((size_t)max_rows * heads * 16) + align256((size_t)max_rows * heads * 4) : 0) +
            (size_t)kMaxSegs * heads * (cols + 1) * padded(dim) * 4;

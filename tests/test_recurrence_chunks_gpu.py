@@ -141,3 +141,54 @@ def test_no_farther_from_64_bits_than_token_by_token(kind, heads, dim, vdim):
             got.append(run(s, (portion, nv)))
         off[portion] = np.linalg.norm(np.concatenate(got) - want) / np.linalg.norm(want)
     assert off[rows] <= 1.5 * off[short] + 2.0 ** -10         # bf16 rounding is in both
+
+
+@pytest.mark.parametrize("kind", ["wkv", "mlstm"])
+def test_long_portions_in_pieces(kind):
+    """Portions longer than a piece of 2048 tokens give the bits that separate portions give, and the workspace does not grow with
+    the capacity beyond a piece."""
+    import torch
+    import meganeura_b200 as mg
+    from meganeura_b200._lib import FMT_BF16, FMT_F32, GATE_SIGMOID, ROWS_TOKENS, lib
+    heads, dim, rank = 8, 32, 4
+    r = rng_of(heads, dim)
+    n = heads * dim
+    tabs = {c: r.standard_normal((90, n)).astype(np.float32) for c in "qkvg"} | {c: r.standard_normal((90, heads)).astype(np.float32) + b for c, b in (("i", 0), ("f", 3))}
+    tabs["low"] = (r.standard_normal((90, rank)) * 0.3).astype(np.float32)
+
+    def build(rows, out_dtype):
+        g = mg.Graph()
+        ids = g.input_u32_rows("ids", rows, ROWS_TOKENS)
+        e = {c: g.embedding_scaled(ids, g.parameter(c, list(a.shape)), 1.0) for c, a in tabs.items()}
+        params = {**tabs, "hw": np.ones(n, np.float32)}
+        if kind == "mlstm":
+            o = g.mlstm(e["q"], e["k"], e["v"], e["i"], e["f"], g.parameter("state", [lib.mgq_mlstm_state_elements(heads, dim, dim)]), heads, 15.0)
+        else:
+            params |= {"w2": bf16_round(r.standard_normal((n, rank)).astype(np.float32) * 0.2), "w0": np.full(n, -4, np.float32), "u": np.ones(n, np.float32)}
+            decay = g.lora_decay(e["low"], g.parameter_bf16("w2", [n, rank]), g.parameter("w0", [n]))
+            o = g.wkv(e["q"], e["k"], e["v"], decay, g.parameter("u", [n]), g.parameter("state", [lib.mgq_wkv_state_elements(heads, dim)]), heads)
+        y = _identity(g, g.head_gate(o, e["g"], heads, g.parameter("hw", [n]), 1e-5, GATE_SIGMOID, out_dtype), n, params) if out_dtype == FMT_BF16 else \
+            g.head_gate(o, e["g"], heads, g.parameter("hw", [n]), 1e-5, GATE_SIGMOID, out_dtype)
+        return session(g, [y], params)
+
+    s, outs = build(4500, FMT_BF16), []
+    for portions in ((4500,), (2048, 2048, 404)):
+        s.reset_state()
+        got, at = [], 0
+        for cnt in portions:
+            s.set_rows(ROWS_TOKENS, cnt)
+            s.set_input_u32("ids", np.arange(at, at + cnt) * 7 % 90)
+            got.append(run(s, (cnt, n)))
+            at += cnt
+        outs.append(np.concatenate(got))
+    assert np.isfinite(outs[0]).all() and np.array_equal(outs[0], outs[1])
+    del s
+
+    def taken(rows, out_dtype):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        keep = build(rows, out_dtype)
+        return before - torch.cuda.mem_get_info()[0]
+    grown = {d: taken(40000, d) - taken(8000, d) for d in (FMT_BF16, FMT_F32)}
+    buffers = 32000 * n * 2                                   # bf16 output beside an f32 one, and the linear layer behind it
+    assert grown[FMT_BF16] <= grown[FMT_F32] + buffers + (8 << 20)
