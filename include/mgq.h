@@ -190,8 +190,12 @@ int mgq_exchange_all_gather_rows(const float *slice, uint32_t slice_pitch, uint3
  * Stands in for the MatMul / FusedMatMulAdd dispatches with a quantized weight_format
  * (src/compile.rs:1408-1419, 1511-1522; src/shaders/matmul.wgsl:28-109).
  * Calls with k > 128, and large ones with k = 128 and bf16, run on the tensor cores (tcgen05, operands as sums of f16 values, f32 accuracy) with a
- * stream-ordered workspace from a memory pool of the library (at most 256 MB of it are kept between calls); shorter k, and
- * calls whose workspace cannot be allocated, run the register-tiled CUDA-core kernel. */
+ * stream-ordered workspace from a memory pool of the library (up to about 150 MB; at most 256 MB are kept between
+ * calls); shorter k, and calls whose workspace cannot be allocated, run the register-tiled CUDA-core kernel, which is
+ * up to 12 times slower for large shapes.  Captured calls put kernels into the graph and no allocations; the graph owns their
+ * workspace, one per stream of the capture, so two executables of one graph must not run at the same time.  An f32 or bf16
+ * value keeps its accuracy beside values up to 2^29 (bf16: 2^27) times larger in the same 128 (256) k; rows that span more are
+ * summed in plain f32, as are rows with infinities and with values from 2^120 on. */
 int mgq_gemm(int fmt, const void *a, int a_dtype, const void *w, const float *addend, float *c,
              uint32_t m, uint32_t k, uint32_t n, void *stream);
 

@@ -55,7 +55,10 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
+#include <utility>
+#include <vector>
 
 #include "mgq_launch.cuh"
 #include "mgq_tcgen05.cuh"
@@ -859,7 +862,13 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
 
 // ------------------------------------------------------------------------------------------ workspace
 
-// Stream-ordered, so calls on different streams and threads never share a block; up to kKeep bytes stay with the pool
+struct RelaxedCapture {                            // what this thread calls meanwhile is no part of any capture
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Outside of captures: stream-ordered, so calls on different streams and threads never share a block; up to kKeep bytes stay with the pool
 // between calls, the rest goes back to the device.
 constexpr unsigned long long kKeep = 256ull << 20;
 cudaMemPool_t g_pool[64] = {};
@@ -875,15 +884,67 @@ cudaMemPool_t workspace_pool(int dev)
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
         cudaMemPool_t pool = nullptr;
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;          // the calling thread may be capturing: this is no part of it
-        cudaThreadExchangeStreamCaptureMode(&mode);
+        RelaxedCapture relaxed;                    // another thread may be capturing
         unsigned long long keep = kKeep;
-        const bool ok = cudaMemPoolCreate(&pool, &props) == cudaSuccess && cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess;
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        if (!ok) { cudaGetLastError(); return nullptr; }
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaGetLastError();
+            cudaMemPoolDestroy(pool);
+            return nullptr;
+        }
         g_pool[dev] = pool;
     }
     return g_pool[dev];
+}
+
+// Inside of a capture an allocation would become a node of the graph, and graphs with such nodes can be neither child graphs
+// nor bodies of conditional nodes.  The workspace is then ordinary memory that the graph owns (a user object), shared by the calls that
+// were captured on one stream, which run one after another; it goes back to the device with the first call, or the first session
+// that ends, after the last executable of the graph is gone (a user object's destructor may not call CUDA itself).
+struct CaptureSpace {
+    unsigned long long capture;
+    cudaStream_t stream;
+    size_t bytes;
+    void *ptr;
+};
+std::vector<CaptureSpace> g_captured;              // their graphs are alive
+std::vector<void *> g_orphans;                     // their graphs are gone
+std::mutex g_capture_mu;
+
+void CUDART_CB graph_gone(void *ptr)
+{
+    std::lock_guard<std::mutex> lock(g_capture_mu);
+    g_captured.erase(std::remove_if(g_captured.begin(), g_captured.end(), [&](const CaptureSpace &c) { return c.ptr == ptr; }), g_captured.end());
+    g_orphans.push_back(ptr);
+}
+
+// Null: no room.
+void *capture_workspace(unsigned long long capture, cudaGraph_t graph, cudaStream_t stream, size_t bytes)
+{
+    {
+        std::lock_guard<std::mutex> lock(g_capture_mu);
+        for (const CaptureSpace &c : g_captured)
+            if (c.capture == capture && c.stream == stream && c.bytes >= bytes) return c.ptr;
+    }
+    RelaxedCapture relaxed;
+    void *ptr = nullptr;
+    cudaUserObject_t owner = nullptr;
+    if (cudaMalloc(&ptr, bytes) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    if (cudaUserObjectCreate(&owner, ptr, graph_gone, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(ptr);
+        return nullptr;
+    }
+    {
+        std::lock_guard<std::mutex> lock(g_capture_mu);
+        g_captured.push_back({capture, stream, bytes, ptr});
+    }
+    if (cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        cudaGetLastError();
+        cudaUserObjectRelease(owner, 1);
+        return nullptr;
+    }
+    return ptr;
 }
 
 template <int FMT, int PLANES>
@@ -896,6 +957,18 @@ int launch_split(const SplitParams &p, uint32_t ctas, cudaStream_t stream)
 
 }  // namespace
 
+void release_graph_workspaces()
+{
+    std::vector<void *> gone;
+    {
+        std::lock_guard<std::mutex> lock(g_capture_mu);
+        gone.swap(g_orphans);
+    }
+    if (gone.empty()) return;
+    RelaxedCapture relaxed;
+    for (void *p : gone) cudaFree(p);
+}
+
 // When there is no room for the workspace, nothing is launched for the rows from *done on.
 int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const float *addend, float *c,
                       uint32_t m, uint32_t k, uint32_t n, void *stream_v, uint32_t *done)
@@ -905,8 +978,14 @@ int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const 
     MGQ_CUDA(cudaGetDevice(&dev));
     MGQ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     *done = 0;
-    cudaMemPool_t pool = workspace_pool(dev);
-    if (!pool) return MGQ_OK;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    unsigned long long capture = 0;
+    cudaGraph_t graph = nullptr;
+    MGQ_CUDA(cudaStreamGetCaptureInfo(stream, &capturing, &capture, &graph));
+    const bool captured = capturing == cudaStreamCaptureStatusActive;
+    if (!captured) release_graph_workspaces();
+    cudaMemPool_t pool = captured ? nullptr : workspace_pool(dev);
+    if (!captured && !pool) return MGQ_OK;
     const bool bf16 = a_dtype == MGQ_A_BF16, q4 = fmt == MGQ_FMT_Q4;
     const uint32_t planes = bf16 ? 1 : 2;
     const size_t elem = bf16 ? 2 : 4;
@@ -938,11 +1017,11 @@ int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const 
         const size_t plane_bytes = (size_t)p.m_tiles * p.chunks * 2 * planes * p.tok * 128;
         const size_t scale_bytes = ((size_t)p.m_tiles * p.chunks * p.tok * 4 + 255) / 256 * 256;
         const size_t part_bytes = (size_t)ctas * 2 * kMaxTok * kCols * 4, odd_bytes = (size_t)p.tiles * 256 * 8, words = (size_t)p.tiles * 9;
+        const size_t all_bytes = plane_bytes + scale_bytes + part_bytes + odd_bytes + words * 4;
         uint8_t *ws = nullptr;
-        if (cudaMallocFromPoolAsync(reinterpret_cast<void **>(&ws), plane_bytes + scale_bytes + part_bytes + odd_bytes + words * 4, pool, stream) != cudaSuccess) {
-            cudaGetLastError();
-            return MGQ_OK;
-        }
+        if (captured) ws = static_cast<uint8_t *>(capture_workspace(capture, graph, stream, all_bytes));
+        else if (cudaMallocFromPoolAsync(reinterpret_cast<void **>(&ws), all_bytes, pool, stream) != cudaSuccess) cudaGetLastError(), ws = nullptr;
+        if (!ws) return MGQ_OK;
         float *scales = reinterpret_cast<float *>(ws + plane_bytes);
         p.planes = ws;
         p.scales = scales;
@@ -957,7 +1036,7 @@ int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const 
         if (rc == MGQ_OK)
             rc = q4 ? (bf16 ? launch_split<MGQ_FMT_Q4, 1>(p, ctas, stream) : launch_split<MGQ_FMT_Q4, 2>(p, ctas, stream))
                     : (bf16 ? launch_split<MGQ_FMT_Q8, 1>(p, ctas, stream) : launch_split<MGQ_FMT_Q8, 2>(p, ctas, stream));
-        const int freed = cuda_check((int)cudaFreeAsync(ws, stream), "cudaFreeAsync", __FILE__, __LINE__);
+        const int freed = captured ? MGQ_OK : cuda_check((int)cudaFreeAsync(ws, stream), "cudaFreeAsync", __FILE__, __LINE__);
         if (rc != MGQ_OK) return rc;
         if (freed != MGQ_OK) return freed;
         *done = r0 + p.m;

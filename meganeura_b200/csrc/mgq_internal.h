@@ -52,6 +52,7 @@ int launch_gemm(int fmt, const void *a, int a_dtype, const void *w, const float 
 // Tensor-core GEMM with split operands (mgq_gemm_split.cu): any shape; rows from *done on are left when there is no room for its workspace.
 int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const float *addend, float *c,
                       uint32_t m, uint32_t k, uint32_t n, void *stream, uint32_t *done);
+void release_graph_workspaces();      // of captured calls whose graphs are gone
 int tc_device_status();
 int linear_tc_status();               // mgq_linear_tc.cu
 

@@ -1576,6 +1576,7 @@ void mgq_session_free(mgq_session *s)
     if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
     if (s->graph) cudaGraphDestroy(s->graph);
+    mgq::release_graph_workspaces();
     for (Buffer &b : s->buffers) if (b.dev) cudaFree(b.dev);
     for (void *w : s->workspaces) if (w) cudaFree(w);
     if (s->greedy_ws) cudaFree(s->greedy_ws);

@@ -310,3 +310,92 @@ def test_one_chunk_of_bf16(fmt, m, n, split):
     assert torch.equal(got, tiled) != split
     want = xd.double().cpu().numpy() @ _dense(fmt, w, k, n)
     assert O.rel_l2(got.cpu().numpy(), want) <= _bound("bf16", k)
+
+
+def test_captured_graph_serves_as_a_child_graph():
+    """Kernels only: a graph that holds allocation nodes is refused as a child graph."""
+    import torch
+    from cuda.bindings import runtime as cudart
+    from meganeura_b200 import ops
+
+    def call(fn, *args):
+        out = fn(*args)
+        assert out[0] == cudart.cudaError_t.cudaSuccess, (fn.__name__, out[0])
+        return out[1] if len(out) == 2 else out[1:]
+    shapes = [(O.FMT_Q4, 40, 1024, 300), (O.FMT_Q8, 200, 2048, 700), (O.FMT_Q4, 130, 512, 1000)]
+    work = []
+    for i, (fmt, m, k, n) in enumerate(shapes):
+        w, x = _inputs(fmt, m, k, n, seed=i)
+        xd, wd = to_dev(x), to_dev(w)
+        work.append((fmt, xd, wd, k, n, torch.zeros((m, n), device="cuda"), ops.matmul(fmt, xd, wd, k, n, route="gemm")))
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    side = torch.cuda.Stream()
+    with torch.cuda.graph(graph):                             # two streams of one capture, two calls on one of them
+        side.wait_stream(torch.cuda.current_stream())
+        for i, (fmt, xd, wd, k, n, out, _) in enumerate(work):
+            with torch.cuda.stream(side if i == 1 else torch.cuda.current_stream()):
+                ops.matmul(fmt, xd, wd, k, n, out=out, route="gemm")
+        torch.cuda.current_stream().wait_stream(side)
+    raw = cudart.cudaGraph_t(graph.raw_cuda_graph())
+    parent = call(cudart.cudaGraphCreate, 0)
+    call(cudart.cudaGraphAddChildGraphNode, parent, None, 0, raw)
+    exe = call(cudart.cudaGraphInstantiate, parent, 0)
+    stream = torch.cuda.current_stream().cuda_stream
+    for _ in range(3):
+        for item in work:
+            item[5].zero_()
+        call(cudart.cudaGraphLaunch, exe, stream)
+        torch.cuda.synchronize()
+        assert all(torch.equal(out, want) for *_, out, want in work)
+    call(cudart.cudaGraphExecDestroy, exe)
+    call(cudart.cudaGraphDestroy, parent)
+    ops.device_status()
+
+
+def test_workspace_of_a_captured_graph_goes_back_with_it():
+    import torch
+    from meganeura_b200 import ops
+    fmt, m, k, n = O.FMT_Q4, 1024, 4096, 512
+    w, x = _inputs(fmt, m, k, n)
+    xd, wd, out = to_dev(x), to_dev(w), torch.zeros((m, n), device="cuda")
+
+    def capture():
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            ops.matmul(fmt, xd, wd, k, n, out=out, route="gemm")
+        graph.replay()
+        torch.cuda.synchronize()
+        del graph
+        torch.cuda.synchronize()
+        ops.matmul(fmt, xd, wd, k, n, out=out, route="gemm")  # the call that follows returns it
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+    capture()
+    free = [capture() for _ in range(6)]
+    assert min(free) >= free[0] - (8 << 20)                   # a workspace of this size is 40 MB
+
+
+@pytest.mark.parametrize("fmt", FMTS)
+def test_session_with_a_prompt_captured(fmt):
+    """A session of matmuls of many rows steps, captures and replays on new inputs."""
+    import meganeura_b200 as mg
+    m, k, n = 37, 512, 384
+    w1, w2 = _inputs(fmt, m, k, n)[0], _inputs(fmt, m, n, k, seed=3)[0]
+    g = mg.Graph()
+    x = g.input("x", [m, k])
+    param = g.parameter_q4 if fmt == O.FMT_Q4 else g.parameter_q8
+    y = g.matmul(g.matmul(x, param("w1", [k, n])), param("w2", [n, k]))
+    g.set_outputs([y])
+    s = mg.build_inference_session(g)
+    s.upload_param("w1", w1)
+    s.upload_param("w2", w2)
+    d1, d2 = _dense(fmt, w1, k, n), _dense(fmt, w2, n, k)
+    for seed in range(4):
+        a = _inputs(fmt, m, k, n, seed=seed)[1]
+        s.set_input("x", a)
+        if seed == 1:
+            s.capture()
+        s.step()
+        s.wait()
+        got = s.read_output(m * k).reshape(m, k)
+        assert O.rel_l2(got, a.astype(np.float64) @ d1 @ d2) <= 2 * _bound("f32", k)
