@@ -107,6 +107,7 @@ int launch_channel_decay_scan(const ChannelDecay &a, void *stream);
 size_t gla_chunks_workspace(uint32_t max_rows, uint32_t heads, uint32_t dim, uint32_t vdim);
 size_t wkv_chunks_workspace(uint32_t max_rows, uint32_t heads, uint32_t dim, uint32_t vdim);
 int launch_channel_decay_chunks(const ChannelDecay &a, void *stream);
+bool decay_in_chunks(uint32_t rank, uint32_t dim, uint32_t rows);        // the chunks' preparation computes the decay itself
 int launch_channel_decay_step(const ChannelDecay &a, const HeadGate &hg, void *stream);      // rows == 1: decay, recurrence, head gate in one launch
 
 // mLSTM recurrence.  q, k [rows, heads * dim], v, o [rows, heads * vdim], gate pre-activations

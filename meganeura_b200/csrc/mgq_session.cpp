@@ -1929,8 +1929,7 @@ static int run_mixer(mgq_session *s, const Dispatch &d)
         a.shift_width = o.inputs[6] >= 0 ? (uint32_t)(s->nodes[o.inputs[6]].elements() / 2) : 0;
         if (!fused) return mgq::launch_channel_decay_scan(a, s->stream);
         if (rows == 1) return mgq::launch_channel_decay_step(a, hg, s->stream);
-        // the preparation computes gated linear attention's decays itself (rank 16); time mixing's (rank 64) are 30 us cheaper in a kernel of their own
-        a.decay_pending = a.split_products && rows >= mgq::kPrefillRows && o.op == Op::Gla;
+        a.decay_pending = a.split_products && rows >= mgq::kPrefillRows && mgq::decay_in_chunks(a.d.rank, o.at[1], rows);
         if (!a.decay_pending)
             if (int rc = mgq::launch_decay(a.d, s->stream)) return rc;
         if (int rc = mgq::launch_channel_decay_scan(a, s->stream)) return rc;
