@@ -22,7 +22,7 @@
 // accumulator and a scale: 5e-7, and half the drains (149 -> 143 us for 512 x 4096 x 14336 in a long run).
 //
 // Up to 16 f32 rows on Q8 weights that no streaming GEMV takes would otherwise be summed in short f32 trees, 1.2e-7 off.  For them an
-// accumulator takes 32 k and its sums are added with what they round away: 1.0e-7 (2.0e-7 with 128 k).  16 x 12320 x 4099: 72 us
+// accumulator takes 32 k and its sums are added with what they round away: 1.0e-7 (2.0e-7 with 128 k).  16 x 12320 x 4099: 66 us
 // (45 with 128 k, 3312 with that GEMV).
 //
 // Weights are the left operand, straight from TMEM: a tile is 128 weight columns (TMEM lanes) by up to 128
@@ -95,7 +95,6 @@ struct SplitParams {
     uint32_t tok, m_tiles, tiles;   // tokens of a tile, tiles
     uint32_t chunks;                // per tile
     uint32_t units;                 // tiles * chunks
-    uint32_t fine;                  // an accumulator per 32 k, compensated sums; one group of 16 tokens only
     uint32_t wide;                  // packed weights can be copied 16 bytes at a time
 };
 
@@ -514,7 +513,8 @@ __device__ __forceinline__ void add_part(const float *src, uint32_t groups, floa
         }
 }
 
-template <int FMT, int PLANES>
+// FINE: an accumulator per 32 k, compensated sums; one group of 16 tokens only.
+template <int FMT, int PLANES, bool FINE>
 __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __grid_constant__ SplitParams p)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -522,7 +522,6 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
     constexpr uint32_t kRawChunk = kCols * raw_bytes(FMT);
     constexpr uint32_t kParts = 2 * PLANES, kDepth = kSlots / kParts;       // sub-tiles of a chunk, chunks in the ring
     const uint32_t group = PLANES == 1 ? group_of(PLANES, p.k) : 1;
-    const bool fine = FMT == MGQ_FMT_Q8 && PLANES == 2 && p.fine;
     uint8_t *ring = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t sub = p.tok * 128u;                          // bytes of a token sub-tile, a multiple of 2048
     const uint32_t scale_bytes = p.tok * 4u;                    // a multiple of 64
@@ -604,7 +603,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t x_lo = ring16 + s * kParts * sub16, x_hi = x_lo + (kParts - 2) * sub16;
-                if (fine) {                                     // all quarters of the chunk but the last
+                if (FINE) {                                     // all quarters of the chunk but the last
                     for (uint32_t from = 0; from < 6; from += 2) {
                         if (leader) {
                             issue_products<PLANES, 2>(tm + b * kMaxTok, w_hi, w_lo, x_hi, x_lo, sub16, instr, from, false);
@@ -619,7 +618,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                     if (!ok) break;
                 }
                 if (leader) {
-                    if (fine) issue_products<PLANES, 2>(tm + b * kMaxTok, w_hi, w_lo, x_hi, x_lo, sub16, instr, 6, false);
+                    if (FINE) issue_products<PLANES, 2>(tm + b * kMaxTok, w_hi, w_lo, x_hi, x_lo, sub16, instr, 6, false);
                     else      issue_products<PLANES, 8>(tm + b * kMaxTok, w_hi, w_lo, x_hi, x_lo, sub16, instr, 0, open);
                     umma_commit(&sh.w_empty[stage]);
                     umma_commit(&sh.slot_empty[s]);
@@ -659,14 +658,14 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                 const uint32_t sc = i % kScaleSlots, span = group > 1 ? min(c % group, c - c0) + 1 : 1;
                 const uint32_t x = i + 1 - lane;                // lane 0: the accumulator, 1..span: scales of its chunks
                 const uint8_t *scale = scale_ring + sc * scale_bytes + first * 4u;
-                for (uint32_t h = fine ? 0 : 3; h < 4; h++) {
+                for (uint32_t h = FINE ? 0 : 3; h < 4; h++) {
                     const uint32_t b = filled & 1u;
                     mbar_wait_lanes(lane == 0 ? &sh.d_full[b] : &sh.sc_full[x % kScaleSlots], lane == 0 ? (filled >> 1) & 1u : (x / kScaleSlots) & 1u, lane <= span, &sh.failed);
                     filled++;
                     __syncwarp();                               // tcgen05.ld is warp-collective
                     tc_fence_after();
                     const uint32_t from = tmem + lane_addr + b * kMaxTok + first;
-                    if (fine) {
+                    if (FINE) {
                         if (mine > 0) drain_fine(from, scale, acc[0], acc[1]);
                     } else {
                         if (mine > 1) drain_part<0, 2>(from, scale, acc);
@@ -682,7 +681,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                     for (uint32_t y = 0; y < span; y++) mbar_arrive(&sh.sc_empty[(i - y) % kScaleSlots]);
             }
             u += c1 - c0;
-            if (fine)                                           // before any part is added: the sum of two must not depend on which comes last
+            if (FINE)                                           // before any part is added: the sum of two must not depend on which comes last
 #pragma unroll
                 for (int e = 0; e < 16; e++) acc[0][e] += acc[1][e];
 
@@ -728,7 +727,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                         for (int g = 0; g < 4; g++)
 #pragma unroll
                             for (int e = 0; e < 16; e++) acc[g][e] = 0.f;
-                        if (fine) {
+                        if (FINE) {
                             for (uint32_t s = head; s <= tail && mine > 0; s++) {
                                 const float *part = part_of(s);
                                 float v[16];
@@ -947,12 +946,12 @@ void *capture_workspace(unsigned long long capture, cudaGraph_t graph, cudaStrea
     return ptr;
 }
 
-template <int FMT, int PLANES>
+template <int FMT, int PLANES, bool FINE = false>
 int launch_split(const SplitParams &p, uint32_t ctas, cudaStream_t stream)
 {
     const size_t smem = 1024 + (size_t)kSlots * p.tok * 128 + (size_t)kScaleSlots * p.tok * 4 + (size_t)kRaw * kCols * raw_bytes(FMT);
-    if (int rc = allow_smem(gemm_split_kernel<FMT, PLANES>, smem)) return rc;
-    return launch(gemm_split_kernel<FMT, PLANES>, dim3(ctas), dim3(kSplitThreads), smem, stream, p);
+    if (int rc = allow_smem(gemm_split_kernel<FMT, PLANES, FINE>, smem)) return rc;
+    return launch(gemm_split_kernel<FMT, PLANES, FINE>, dim3(ctas), dim3(kSplitThreads), smem, stream, p);
 }
 
 }  // namespace
@@ -1011,7 +1010,7 @@ int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const 
         p.units = (uint32_t)units;
         // Q8: whole 16-byte pieces of 4 blocks; Q4: nibbles behind num_blocks header words
         p.wide = q4 ? p.num_blocks % 4 == 0 : p.bpc % 4 == 0;
-        p.fine = !q4 && !bf16 && m <= MGQ_GEMV_MAX_M && !gemv_streamable(fmt, a, k, n) && !gemv_mma_eligible(m, k, n, a, w);
+        const bool fine = !q4 && !bf16 && m <= MGQ_GEMV_MAX_M && !gemv_streamable(fmt, a, k, n) && !gemv_mma_eligible(m, k, n, a, w);
         const uint32_t ctas = p.units / 2 < 1 ? 1 : p.units / 2 < (uint32_t)sms ? p.units / 2 : (uint32_t)sms;
 
         const size_t plane_bytes = (size_t)p.m_tiles * p.chunks * 2 * planes * p.tok * 128;
@@ -1035,7 +1034,7 @@ int launch_gemm_split(int fmt, const void *a, int a_dtype, const void *w, const 
         int rc = cuda_check((int)cudaGetLastError(), "split_rows_kernel", __FILE__, __LINE__);
         if (rc == MGQ_OK)
             rc = q4 ? (bf16 ? launch_split<MGQ_FMT_Q4, 1>(p, ctas, stream) : launch_split<MGQ_FMT_Q4, 2>(p, ctas, stream))
-                    : (bf16 ? launch_split<MGQ_FMT_Q8, 1>(p, ctas, stream) : launch_split<MGQ_FMT_Q8, 2>(p, ctas, stream));
+                    : (bf16 ? launch_split<MGQ_FMT_Q8, 1>(p, ctas, stream) : fine ? launch_split<MGQ_FMT_Q8, 2, true>(p, ctas, stream) : launch_split<MGQ_FMT_Q8, 2>(p, ctas, stream));
         const int freed = captured ? MGQ_OK : cuda_check((int)cudaFreeAsync(ws, stream), "cudaFreeAsync", __FILE__, __LINE__);
         if (rc != MGQ_OK) return rc;
         if (freed != MGQ_OK) return freed;
