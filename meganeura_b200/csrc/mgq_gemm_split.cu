@@ -237,25 +237,6 @@ __device__ __forceinline__ void copy4(uint32_t dst, const void *src, bool live)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(live ? 4u : 0u) : "memory");
 }
 
-// D[128 lanes, N] (+)= A (f16 pairs in TMEM, 8 columns) . B (shared memory)
-template <bool ACC>
-__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint32_t b16, uint32_t instr)
-{
-    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-                 "setp.ne.b32 p, %5, 0;\n\t"
-                 "mov.b64 db, {%2, %4};\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
-                 ::"r"(d), "r"(a), "r"(b16 | 0x10000u), "r"(instr), "r"(kDescHigh), "n"(ACC ? 1 : 0) : "memory");
-}
-// D = A . B + D * 2^-kLowShift
-__device__ __forceinline__ void umma_f16_ts_scaled(uint32_t d, uint32_t a, uint32_t b16, uint32_t instr)
-{
-    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-                 "setp.ne.b32 p, 1, 0;\n\t"
-                 "mov.b64 db, {%2, %4};\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p, %5;\n\t}"
-                 ::"r"(d), "r"(a), "r"(b16 | 0x10000u), "r"(instr), "r"(kDescHigh), "n"(kLowShift) : "memory");
-}
 // Products of the K = 16 steps from .. from + COUNT - 1 of a chunk into one accumulator, the small ones first.  open: it holds a chunk already.
 template <int PLANES, int COUNT>
 __device__ __forceinline__ void issue_products(uint32_t d, uint32_t w_hi, uint32_t w_lo, uint32_t x_hi, uint32_t x_lo, uint32_t sub16, uint32_t instr, uint32_t from, bool open)
@@ -266,7 +247,7 @@ __device__ __forceinline__ void issue_products(uint32_t d, uint32_t w_hi, uint32
         umma_f16_ts<false>(d, w_at(w_hi, 0), x_at(x_lo, 0), instr);
 #pragma unroll
         for (uint32_t j = 1; j < COUNT; j++) umma_f16_ts<true>(d, w_at(w_hi, j), x_at(x_lo, j), instr);
-        umma_f16_ts_scaled(d, w_at(w_lo, 0), x_at(x_hi, 0), instr);
+        umma_f16_ts_scaled<kLowShift>(d, w_at(w_lo, 0), x_at(x_hi, 0), instr);
     } else if (open) umma_f16_ts<true>(d, w_at(w_lo, 0), x_at(x_hi, 0), instr);
     else             umma_f16_ts<false>(d, w_at(w_lo, 0), x_at(x_hi, 0), instr);
 #pragma unroll
@@ -274,29 +255,8 @@ __device__ __forceinline__ void issue_products(uint32_t d, uint32_t w_hi, uint32
 #pragma unroll
     for (uint32_t j = 0; j < COUNT; j++) umma_f16_ts<true>(d, w_at(w_hi, j), x_at(x_hi, j), instr);
 }
-// A converged warp waits for several barriers at once, a lane (with `mine` set) for each: the try_waits share one latency.
-__device__ __forceinline__ bool mbar_wait_lanes(unsigned long long *bar, uint32_t parity, bool mine, volatile int *failed)
-{
-    bool done = !mine;
-    for (uint32_t i = 0; i < kWaitLimit; i++) {
-        if (!done) done = mbar_try_wait(bar, parity);
-        if (__all_sync(0xffffffffu, done)) return true;
-        if (__any_sync(0xffffffffu, *failed != 0)) return false;
-    }
-    *failed = 1;
-    atomicExch(&g_split_error, 1u);
-    return false;
-}
 // kind::f16 instruction descriptor: D f32, A and B f16, both K-major.
 __device__ __forceinline__ uint32_t split_instr(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((kCols >> 4) << 24); }
-
-__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16])
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-                 "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-                 ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
 
 __device__ __forceinline__ __half2 as_half2(uint32_t v) { return *reinterpret_cast<const __half2 *>(&v); }
 __device__ __forceinline__ uint32_t as_word(__half2 v) { return *reinterpret_cast<const uint32_t *>(&v); }
@@ -449,16 +409,6 @@ __device__ __forceinline__ void fetch_weights(const SplitParams &p, uint32_t dst
     }
 }
 
-// a += v * s for two neighbours in one instruction (each rounded as by fmaf).
-__device__ __forceinline__ void fma_pair(float &a0, float &a1, uint32_t v0, uint32_t v1, float s0, float s1)
-{
-    asm("{\n\t.reg .b64 a, v, s;\n\t"
-        "mov.b64 a, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tmov.b64 s, {%4, %5};\n\t"
-        "fma.rn.f32x2 a, v, s, a;\n\t"
-        "mov.b64 {%0, %1}, a;\n\t}"
-        : "+f"(a0), "+f"(a1) : "r"(v0), "r"(v1), "f"(s0), "f"(s1));
-}
-
 // COUNT groups of 16 tokens: sums += accumulator * scale.
 template <int G0, int COUNT>
 __device__ __forceinline__ void drain_part(uint32_t from, const uint8_t *scale, float (&acc)[4][16])
@@ -477,8 +427,8 @@ __device__ __forceinline__ void drain_part(uint32_t from, const uint8_t *scale, 
 #pragma unroll
         for (int e = 0; e < 16; e += 4) {
             const float4 s = *reinterpret_cast<const float4 *>(scale + ((G0 + g) * 16 + e) * 4);
-            fma_pair(acc[G0 + g][e], acc[G0 + g][e + 1], r[g][e], r[g][e + 1], s.x, s.y);
-            fma_pair(acc[G0 + g][e + 2], acc[G0 + g][e + 3], r[g][e + 2], r[g][e + 3], s.z, s.w);
+            fma_pair(acc[G0 + g][e], acc[G0 + g][e + 1], __uint_as_float(r[g][e]), __uint_as_float(r[g][e + 1]), s.x, s.y);
+            fma_pair(acc[G0 + g][e + 2], acc[G0 + g][e + 3], __uint_as_float(r[g][e + 2]), __uint_as_float(r[g][e + 3]), s.z, s.w);
         }
 }
 
@@ -599,7 +549,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                 // lane 0: accumulator, 1: weights, 4..: the chunk's sub-tiles
                 unsigned long long *bar = lane == 0 ? &sh.d_empty[b] : lane == 1 ? &sh.w_full[stage] : &sh.slot_full[(s * kParts + lane - 4u) % kSlots];
                 const uint32_t parity = lane == 0 ? ((filled >> 1) & 1u) ^ 1u : lane == 1 ? ph : (i / kDepth) & 1u;
-                ok = mbar_wait_lanes(bar, parity, lane < 2 || (lane >= 4 && lane < 4 + kParts), &sh.failed);
+                ok = mbar_wait_lanes(bar, parity, lane < 2 || (lane >= 4 && lane < 4 + kParts), &sh.failed, &g_split_error);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t x_lo = ring16 + s * kParts * sub16, x_hi = x_lo + (kParts - 2) * sub16;
@@ -612,7 +562,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                         __syncwarp();
                         filled++;
                         b = filled & 1u;
-                        ok = ok && mbar_wait_lanes(&sh.d_empty[b], ((filled >> 1) & 1u) ^ 1u, lane == 0, &sh.failed);
+                        ok = ok && mbar_wait_lanes(&sh.d_empty[b], ((filled >> 1) & 1u) ^ 1u, lane == 0, &sh.failed, &g_split_error);
                         tc_fence_after();
                     }
                     if (!ok) break;
@@ -660,7 +610,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split_kernel(const __gr
                 const uint8_t *scale = scale_ring + sc * scale_bytes + first * 4u;
                 for (uint32_t h = FINE ? 0 : 3; h < 4; h++) {
                     const uint32_t b = filled & 1u;
-                    mbar_wait_lanes(lane == 0 ? &sh.d_full[b] : &sh.sc_full[x % kScaleSlots], lane == 0 ? (filled >> 1) & 1u : (x / kScaleSlots) & 1u, lane <= span, &sh.failed);
+                    mbar_wait_lanes(lane == 0 ? &sh.d_full[b] : &sh.sc_full[x % kScaleSlots], lane == 0 ? (filled >> 1) & 1u : (x / kScaleSlots) & 1u, lane <= span, &sh.failed, &g_split_error);
                     filled++;
                     __syncwarp();                               // tcgen05.ld is warp-collective
                     tc_fence_after();

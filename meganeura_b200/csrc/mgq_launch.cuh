@@ -78,6 +78,16 @@ __device__ __forceinline__ float warp_max(float v)
     return v;
 }
 
+// (a0, a1) += (x0, x1) * (y0, y1) in one instruction, each rounded as by fmaf.
+__device__ __forceinline__ void fma_pair(float &a0, float &a1, float x0, float x1, float y0, float y1)
+{
+    asm("{\n\t.reg .b64 a, x, y;\n\t"
+        "mov.b64 a, {%0, %1};\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+        "fma.rn.f32x2 a, x, y, a;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t}"
+        : "+f"(a0), "+f"(a1) : "f"(x0), "f"(x1), "f"(y0), "f"(y1));
+}
+
 __device__ __forceinline__ float to_f32(float v) { return v; }
 __device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ float to_f32(__half v) { return __half2float(v); }

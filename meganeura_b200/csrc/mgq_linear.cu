@@ -171,16 +171,6 @@ __device__ __forceinline__ float4 cluster_load4(const float *p, uint32_t rank)
     return v;
 }
 
-// (c0, c1) += a * (w0, w1), each rounded as by fmaf.
-__device__ __forceinline__ void fma_pair(float &c0, float &c1, float a, float w0, float w1)
-{
-    asm("{\n\t.reg .b64 c, a, w;\n\t"
-        "mov.b64 c, {%0, %1};\n\tmov.b64 a, {%2, %2};\n\tmov.b64 w, {%3, %4};\n\t"
-        "fma.rn.f32x2 c, a, w, c;\n\t"
-        "mov.b64 {%0, %1}, c;\n\t}"
-        : "+f"(c0), "+f"(c1) : "f"(a), "f"(w0), "f"(w1));
-}
-
 __device__ __forceinline__ void load4(const float *p, float (&v)[4])
 {
     const float4 q = *reinterpret_cast<const float4 *>(p);
@@ -311,8 +301,8 @@ __global__ void __launch_bounds__(128) linear_tiled_kernel(const __grid_constant
                 const float4 v = *reinterpret_cast<const float4 *>(s_w + (u * BK + kk) * LW + tx * 4);
 #pragma unroll
                 for (int i = 0; i < RM; i++) {
-                    fma_pair(acc[u][i][0], acc[u][i][1], ar[i], v.x, v.y);
-                    fma_pair(acc[u][i][2], acc[u][i][3], ar[i], v.z, v.w);
+                    fma_pair(acc[u][i][0], acc[u][i][1], ar[i], ar[i], v.x, v.y);
+                    fma_pair(acc[u][i][2], acc[u][i][3], ar[i], ar[i], v.z, v.w);
                 }
             }
         }

@@ -47,6 +47,19 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t pari
     atomicExch(error, 1u);
     return false;
 }
+// A converged warp waits for several barriers at once, a lane (with `mine` set) for each: the try_waits share one latency.
+__device__ __forceinline__ bool mbar_wait_lanes(unsigned long long *bar, uint32_t parity, bool mine, volatile int *failed, unsigned int *error)
+{
+    bool done = !mine;
+    for (uint32_t i = 0; i < kWaitLimit; i++) {
+        if (!done) done = mbar_try_wait(bar, parity);
+        if (__all_sync(0xffffffffu, done)) return true;
+        if (__any_sync(0xffffffffu, *failed != 0)) return false;
+    }
+    *failed = 1;
+    atomicExch(error, 1u);
+    return false;
+}
 
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, unsigned long long *bar)
 {
@@ -54,29 +67,13 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
                  ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
 }
 
-// K-major, 128-byte swizzle: rows are 128 B apart, 8-row groups 1024 B apart (SBO), version 1.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr)
-{
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);          // start address, 16-byte units
-    d |= (uint64_t)1 << 16;                                // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;                      // stride byte offset
-    d |= (uint64_t)1 << 46;                                // descriptor version (Blackwell)
-    d |= (uint64_t)2 << 61;                                // SWIZZLE_128B
-    return d;
-}
 // kind::f16 instruction descriptor: D f32, A bf16, B bf16, both K-major.
 __host__ __device__ constexpr uint32_t umma_instr(uint32_t m, uint32_t n) { return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24); }
 
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t instr, uint32_t accumulate)
-{
-    asm volatile("{\n\t.reg .pred p;\n\t"
-                 "setp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-                 ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(instr), "r"(accumulate), "r"(0u) : "memory");
-}
-// The same for operands in the layout of umma_desc, from the low words of their descriptors (address / 16, rest fixed): the
-// high words are constants, so that a step costs one add per operand.
+// Operands in shared memory are K-major in the 128-byte swizzle, their descriptors given by the low word: address / 16 in bits 0-13,
+// a leading byte offset (unused for a swizzled K-major operand) in bits 16-29.  The high word is a constant, so that a step
+// costs one add per operand: stride byte offset (8-row groups, 1024 B) / 16 in bits 32-45, version 1 (Blackwell) in bits 46-47,
+// SWIZZLE_128B = 2 in bits 61-63.
 constexpr uint32_t kDescHigh = (1024 >> 4) | (1u << 14) | (2u << 29);
 template <bool ACC>
 __device__ __forceinline__ void umma_step(uint32_t tmem_d, uint32_t a16, uint32_t b16, uint32_t instr)
@@ -86,6 +83,26 @@ __device__ __forceinline__ void umma_step(uint32_t tmem_d, uint32_t a16, uint32_
                  "mov.b64 da, {%1, %4};\n\tmov.b64 db, {%2, %4};\n\t"
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}"
                  ::"r"(tmem_d), "r"(a16 | 0x10000u), "r"(b16 | 0x10000u), "r"(instr), "r"(kDescHigh), "n"(ACC ? 1 : 0) : "memory");
+}
+// D[128 lanes, N] (+)= A (f16 pairs in TMEM, 8 columns) . B (shared memory)
+template <bool ACC>
+__device__ __forceinline__ void umma_f16_ts(uint32_t d, uint32_t a, uint32_t b16, uint32_t instr)
+{
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+                 "setp.ne.b32 p, %5, 0;\n\t"
+                 "mov.b64 db, {%2, %4};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n\t}"
+                 ::"r"(d), "r"(a), "r"(b16 | 0x10000u), "r"(instr), "r"(kDescHigh), "n"(ACC ? 1 : 0) : "memory");
+}
+// D = A . B + D * 2^-SHIFT
+template <uint32_t SHIFT>
+__device__ __forceinline__ void umma_f16_ts_scaled(uint32_t d, uint32_t a, uint32_t b16, uint32_t instr)
+{
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+                 "setp.ne.b32 p, 1, 0;\n\t"
+                 "mov.b64 db, {%2, %4};\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p, %5;\n\t}"
+                 ::"r"(d), "r"(a), "r"(b16 | 0x10000u), "r"(instr), "r"(kDescHigh), "n"(SHIFT) : "memory");
 }
 // One lane of a converged warp.
 __device__ __forceinline__ bool elect_one()
@@ -126,6 +143,14 @@ __device__ __forceinline__ void tmem_ld32(uint32_t addr, float (&y)[32])
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < 32; i++) y[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+                 "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t *base_smem, uint32_t columns)
