@@ -277,20 +277,21 @@ def decode_tokens_per_s(model: str, steps: int = 128, context: int = 2048):
         s.step()
     s.wait()
     dec.set_position(1, context)
+    launched = s.launch_count()
     t0 = time.perf_counter()
     for _ in range(steps):
         s.step()
     s.wait()
     tokens = s.read_tokens(context, steps)
     dt = time.perf_counter() - t0
+    launched = s.launch_count() - launched
     last = s.read_output(cfg.vocab_size)
     finite = finite and bool(np.isfinite(last).all())
-    plan = s.plan().dispatches
     kv_bytes = 2 * cfg.num_hidden_layers * cfg.kv_dim * 4 * (context + steps // 2)
     distinct = int(len(set(int(t) for t in tokens)))
     out = {"model": f"{cfg.name}-shaped, seeded N(0,0.02^2) weights through the quantizer", "tokens_per_s": round(steps / dt, 1),
            "ms_per_token": round(dt / steps * 1e3, 4), "steps": steps, "kv_context": context, "batch": 1,
-           "launches_per_token": len(plan) + 1, "greedy_pick": "device", "timing": "host wall clock around launch + final token read",
+           "launches_per_token": launched // steps, "greedy_pick": "device", "timing": "host wall clock around launch + final token read",
            "weight_plus_kv_gbs": round((M.packed_weight_bytes(cfg) + kv_bytes) / (dt / steps) / 1e9, 1),
            "distinct_tokens": distinct, "logits_finite": finite, "build_s": round(build_s, 1)}
     if distinct <= 1 or not finite:
@@ -331,10 +332,12 @@ def decode_sharded_tokens_per_s(model: str, rank: int, world: int, steps: int = 
     s.wait()
     dec.set_position(1, context)
     dist.barrier()
+    launches = s.launch_count()
     t0 = time.perf_counter()
     for _ in range(steps):
         s.step()
     s.wait()
+    launches = (s.launch_count() - launches) // steps
     tokens = np.asarray(s.read_tokens(context, steps), dtype=np.int64)
     dt = torch.tensor([time.perf_counter() - t0], dtype=torch.float64, device="cuda")
     dist.all_reduce(dt, op=dist.ReduceOp.MAX)
@@ -351,7 +354,6 @@ def decode_sharded_tokens_per_s(model: str, rank: int, world: int, steps: int = 
     same = all(bool(torch.equal(t, mine)) for t in everyone)
     flag = torch.tensor([1 if timeout else 0], device="cuda")
     dist.all_reduce(flag, op=dist.ReduceOp.MAX)
-    launches = len(s.plan().dispatches) + 2
     del dec, s
     torch.cuda.empty_cache()
     if rank != 0:
