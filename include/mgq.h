@@ -77,7 +77,8 @@ const char *mgq_version(void);
  *                               1 gate|up under a SwiGLU only (the reference's rule,
  *                               src/optimize.rs:776-879), 2 every such group, e.g. q|k|v (default)
  *   "session.fuse_rope_cache"   1 (default): RoPE(q), RoPE(k), CacheWrite(k), CacheWrite(v) of a decode
- *                               layer run as one launch; 0: four dispatches like the reference
+ *                               layer are one dispatch, which the cached attention behind it runs along (its
+ *                               profile entry is then 0); 0: four dispatches like the reference
  *   "session.fuse_mixer"        1 (default): in graphs with bf16 linear layers biases, residual adds, clamped
  *                               GLUs, head gates and row picks run inside their producers, and independent
  *                               linear layers of one K as one launch; 0: one launch per node

@@ -43,9 +43,10 @@
 //
 // What bounds it: of the 2650 cycles that a chunk of 128 x 128 takes with f32 activations the tensor core needs 1536 (2100 and 1024
 // for bf16), the rest is the hand-over of a weight stage: products of chunk i - 2 done, conversion (1500 cycles, four warps),
-// products of chunk i; 52 % of the issue slots are taken.  Measured and dropped: weight stages of 64 k (147 instead
-// of 112 us for bf16, twice the waits), two issuing warps, both groups on every chunk, two token tiles per converted weight (no change).
-// In a long run (the power cap adds a tenth) 512 x 4096 x 12288 Q4 f32 takes 161 us against 1993 on the CUDA cores, 512 x 4096 x 14336 Q8
+// products of chunk i; 52 % of the issue slots are taken (62 % with Q4, whose weights take three times the instructions of Q8's).
+// Measured and dropped: weight stages of 64 k (147 instead of 112 us for bf16, twice the waits), two issuing warps, both groups on
+// every chunk, two token tiles per converted weight (no change).
+// In a long run (the power cap adds a tenth) 512 x 4096 x 12288 Q4 f32 takes 167 us against 1993 on the CUDA cores, 512 x 4096 x 14336 Q8
 // bf16 143 against 147 us of a kernel with one 112-column strip of bf16 weight pairs per CTA and 512 tokens, whose sums were
 // 9.4e-6 off.
 //
