@@ -857,23 +857,33 @@ struct CaptureSpace {
     size_t bytes;
     void *ptr;
 };
-std::vector<CaptureSpace> g_captured;              // their graphs are alive
-std::vector<void *> g_orphans;                     // their graphs are gone
-std::mutex g_capture_mu;
+struct GraphSpaces {
+    std::vector<CaptureSpace> captured;            // their graphs are alive
+    std::vector<void *> orphans;                   // their graphs are gone
+    std::mutex mu;
+};
+// Never destroyed: a destructor may run on a thread of the driver's while the process ends.
+GraphSpaces &graph_spaces()
+{
+    static GraphSpaces *spaces = new GraphSpaces;
+    return *spaces;
+}
 
 void CUDART_CB graph_gone(void *ptr)
 {
-    std::lock_guard<std::mutex> lock(g_capture_mu);
-    g_captured.erase(std::remove_if(g_captured.begin(), g_captured.end(), [&](const CaptureSpace &c) { return c.ptr == ptr; }), g_captured.end());
-    g_orphans.push_back(ptr);
+    GraphSpaces &g = graph_spaces();
+    std::lock_guard<std::mutex> lock(g.mu);
+    g.captured.erase(std::remove_if(g.captured.begin(), g.captured.end(), [&](const CaptureSpace &c) { return c.ptr == ptr; }), g.captured.end());
+    g.orphans.push_back(ptr);
 }
 
 // Null: no room.
 void *capture_workspace(unsigned long long capture, cudaGraph_t graph, cudaStream_t stream, size_t bytes)
 {
+    GraphSpaces &g = graph_spaces();
     {
-        std::lock_guard<std::mutex> lock(g_capture_mu);
-        for (const CaptureSpace &c : g_captured)
+        std::lock_guard<std::mutex> lock(g.mu);
+        for (const CaptureSpace &c : g.captured)
             if (c.capture == capture && c.stream == stream && c.bytes >= bytes) return c.ptr;
     }
     RelaxedCapture relaxed;
@@ -886,8 +896,8 @@ void *capture_workspace(unsigned long long capture, cudaGraph_t graph, cudaStrea
         return nullptr;
     }
     {
-        std::lock_guard<std::mutex> lock(g_capture_mu);
-        g_captured.push_back({capture, stream, bytes, ptr});
+        std::lock_guard<std::mutex> lock(g.mu);
+        g.captured.push_back({capture, stream, bytes, ptr});
     }
     if (cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove) != cudaSuccess) {
         cudaGetLastError();
@@ -911,8 +921,8 @@ void release_graph_workspaces()
 {
     std::vector<void *> gone;
     {
-        std::lock_guard<std::mutex> lock(g_capture_mu);
-        gone.swap(g_orphans);
+        std::lock_guard<std::mutex> lock(graph_spaces().mu);
+        gone.swap(graph_spaces().orphans);
     }
     if (gone.empty()) return;
     RelaxedCapture relaxed;
