@@ -46,8 +46,8 @@
 // products of chunk i; 52 % of the issue slots are taken (62 % with Q4, whose weights take three times the instructions of Q8's).
 // Measured and dropped: weight stages of 64 k (147 instead of 112 us for bf16, twice the waits), two issuing warps, both groups on
 // every chunk, two token tiles per converted weight (no change).
-// In a long run (the power cap adds a tenth) 512 x 4096 x 12288 Q4 f32 takes 167 us against 1993 on the CUDA cores, 512 x 4096 x 14336 Q8
-// bf16 143 against 147 us of a kernel with one 112-column strip of bf16 weight pairs per CTA and 512 tokens, whose sums were
+// In a long run (the power cap adds a tenth) 512 x 4096 x 12288 Q4 f32 takes 155 us against 1993 on the CUDA cores, 512 x 4096 x 14336 Q8
+// bf16 142 against 147 us of a kernel with one 112-column strip of bf16 weight pairs per CTA and 512 tokens, whose sums were
 // 9.4e-6 off.
 //
 // Every mbarrier wait is bounded; when one runs out the device-wide error word is raised (mgq_device_status reports
